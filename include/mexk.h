@@ -221,7 +221,7 @@ int mexk_bincsr_probe(const char* path, mexk_bincsr_info_t* info);
 int mexk_context_load_bincsr(mexk_context_t ctx, const char* path, int m_alloc_max, mexk_bincsr_info_t* info);
 
 /* E = exp(A) for a k-by-k FP64 matrix (device pointers, column-major,
- * leading dimensions lda/lde), single thread block Pade scaling-and-squaring
+ * leading dimensions lda/lde), Pade scaling-and-squaring on one thread-block cluster
  * (replaces Eigen's MatrixXd::exp at main.cu:33-36). k <= MEXK_M_MAX. */
 int mexk_expm_f64(int k, const double* A, int lda, double* E, int lde, void* stream);
 

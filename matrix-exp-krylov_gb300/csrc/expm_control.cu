@@ -3,16 +3,20 @@
 // The reference computes the small exponential on the host with Eigen
 // (matrix_exp_stable, main.cu:33-36), twice per attempt (small_expm_and_lift
 // main.cu:1954-1978 and residual_estimate main.cu:2004-2020), after copying
-// every H entry to the host. Here one thread block holds the k-by-k matrices
-// in shared memory and evaluates the Pade scaling-and-squaring method of
+// every H entry to the host. Here a thread-block cluster holds the k-by-k
+// matrices in shared memory, each block its share of the columns, and
+// evaluates the Pade scaling-and-squaring method of
 // N. J. Higham, SIAM J. Matrix Anal. Appl. 26(4), 2005 (the method Eigen
 // 3.4's MatrixExponential implements): degree 3/5/7/9/13 from the 1-norm,
 // 2^-s scaling before degree 13, an LU solve with partial pivoting for
-// (V-U)^{-1}(V+U), then s squarings. The same exponential feeds the lift
-// coefficients and the residual estimate |H(k,k-1) [exp(dt H_k) e1]_{k-1}| |v|.
+// (V-U)^{-1}(V+U), then s squarings. Only the first column of the result is
+// used (the lift coefficients and the residual estimate
+// |H(k,k-1) [exp(dt H_k) e1]_{k-1}| |v|), so the last squaring forms that
+// column alone. Per attempt, one SM against 16: 250 -> 70 us at k = 30,
+// 1.9 -> 0.45 ms at k = 100.
 //
 // The controller (ArnoldiRunner::compute_expmv, main.cu:1431-1518) runs in
-// the same block with the reference's arithmetic: accept if err <= tol or
+// the cluster's leading block with the reference's arithmetic: accept if err <= tol or
 // breakdown; grow dt by 1.5*0.8 when err < 0.1*tol (capped at dt_max);
 // otherwise shrink by 0.5*0.8 (floored at dt_min) and retry, aborting after
 // 20 rejects. The reference rebuilds the whole Arnoldi basis on every retry;
@@ -89,120 +93,8 @@ __device__ __forceinline__ double dot_banded(int k, int i, int j, const double* 
     return dot_k_band(k, lo, hi, X + i, k, Y + j * k);
 }
 
-__device__ void mm(int k, const double* X, const double* Y, double* Z) {
-    const int kk = k * k;
-    for (int e = threadIdx.x; e < kk; e += blockDim.x) {
-        const int i = e % k, j = e / k;
-        Z[e] = dot_k(k, X + i, k, Y + j * k);
-    }
-    __syncthreads();
-}
-
-// Z = c0*M0 + c1*M1 + c2*M2 + c3*M3 + cid*I, terms left to right (nt <= 4).
-__device__ void lincomb(int k, int nt, const double* c, const double* const* M, double cid, double* Z) {
-    const int kk = k * k;
-    for (int e = threadIdx.x; e < kk; e += blockDim.x) {
-        double s = c[0] * M[0][e];
-        for (int t = 1; t < nt; ++t) s = s + c[t] * M[t][e];
-        if (cid != 0.0 && (e % k) == (e / k)) s = s + cid;
-        Z[e] = s;
-    }
-    __syncthreads();
-}
-
-__device__ void lu_factor(int k, double* D, int* piv, int* status) {
-    for (int c = 0; c < k; ++c) {
-        if (threadIdx.x < 32) {
-            double best = -1.0;
-            int bi = k;
-            for (int i = c + threadIdx.x; i < k; i += 32) {
-                const double v = fabs(D[i + c * k]);
-                if (v > best) {
-                    best = v;
-                    bi = i;
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (ob > best || (ob == best && oi < bi)) {
-                    best = ob;
-                    bi = oi;
-                }
-            }
-            if (threadIdx.x == 0) piv[c] = (bi < k) ? bi : c;
-        }
-        __syncthreads();
-        const int p = piv[c];
-        if (p != c) {
-            for (int j = threadIdx.x; j < k; j += blockDim.x) {
-                const double t = D[c + j * k];
-                D[c + j * k] = D[p + j * k];
-                D[p + j * k] = t;
-            }
-            __syncthreads();
-        }
-        const double d = D[c + c * k];
-        if (d != 0.0) {
-            for (int i = c + 1 + threadIdx.x; i < k; i += blockDim.x) D[i + c * k] /= d;
-            __syncthreads();
-            const int r = k - c - 1;
-            for (int e = threadIdx.x; e < r * r; e += blockDim.x) {
-                const int i = c + 1 + e % r, j = c + 1 + e / r;
-                D[i + j * k] -= D[i + c * k] * D[c + j * k];
-            }
-        } else if (threadIdx.x == 0) {
-            *status |= ST_LU_SINGULAR;
-        }
-        __syncthreads();
-    }
-}
-
-__device__ void lu_solve(int k, const double* LU, const int* piv, double* B) {
-    for (int i = 0; i < k; ++i) {
-        const int p = piv[i];
-        if (p != i) {
-            for (int c = threadIdx.x; c < k; c += blockDim.x) {
-                const double t = B[i + c * k];
-                B[i + c * k] = B[p + c * k];
-                B[p + c * k] = t;
-            }
-            __syncthreads();
-        }
-    }
-    for (int i = 0; i < k - 1; ++i) {
-        const int r = k - i - 1;
-        for (int e = threadIdx.x; e < r * k; e += blockDim.x) {
-            const int l = i + 1 + e % r, c = e / r;
-            B[l + c * k] -= LU[l + i * k] * B[i + c * k];
-        }
-        __syncthreads();
-    }
-    for (int i = k - 1; i >= 0; --i) {
-        for (int c = threadIdx.x; c < k; c += blockDim.x) B[i + c * k] /= LU[i + i * k];
-        __syncthreads();
-        for (int e = threadIdx.x; e < i * k; e += blockDim.x) {
-            const int l = e % i, c = e / i;
-            B[l + c * k] -= LU[l + i * k] * B[i + c * k];
-        }
-        __syncthreads();
-    }
-}
-
-// Pade [m/m] coefficients b_j = (2m-j)! / (j! (m-j)!), exact integers.
-__device__ void pade_coefficients(int m, double* b) {
-    for (int j = 0; j <= m; ++j) {
-        unsigned long long num = 1ull, den = 1ull;
-        for (int i = m - j + 1; i <= 2 * m - j; ++i) num *= static_cast<unsigned long long>(i);
-        for (int i = 2; i <= j; ++i) den *= static_cast<unsigned long long>(i);
-        b[j] = static_cast<double>(num / den);
-    }
-}
-
 struct ExpmBuf {
     double *A, *A2, *A4, *A6, *U, *T;
-    int* piv;
     double* red;  // >= k doubles
 };
 
@@ -220,119 +112,420 @@ __device__ __forceinline__ double col_abs_sum(int k, const double* A, int j) {
     return (c0 + c1) + (c2 + c3);
 }
 
-// exp of the k-by-k matrix in B.A (ld k) by Pade scaling and squaring;
-// returns the buffer holding the result. All threads of the block must call it.
-__device__ double* expm_block(const ExpmBuf& B, int k, int* status) {
-    __shared__ int s_deg, s_sq;
-    __shared__ double s_b[14];
-    if (threadIdx.x < k) B.red[threadIdx.x] = col_abs_sum(k, B.A, threadIdx.x);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double l1 = 0.0;
-        for (int j = 0; j < k; ++j)
-            if (B.red[j] > l1) l1 = B.red[j];
-        int sq = 0, deg;
-        // A non-finite norm (Inf or NaN entries) keeps degree 13 without
-        // scaling: frexp's exponent is unspecified there, and the squaring
-        // loop must stay bounded; the result is then non-finite as well.
-        if (!(l1 <= 1.7976931348623157e308)) {
-            deg = 13;
-            *status |= ST_NONFINITE;
-        } else if (l1 < 1.495585217958292e-002) deg = 3;
-        else if (l1 < 2.539398330063230e-001) deg = 5;
-        else if (l1 < 9.504178996162932e-001) deg = 7;
-        else if (l1 < 2.097847961257068e+000) deg = 9;
-        else {
-            deg = 13;
-            (void)frexp(l1 / 5.371920351148152, &sq);
-            if (sq < 0) sq = 0;
-            if (sq > 1100) sq = 1100;  // beyond the double range: l1 is finite here
-        }
-        s_deg = deg;
-        s_sq = sq;
-        pade_coefficients(deg, s_b);
+// Pade [m/m] coefficients b_j = (2m-j)! / (j! (m-j)!): exact integers, each
+// rounded once to double.
+constexpr double pade_coefficient(int m, int j) {
+    unsigned long long num = 1ull, den = 1ull;
+    for (int i = m - j + 1; i <= 2 * m - j; ++i) num *= static_cast<unsigned long long>(i);
+    for (int i = 2; i <= j; ++i) den *= static_cast<unsigned long long>(i);
+    return static_cast<double>(num / den);
+}
+struct PadeTable {
+    double b[14];
+};
+constexpr PadeTable pade_table(int m) {
+    PadeTable t{};
+    for (int j = 0; j <= m; ++j) t.b[j] = pade_coefficient(m, j);
+    return t;
+}
+__constant__ PadeTable kPade[5] = {pade_table(3), pade_table(5), pade_table(7), pade_table(9), pade_table(13)};
+
+// The Pade exponential of one k x k matrix over the thread blocks of a
+// cluster. This GPU executes about two FP64 FMAs per clock per SM, so a
+// product of two k x k matrices takes k^3 / 2 clocks on one SM (6.5 us at
+// k = 30, 240 us at k = 100) and the whole exponential, on one SM, took
+// 250 us and 1.9 ms. Here block r owns columns [r w, (r+1) w) of every matrix
+// (w = ceil(k / blocks)) and keeps one full copy of a product's left factor,
+// pulled from the owners' shared memory when the factor changes; products,
+// linear combinations and the solve then touch own columns only. Every
+// element is computed by the operations, in the order, of a single block's
+// right-looking LU and dot_k products, so the result does not depend on the
+// cluster size.
+extern __shared__ double expm_smem[];  // named here so that accesses compile to shared-memory ones
+
+struct ClusterExpm {
+    int k, w, j0, nj;   // own columns j0 .. j0+nj-1
+    int o_own, o_red;   // offsets into expm_smem: five k x w buffers, k doubles
+
+    __device__ explicit ClusterExpm(int kk) {
+        const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        const int c = static_cast<int>(cl.num_blocks()), r = static_cast<int>(cl.block_rank());
+        k = kk;
+        w = (k + c - 1) / c;
+        j0 = min(k, r * w);
+        nj = min(k, (r + 1) * w) - j0;
+        o_own = k * k;
+        o_red = o_own + 5 * k * w;
     }
-    __syncthreads();
-    const int deg = s_deg, sq = s_sq;
-    const int kk = k * k;
-    if (sq > 0) {
-        for (int e = threadIdx.x; e < kk; e += blockDim.x) B.A[e] = ldexp(B.A[e], -sq);
+    // the left factor of the products, then the LU: k x k
+    __device__ double* left() const { return expm_smem; }
+    __device__ double* own(int i) const { return expm_smem + o_own + i * k * w; }
+    __device__ double* red() const { return expm_smem + o_red; }
+    static size_t smem_bytes(int k, int blocks) {
+        const size_t w = (k + blocks - 1) / blocks;
+        return sizeof(double) * (static_cast<size_t>(k) * k + 5 * k * w + MEXK_M_MAX);
+    }
+    // The left factor = the matrix whose own columns every block holds in
+    // own(b) (final: the cluster barrier orders them before the reads).
+    __device__ void gather(int b) const {
+        const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        cl.sync();
+        double* L = left();
+        const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+        for (int col = threadIdx.x >> 5; col < k; col += nw) {
+            const int owner = col / w;
+            const double* src = cl.map_shared_rank(own(b), owner) + static_cast<size_t>(col - owner * w) * k;
+            for (int i = lane; i < k; i += 32) L[i + col * k] = src[i];
+        }
         __syncthreads();
     }
-    const double* b = s_b;
-    mm(k, B.A, B.A, B.A2);
-    if (deg >= 5) mm(k, B.A2, B.A2, B.A4);
-    if (deg >= 7) mm(k, B.A4, B.A2, B.A6);
-    double *pU, *pV;
+    // Column c, row i of L Y: dot_k's four running sums in four adjacent lanes
+    // (q = lane % 4; the first also takes the tail), combined by a butterfly.
+    // A warp's FP64 instruction occupies its quarter of the SM for 64 clocks
+    // whatever its independence from the last one, so the sums are spread over
+    // warps instead of kept in one thread.
+    __device__ __forceinline__ double dot4(int i, const double* Y, int q) const {
+        double s = 0.0;
+        const double* X = left() + i;
+        for (int l = q; l + 3 - q < k; l += 4) s = fma(X[l * k], Y[l], s);
+        if (q == 0)
+            for (int l = k & ~3; l < k; ++l) s = fma(X[l * k], Y[l], s);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        return s + __shfl_xor_sync(0xffffffffu, s, 2);
+    }
+    // f(e, value) for every element e = i + j k of the own columns of L Y (Y:
+    // its own columns, ld k; cols of them)
+    template <typename F>
+    __device__ __forceinline__ void product(const double* Y, int cols, F f) const {
+        const int cnt = k * cols;
+        for (int t = threadIdx.x; t < ((4 * cnt + 31) & ~31); t += blockDim.x) {
+            const int e = min(t >> 2, cnt - 1);
+            const int i = e % k, j = e / k;
+            const double v = dot4(i, Y + j * k, t & 3);
+            if ((t & 3) == 0 && (t >> 2) < cnt) f(e, v);
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ void mm(const double* Y, double* Z) const {
+        if (nj > 0) product(Y, nj, [&](int e, double v) { Z[e] = v; });
+    }
+    // own columns of c0*M0 + c1*M1 + c2*M2 + cid*I, terms left to right
+    __device__ __forceinline__ void lincomb(int nt, const double* c, const double* const* M, double cid, double* Z) const {
+        for (int e = threadIdx.x; e < k * nj; e += blockDim.x) {
+            double s = c[0] * M[0][e];
+            for (int t = 1; t < nt; ++t) s = s + c[t] * M[t][e];
+            if (cid != 0.0 && (e % k) == j0 + e / k) s = s + cid;
+            Z[e] = s;
+        }
+        __syncthreads();
+    }
+    // x / d for a finite nonzero d. A zero x takes no division: a quotient
+    // outside the fast range costs a warp about 1000 clocks more, and the
+    // denominator polynomial of a Hessenberg matrix is zero below its band.
+    static __device__ __forceinline__ double quotient(double x, double d) {
+        const bool zero = (__double2hiint(x) & 0x7fffffff) == 0 && __double2loint(x) == 0;
+        if (zero) return __hiloint2double((__double2hiint(x) ^ __double2hiint(d)) & 0x80000000, 0);
+        return x / d;
+    }
+    // LU with partial pivoting of the k x k matrix in L (every block its own
+    // copy), the eliminations also applied to the own columns of B as they
+    // go; then the back substitution, one warp per column. Warp 0 runs one
+    // column ahead: it eliminates the next pivot column in registers (rows
+    // lane + 32 u), searches its pivot by integer comparison of the
+    // magnitudes' bits, divides and stores it, while the other warps still
+    // eliminate the last one (one barrier per column).
+    template <int U>
+    __device__ __forceinline__ void solve_u(double* B, int* status) const {
+        __shared__ int s_piv[2];
+        double* const L = left();
+        const int k = this->k, nj = this->nj;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        double v[U];
+        if (warp == 0) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = lane + 32 * u < k ? L[lane + 32 * u] : 0.0;
+        }
+        auto row_of = [&](int r) {  // row r of the register column, in every lane
+            double x = 0.0;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if ((r >> 5) == u) x = __shfl_sync(0xffffffffu, v[u], r & 31);
+            return x;
+        };
+        auto swap_rows = [&](int c, int p) {
+            const double vc = row_of(c), vp = row_of(p);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (lane + 32 * u == c) v[u] = vp;
+                else if (lane + 32 * u == p) v[u] = vc;
+            }
+            return vp;  // row c after the swap
+        };
+        for (int c = 0; c < k; ++c) {
+            if (warp == 0) {
+                // the largest magnitude in rows >= c, the lowest such row, NaN never
+                unsigned bh = 0, bl = 0;
+                int bi = k;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int i = lane + 32 * u;
+                    const unsigned hi = static_cast<unsigned>(__double2hiint(v[u])) & 0x7fffffffu;
+                    const unsigned lo = static_cast<unsigned>(__double2loint(v[u]));
+                    const bool cand = i >= c && i < k && !(hi > 0x7ff00000u || (hi == 0x7ff00000u && lo != 0u));
+                    if (cand && (hi + 1u > bh || (hi + 1u == bh && lo > bl))) {
+                        bh = hi + 1u;
+                        bl = lo;
+                        bi = i;
+                    }
+                }
+                const unsigned mh = __reduce_max_sync(0xffffffffu, bh);
+                const unsigned ml = __reduce_max_sync(0xffffffffu, bh == mh ? bl : 0u);
+                const int mi = __reduce_min_sync(0xffffffffu, (bh == mh && bl == ml) ? bi : k);
+                const int p = mi < k ? mi : c;
+                const double d = swap_rows(c, p);
+                const bool live = (__double2hiint(d) & 0x7fffffff) != 0 || __double2loint(d) != 0;
+                const bool finite = (__double2hiint(d) & 0x7ff00000) != 0x7ff00000;
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const int i = lane + 32 * u;
+                    if (live && i > c && i < k) v[u] = finite ? quotient(v[u], d) : v[u] / d;
+                    if (i < k) L[i + c * k] = v[u];
+                }
+                if (lane == 0) {
+                    s_piv[c & 1] = live ? p : -1 - p;
+                    if (!live) *status |= ST_LU_SINGULAR;
+                }
+            }
+            __syncthreads();
+            const int pv = s_piv[c & 1];
+            const bool live = pv >= 0;
+            const int p = live ? pv : -1 - pv;
+            if (warp == 0) {
+                if (c + 1 < k) {
+                    double l[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        l[u] = v[u];
+                        v[u] = lane + 32 * u < k ? L[lane + 32 * u + (c + 1) * k] : 0.0;
+                    }
+                    const double top = swap_rows(c, p);
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+                        if (live && lane + 32 * u > c && lane + 32 * u < k) v[u] -= l[u] * top;
+                }
+            } else {
+                const double* lc = L + c * k;
+                const int rest = max(k - 2 - c, 0);  // columns c+2 .. k-1 of L, then the own columns of B
+                for (int q = warp - 1; q < rest + nj; q += nw - 1) {
+                    double* col = q < rest ? L + static_cast<size_t>(c + 2 + q) * k : B + static_cast<size_t>(q - rest) * k;
+                    const double top = col[p], old = col[c];
+                    __syncwarp();
+                    if (lane == 0 && p != c) {
+                        col[c] = top;
+                        col[p] = old;
+                    }
+                    __syncwarp();
+                    if (live)
+                        for (int i = c + 1 + lane; i < k; i += 32) col[i] -= lc[i] * top;
+                }
+            }
+        }
+        __syncthreads();
+        for (int q = warp; q < nj; q += nw) {
+            double* col = B + static_cast<size_t>(q) * k;
+            double x[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) x[u] = lane + 32 * u < k ? col[lane + 32 * u] : 0.0;
+#pragma unroll
+            for (int u = U - 1; u >= 0; --u) {
+                for (int i = min(k, 32 * (u + 1)) - 1; i >= 32 * u; --i) {
+                    double xi = x[u];
+                    if (lane == (i & 31)) xi = xi / L[i + i * k];
+                    xi = __shfl_sync(0xffffffffu, xi, i & 31);
+                    if (lane == (i & 31)) x[u] = xi;
+#pragma unroll
+                    for (int t = 0; t <= u; ++t)
+                        if (lane + 32 * t < i) x[t] -= L[lane + 32 * t + i * k] * xi;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (lane + 32 * u < k) col[lane + 32 * u] = x[u];
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ void solve(double* B, int* status) const {
+        static_assert(MEXK_M_MAX <= 128, "four rows per lane");
+        if (k <= 32) solve_u<1>(B, status);
+        else if (k <= 64) solve_u<2>(B, status);
+        else solve_u<4>(B, status);
+    }
+};
+
+// exp(dt H_k) (H: column-major, leading dimension ldh) by Pade scaling and
+// squaring over the cluster; every thread of every block calls it. Returns
+// the buffer of own columns. first_only: only column 0 of the result is
+// wanted (block 0's first own column): the last squaring then forms that
+// column alone.
+__device__ __forceinline__ double* expm_pade(const ClusterExpm& B, double dt, const double* H, size_t ldh, bool first_only,
+                                          int* status) {
+    __shared__ int s_deg, s_sq;
+    const int k = B.k, kk = k * k;
+    double *const L = B.left(), *const red = B.red();
+    int sq = 0;
+    auto load_left = [&]() {  // L = dt H_k / 2^sq
+        // one multiplication by the power of two rounds as ldexp does
+        const double scale = sq <= 1022 ? __hiloint2double((1023 - sq) << 20, 0) : 0.0;
+        for (int e = threadIdx.x; e < kk; e += blockDim.x) {
+            const double v = dt * H[(e % k) + (e / k) * ldh];
+            L[e] = sq == 0 ? v : (sq <= 1022 ? v * scale : ldexp(v, -sq));
+        }
+        __syncthreads();
+    };
+    load_left();
+    // column sums of the magnitudes: col_abs_sum's four running sums in four adjacent lanes
+    for (int t = threadIdx.x; t < ((4 * k + 31) & ~31); t += blockDim.x) {
+        const int j = min(t >> 2, k - 1), q = t & 3;
+        double c = 0.0;
+        for (int i = q; i + 3 - q < k; i += 4) c += fabs(L[i + j * k]);
+        if (q == 0)
+            for (int i = k & ~3; i < k; ++i) c += fabs(L[i + j * k]);
+        c += __shfl_xor_sync(0xffffffffu, c, 1);
+        c += __shfl_xor_sync(0xffffffffu, c, 2);
+        if (q == 0 && (t >> 2) < k) red[j] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        // the largest sum, by the bits of non-negative doubles; a NaN sum never is
+        unsigned long long best = 0;
+        for (int j = threadIdx.x; j < k; j += 32) {
+            const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(red[j]));
+            if (u <= 0x7ff0000000000000ull && u > best) best = u;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long u = __shfl_xor_sync(0xffffffffu, best, o);
+            if (u > best) best = u;
+        }
+        if (threadIdx.x == 0) {
+            const double l1 = __longlong_as_double(static_cast<long long>(best));
+            int q = 0, deg;
+            // A non-finite norm (Inf or NaN entries) keeps degree 13 without
+            // scaling: frexp's exponent is unspecified there, and the squaring
+            // loop must stay bounded; the result is then non-finite as well.
+            if (!(l1 <= 1.7976931348623157e308)) {
+                deg = 13;
+                *status |= ST_NONFINITE;
+            } else if (l1 < 1.495585217958292e-002) deg = 3;
+            else if (l1 < 2.539398330063230e-001) deg = 5;
+            else if (l1 < 9.504178996162932e-001) deg = 7;
+            else if (l1 < 2.097847961257068e+000) deg = 9;
+            else {
+                deg = 13;
+                (void)frexp(l1 / 5.371920351148152, &q);
+                if (q < 0) q = 0;
+                if (q > 1100) q = 1100;  // beyond the double range: l1 is finite here
+            }
+            s_deg = deg;
+            s_sq = q;
+        }
+    }
+    __syncthreads();
+    const int deg = s_deg;
+    sq = s_sq;
+    if (sq > 0) load_left();
+    const double* b = kPade[deg == 13 ? 4 : (deg - 3) / 2].b;
+    double *A2 = B.own(0), *A4 = B.own(1), *A6 = B.own(2), *X = B.own(3), *Y = B.own(4);
+    int iu, iv;  // the buffers of U and V
+    const int cnt = k * B.nj;
+    const double* Aown = L + static_cast<size_t>(B.j0) * k;
+    B.mm(Aown, A2);
+    if (deg >= 5) {
+        B.gather(0);
+        B.mm(A2, A4);
+    }
+    if (deg >= 7) {
+        B.gather(1);
+        B.mm(A2, A6);
+    }
     if (deg <= 7) {
-        const double* M[3] = {deg == 3 ? B.A2 : (deg == 5 ? B.A4 : B.A6), deg == 7 ? B.A4 : B.A2, B.A2};
+        const double* M[3] = {deg == 3 ? A2 : (deg == 5 ? A4 : A6), deg == 7 ? A4 : A2, A2};
         const int nt = deg == 3 ? 1 : (deg == 5 ? 2 : 3);
         double cu[3], cv[3];
         if (deg == 3) { cu[0] = b[3]; cv[0] = b[2]; }
         if (deg == 5) { cu[0] = b[5]; cu[1] = b[3]; cv[0] = b[4]; cv[1] = b[2]; }
         if (deg == 7) { cu[0] = b[7]; cu[1] = b[5]; cu[2] = b[3]; cv[0] = b[6]; cv[1] = b[4]; cv[2] = b[2]; }
-        lincomb(k, nt, cu, M, b[1], B.T);
-        mm(k, B.A, B.T, B.U);
-        lincomb(k, nt, cv, M, b[0], B.T);
-        pU = B.U;
-        pV = B.T;
+        B.lincomb(nt, cu, M, b[1], X);
+        if (deg > 3) load_left();
+        B.mm(X, Y);
+        B.lincomb(nt, cv, M, b[0], X);
+        iu = 4;
+        iv = 3;
     } else if (deg == 9) {
-        mm(k, B.A6, B.A2, B.U);  // A8 in U
-        for (int e = threadIdx.x; e < kk; e += blockDim.x) {
-            const double a8 = B.U[e], a6 = B.A6[e], a4 = B.A4[e], a2 = B.A2[e];
-            const bool dg = (e % k) == (e / k);
+        B.gather(2);
+        B.mm(A2, Y);  // A8
+        for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
+            const double a8 = Y[e], a6 = A6[e], a4 = A4[e], a2 = A2[e];
+            const bool dg = (e % k) == B.j0 + e / k;
             double u = b[9] * a8 + b[7] * a6 + b[5] * a4 + b[3] * a2;
             double v = b[8] * a8 + b[6] * a6 + b[4] * a4 + b[2] * a2;
             if (dg) { u = u + b[1]; v = v + b[0]; }
-            B.T[e] = u;
-            B.U[e] = v;
+            X[e] = u;
+            Y[e] = v;
         }
         __syncthreads();
-        mm(k, B.A, B.T, B.A2);
-        pU = B.A2;
-        pV = B.U;
+        load_left();
+        B.mm(X, A2);
+        iu = 0;
+        iv = 4;
     } else {
-        const double* M[3] = {B.A6, B.A4, B.A2};
+        B.gather(2);
+        const double* M[3] = {A6, A4, A2};
         const double c1[3] = {b[13], b[11], b[9]};
-        lincomb(k, 3, c1, M, 0.0, B.T);
-        mm(k, B.A6, B.T, B.U);
-        for (int e = threadIdx.x; e < kk; e += blockDim.x) {
-            double s = b[7] * B.A6[e] + b[5] * B.A4[e] + b[3] * B.A2[e];
-            if ((e % k) == (e / k)) s = s + b[1];
-            B.U[e] = B.U[e] + s;
+        B.lincomb(3, c1, M, 0.0, X);
+        B.mm(X, Y);
+        for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
+            double s = b[7] * A6[e] + b[5] * A4[e] + b[3] * A2[e];
+            if ((e % k) == B.j0 + e / k) s = s + b[1];
+            Y[e] = Y[e] + s;
         }
-        __syncthreads();
-        mm(k, B.A, B.U, B.T);  // U final in T
         const double c3[3] = {b[12], b[10], b[8]};
-        lincomb(k, 3, c3, M, 0.0, B.U);
-        mm(k, B.A6, B.U, B.A);  // V in A
-        for (int e = threadIdx.x; e < kk; e += blockDim.x) {
-            double s = b[6] * B.A6[e] + b[4] * B.A4[e] + b[2] * B.A2[e];
-            if ((e % k) == (e / k)) s = s + b[0];
-            B.A[e] = B.A[e] + s;
-        }
-        __syncthreads();
-        pU = B.T;
-        pV = B.A;
+        B.lincomb(3, c3, M, 0.0, X);
+        if (B.nj > 0)
+            B.product(X, B.nj, [&](int e, double v) {
+                double s = b[6] * A6[e] + b[4] * A4[e] + b[2] * A2[e];
+                if ((e % k) == B.j0 + e / k) s = s + b[0];
+                A2[e] = v + s;  // V; this thread alone reads A2[e]
+            });
+        load_left();
+        B.mm(Y, A4);  // U
+        iu = 1;
+        iv = 0;
     }
+    double *const pU = B.own(iu), *const pV = B.own(iv);
     // numer = U + V (into pU), denom = -U + V (into pV)
-    for (int e = threadIdx.x; e < kk; e += blockDim.x) {
+    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
         const double u = pU[e], v = pV[e];
         pU[e] = u + v;
         pV[e] = -u + v;
     }
-    __syncthreads();
-    lu_factor(k, pV, B.piv, status);
-    lu_solve(k, pV, B.piv, pU);
-    double* R = pU;
-    double* F = pV;
-    for (int s = 0; s < sq; ++s) {
-        mm(k, R, R, F);
-        double* t = R;
-        R = F;
-        F = t;
+    B.gather(iv);
+    B.solve(pU, status);
+    int r = iu;
+    for (int q = 0; q < sq; ++q) {
+        const int f = r == 2 ? 3 : 2;
+        B.gather(r);
+        if (first_only && q == sq - 1) {
+            if (B.j0 == 0 && B.nj > 0) {
+                double* const Z = B.own(f);
+                B.product(B.own(r), 1, [&](int e, double v) { Z[e] = v; });
+            }
+        } else {
+            B.mm(B.own(r), B.own(f));
+        }
+        r = f;
     }
-    return R;
+    return B.own(r);
 }
 
 // 1/i!, i = 0..18: the factorials are exact in double, one rounding each.
@@ -512,51 +705,59 @@ __device__ ExpmBuf carve(double* smem, int k) {
     B.U = B.A6 + kk;
     B.T = B.U + kk;
     B.red = B.T + kk;
-    B.piv = reinterpret_cast<int*>(B.red + MEXK_M_MAX);
     return B;
 }
 
 size_t expm_smem_bytes(int k) {
-    return sizeof(double) * (6 * static_cast<size_t>(k) * k + MEXK_M_MAX) + sizeof(int) * MEXK_M_MAX;
+    return sizeof(double) * (6 * static_cast<size_t>(k) * k + MEXK_M_MAX);
 }
-
-// Dynamic shared memory of an exponential kernel for dimensions up to m:
-// none when the matrices live in the global workspace.
-size_t expm_launch_smem(int m) { return m > EXPM_SMEM_K ? 0 : expm_smem_bytes(m); }
 
 __global__ void __launch_bounds__(EXPM_THREADS)
     expm_standalone_kernel(int k, const double* __restrict__ A, int lda, double* __restrict__ E, int lde,
-                           int* status, double* ws) {
-    extern __shared__ double smem[];
-    ExpmBuf B = carve(k > EXPM_SMEM_K ? ws : smem, k);
-    for (int e = threadIdx.x; e < k * k; e += blockDim.x) B.A[e] = A[(e % k) + static_cast<size_t>(e / k) * lda];
+                           int* status) {
+    const ClusterExpm B(k);
+    __shared__ int s_st;  // every block meets the same conditions; block 0 reports them
+    if (threadIdx.x == 0) s_st = 0;
     __syncthreads();
-    double* R = expm_block(B, k, status);
-    for (int e = threadIdx.x; e < k * k; e += blockDim.x) E[(e % k) + static_cast<size_t>(e / k) * lde] = R[e];
+    const double* R = expm_pade(B, 1.0, A, static_cast<size_t>(lda), false, &s_st);
+    for (int e = threadIdx.x; e < k * B.nj; e += blockDim.x)
+        E[(e % k) + static_cast<size_t>(B.j0 + e / k) * lde] = R[e];
+    const cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    if (cl.block_rank() == 0 && threadIdx.x == 0 && s_st) atomicOr(status, s_st);
+    cl.sync();  // no block leaves while another may read its shared memory
 }
 
 enum : int { DEC_REJECT = 0, DEC_ACCEPT = 1, DEC_ABORT = 2, DEC_REBUILD = 3 };
 
 __global__ void __launch_bounds__(EXPM_THREADS) controller_kernel(ControlArgs a, int m) {
-    extern __shared__ double smem[];
-    __shared__ int s_k, s_bd, s_dec, s_mcur, s_cyc_bd, s_cyc_k;
+    // s_next: the decision every block of the cluster acts on, {k, breakdown,
+    // decision}, and the next attempt's step, written by the leading block
+    __shared__ int s_mcur, s_cyc_bd, s_cyc_k, s_st;
+    __shared__ int s_next[3];
     __shared__ double s_dt;
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const int nblocks = static_cast<int>(cl.num_blocks());
+    const bool lead = cl.block_rank() == 0;
     pdl_wait();  // launched as a dependent of the basis's last kernel
     pdl_trigger();
-    // One block per state: block b drives state b (a batch), or the only one.
-    DevState* st = a.st + blockIdx.x;
-    const double* Hb = a.H + blockIdx.x * a.h_stride;
-    double* coef = a.coef + blockIdx.x * a.coef_stride;
+    // One cluster per state: cluster b drives state b (a batch), or the only one.
+    const int state = static_cast<int>(blockIdx.x) / nblocks;
+    DevState* st = a.st + state;
+    const double* Hb = a.H + state * a.h_stride;
+    double* coef = a.coef + state * a.coef_stride;
+    // the state changes only in the leading block after the last cluster
+    // barrier (or when every block has read it): all blocks read the same here
     if (st->done) return;
     if (threadIdx.x == 0) {
         const int bd = st->breakdown;
         int k = bd ? st->k_used : m;
+        s_st = 0;
         if (k < 1 || k > m) {
-            st->status |= ST_BAD_K;
+            s_st = ST_BAD_K;
             k = k < 1 ? 1 : m;
         }
-        s_k = k;
-        s_bd = bd;
+        s_next[0] = k;
+        s_next[1] = bd;
         s_dt = st->dt;
         s_mcur = m;
         s_cyc_bd = bd;  // the basis built this cycle: m columns, or k_used up to a breakdown
@@ -564,20 +765,19 @@ __global__ void __launch_bounds__(EXPM_THREADS) controller_kernel(ControlArgs a,
     }
     __syncthreads();
     const size_t ldh = static_cast<size_t>(a.ldh);
-    // The matrices in shared memory, or (m > EXPM_SMEM_K) in the workspace.
-    double* const base = m > EXPM_SMEM_K ? a.ws : smem;
     int rejects = st->rejects;
     double err = 0.0;
-    double* R = nullptr;
+    const double* R = nullptr;
+    int dec = DEC_REJECT;
     while (true) {
-        const int k = s_k;
-        const bool bd = s_bd != 0;
-        ExpmBuf B = carve(base, k);
+        const int k = s_next[0];
+        const bool bd = s_next[1] != 0;
         const double dt = s_dt;
-        for (int e = threadIdx.x; e < k * k; e += blockDim.x) B.A[e] = dt * Hb[(e % k) + (e / k) * ldh];
-        __syncthreads();
-        R = expm_block(B, k, &st->status);
-        if (threadIdx.x == 0) {
+        const ClusterExpm B(k);
+        R = expm_pade(B, dt, Hb, ldh, true, &s_st);  // column 0, in the leading block
+        if (lead && threadIdx.x == 0) {
+            int nk = k, nbd = bd ? 1 : 0;
+            double ndt = dt;
             err = bd ? 0.0 : fabs(Hb[k + (k - 1) * ldh] * R[k - 1]) * st->v_norm;
             if (st->nlog < st->log_cap && a.log != nullptr) {
                 mexk_step_t& L = a.log[st->nlog];
@@ -591,7 +791,6 @@ __global__ void __launch_bounds__(EXPM_THREADS) controller_kernel(ControlArgs a,
             }
             st->nlog += 1;
             st->attempts += 1;
-            int dec;
             if (err <= st->tol || bd) {
                 dec = DEC_ACCEPT;
             } else {
@@ -612,24 +811,33 @@ __global__ void __launch_bounds__(EXPM_THREADS) controller_kernel(ControlArgs a,
                     } else {
                         dec = DEC_REJECT;
                         const double dt_new = (dt * st->shrink) * st->safety;
-                        s_dt = dt_new > st->dt_min ? dt_new : st->dt_min;
+                        ndt = dt_new > st->dt_min ? dt_new : st->dt_min;
                         mc = st->m_base;
                     }
                     s_mcur = mc;
                     if (dec == DEC_REJECT) {
                         const bool bd2 = s_cyc_bd && s_cyc_k <= mc;
-                        s_k = bd2 ? s_cyc_k : mc;
-                        s_bd = bd2 ? 1 : 0;
+                        nk = bd2 ? s_cyc_k : mc;
+                        nbd = bd2 ? 1 : 0;
                     }
                 }
             }
-            s_dec = dec;
+            for (int p = 0; p < nblocks; ++p) {
+                int* nx = cl.map_shared_rank(s_next, p);
+                nx[0] = nk;
+                nx[1] = nbd;
+                nx[2] = dec;
+                *cl.map_shared_rank(&s_dt, p) = ndt;
+            }
         }
-        __syncthreads();
-        if (s_dec != DEC_REJECT) break;
+        cl.sync();
+        dec = s_next[2];
+        if (dec != DEC_REJECT) break;
     }
-    const int k = s_k;
-    if (s_dec == DEC_REBUILD) {
+    if (!lead) return;  // after the barrier nothing reads this block's shared memory
+    const int k = s_next[0];
+    if (threadIdx.x == 0 && s_st) st->status |= s_st;
+    if (dec == DEC_REBUILD) {
         if (threadIdx.x == 0) {
             st->rejects = rejects;
             st->m_next = s_mcur;
@@ -652,7 +860,7 @@ __global__ void __launch_bounds__(EXPM_THREADS) controller_kernel(ControlArgs a,
         double dt = s_dt;
         st->rejects = 0;
         st->m_next = st->m_base;
-        if (s_dec == DEC_ACCEPT) {
+        if (dec == DEC_ACCEPT) {
             st->t_done += dt;
             st->accepted += 1;
             st->last_residual = err;
@@ -1047,31 +1255,79 @@ int launch_controller_search(const SearchArgs& a, int m, cudaStream_t s) {
     return MEXK_OK;
 }
 
-size_t expm_ws_doubles(int k) {
-    return 6 * static_cast<size_t>(k) * k + MEXK_M_MAX + (sizeof(int) * MEXK_M_MAX + sizeof(double) - 1) / sizeof(double);
+// Thread blocks per cluster of the Pade kernels: 16 where the device places
+// such a cluster (non-portable), else 8. Called after expm_init_attributes.
+static int pade_cluster() {
+    static const int blocks = [] {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(EXPM_THREADS);
+        cfg.dynamicSmemBytes = ClusterExpm::smem_bytes(MEXK_M_MAX, 16);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 16;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&fit, controller_kernel, &cfg);
+        if (e != cudaSuccess) (void)cudaGetLastError();
+        return (e == cudaSuccess && fit >= 1) ? 16 : 8;
+    }();
+    return blocks;
 }
 
 int expm_init_attributes() {
-    const int bytes = static_cast<int>(expm_smem_bytes(EXPM_SMEM_K));
+    MEXK_CK(cudaFuncSetAttribute(controller_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(expm_smem_bytes(EXPM_SMEM_K))));
+    const int bytes = static_cast<int>(ClusterExpm::smem_bytes(MEXK_M_MAX, 8));
     MEXK_CK(cudaFuncSetAttribute(expm_standalone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    MEXK_CK(cudaFuncSetAttribute(expm_standalone_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     MEXK_CK(cudaFuncSetAttribute(controller_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    MEXK_CK(cudaFuncSetAttribute(controller_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    MEXK_CK(cudaFuncSetAttribute(controller_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    (void)pade_cluster();  // resolved outside any stream capture
     return MEXK_OK;
 }
 
-int launch_expm_standalone(int k, const double* A, int lda, double* E, int lde, int* status, double* ws,
-                           cudaStream_t s) {
-    if (k > EXPM_SMEM_K && ws == nullptr) return MEXK_ERR_INVALID;
-    const size_t smem = expm_launch_smem(k);
-    expm_standalone_kernel<<<1, EXPM_THREADS, smem, s>>>(k, A, lda, E, lde, status, ws);
-    MEXK_CK_LAUNCH("expm_standalone_kernel");
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_clusters(void (*kernel)(KArgs...), int clusters, int blocks, size_t smem, cudaStream_t s,
+                                   Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(clusters * blocks);
+    cfg.blockDim = dim3(EXPM_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = blocks;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+int launch_expm_standalone(int k, const double* A, int lda, double* E, int lde, int* status, cudaStream_t s) {
+    const cudaError_t e = launch_clusters(expm_standalone_kernel, 1, pade_cluster(),
+                                          ClusterExpm::smem_bytes(k, pade_cluster()), s, k, A, lda, E, lde, status);
+    if (e != cudaSuccess) {
+        set_cuda_error(e, "expm_standalone_kernel", __FILE__, __LINE__);
+        return MEXK_ERR_CUDA;
+    }
     return MEXK_OK;
 }
 
 int launch_controller(const ControlArgs& a, int m, cudaStream_t s, int nstates) {
-    if (m > EXPM_SMEM_K && (a.ws == nullptr || nstates != 1)) return MEXK_ERR_INVALID;
-    const size_t smem = expm_launch_smem(m);
-    const cudaError_t e = launch_dependent(controller_kernel, nstates, EXPM_THREADS, smem, s, a, m);
+    // One cluster per state. A single solve takes the whole cluster; a batch
+    // as many blocks per state as leave every state an SM of its own (more
+    // states than SMs: one block each, the products' total work is the bound).
+    int blocks = pade_cluster();
+    while (blocks > 1 && static_cast<long long>(nstates) * blocks > device_sm_count()) blocks >>= 1;
+    const cudaError_t e =
+        launch_clusters(controller_kernel, nstates, blocks, ClusterExpm::smem_bytes(m, blocks), s, a, m);
     if (e != cudaSuccess) {
         set_cuda_error(e, "controller_kernel", __FILE__, __LINE__);
         return MEXK_ERR_CUDA;
@@ -1087,18 +1343,9 @@ extern "C" int mexk_expm_f64(int k, const double* A, int lda, double* E, int lde
     int rc0 = mexk::expm_init_attributes();
     if (rc0 != MEXK_OK) return rc0;
     int* d_status = nullptr;
-    double* d_ws = nullptr;
     MEXK_CK(cudaMallocAsync(reinterpret_cast<void**>(&d_status), sizeof(int), s));
-    if (k > mexk::EXPM_SMEM_K) {
-        const cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&d_ws), sizeof(double) * mexk::expm_ws_doubles(k), s);
-        if (e != cudaSuccess) {
-            cudaFreeAsync(d_status, s);
-            mexk::set_cuda_error(e, "cudaMallocAsync", __FILE__, __LINE__);
-            return MEXK_ERR_ALLOC;
-        }
-    }
     MEXK_CK(cudaMemsetAsync(d_status, 0, sizeof(int), s));
-    int rc = mexk::launch_expm_standalone(k, A, lda, E, lde, d_status, d_ws, s);
+    int rc = mexk::launch_expm_standalone(k, A, lda, E, lde, d_status, s);
     int h_status = 0;
     if (rc == MEXK_OK) {
         cudaError_t e = cudaMemcpyAsync(&h_status, d_status, sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -1109,7 +1356,6 @@ extern "C" int mexk_expm_f64(int k, const double* A, int lda, double* E, int lde
         }
     }
     cudaFreeAsync(d_status, s);
-    if (d_ws) cudaFreeAsync(d_ws, s);
     cudaStreamSynchronize(s);
     if (rc == MEXK_OK && (h_status & mexk::ST_LU_SINGULAR)) rc = MEXK_ERR_DEVICE;
     return rc;

@@ -472,12 +472,10 @@ int lanczos_cycle_test_hook(int enable);
 // Raises the dynamic shared-memory limits of the expm kernels; call once
 // per device before any launch or stream capture.
 int expm_init_attributes();
-// Largest k whose Pade matrices fit in shared memory; larger k (up to
-// MEXK_M_MAX) work in a global-memory workspace of expm_ws_doubles(k) doubles.
+// Largest k of the candidate-step controllers (their six matrices in one
+// block's shared memory). The Pade exponential takes k <= MEXK_M_MAX.
 constexpr int EXPM_SMEM_K = 64;
-size_t expm_ws_doubles(int k);
-int launch_expm_standalone(int k, const double* A, int lda, double* E, int lde, int* status, double* ws,
-                           cudaStream_t s);
+int launch_expm_standalone(int k, const double* A, int lda, double* E, int lde, int* status, cudaStream_t s);
 
 struct ControlArgs {
     DevState* st;
@@ -487,9 +485,8 @@ struct ControlArgs {
     mexk_step_t* log;   // attempt log (log_cap entries)
     size_t h_stride = 0;     // batch: state b uses st + b, H + b*h_stride,
     size_t coef_stride = 0;  //        coef + b*coef_stride (no log)
-    double* ws = nullptr;    // expm_ws_doubles(m) doubles of global memory for k > EXPM_SMEM_K
 };
-// One thread block per state (nstates > 1: a batch of independent solves).
+// One thread-block cluster per state (nstates > 1: a batch of independent solves).
 int launch_controller(const ControlArgs& a, int m, cudaStream_t s, int nstates = 1);
 
 // Candidate-step controller: one thread block per candidate step.

@@ -109,7 +109,6 @@ struct mexk_context_s {
     double* d_h2 = nullptr;
     double* d_coef = nullptr;
     double* d_cand = nullptr;
-    double* d_expm_ws = nullptr;  // Pade workspace of the reference controller for m > EXPM_SMEM_K
     float* d_mlp = nullptr;
     float* d_mlp_win = nullptr;  // the network for solves with a window (may be null)
     double* d_partials = nullptr;
@@ -417,7 +416,6 @@ int enqueue_controller(mexk_context_t ctx, int m, int ctrl, mexk_step_t* log, cu
         c.ldh = ctx->ldh;
         c.coef = ctx->d_coef;
         c.log = log;
-        c.ws = ctx->d_expm_ws;
         return launch_controller(c, m, s);
     }
     SearchArgs c;
@@ -738,7 +736,6 @@ int context_csr_finish(mexk_context_t ctx, const int* row_ptr) {
     const size_t hcount = static_cast<size_t>(ctx->ldh) * m_alloc_max;
     if ((rc = dalloc(&ctx->d_H, hcount))) return rc;
     MEXK_CK(cudaMemset(ctx->d_H, 0, sizeof(double) * hcount));
-    if (m_alloc_max > EXPM_SMEM_K && (rc = dalloc(&ctx->d_expm_ws, expm_ws_doubles(m_alloc_max)))) return rc;
     if ((rc = dalloc(&ctx->d_h1, MEXK_M_MAX + 2))) return rc;
     if ((rc = dalloc(&ctx->d_h2, MEXK_M_MAX + 2))) return rc;
     if ((rc = dalloc(&ctx->d_coef, MEXK_M_MAX + 2))) return rc;
@@ -895,7 +892,6 @@ int mexk_context_destroy(mexk_context_t ctx) {
     dfree(ctx->d_h2);
     dfree(ctx->d_coef);
     dfree(ctx->d_cand);
-    dfree(ctx->d_expm_ws);
     dfree(ctx->d_mlp);
     dfree(ctx->d_mlp_win);
     dfree(ctx->d_partials);
