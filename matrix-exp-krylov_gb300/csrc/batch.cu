@@ -40,6 +40,7 @@ struct Wave {
     long long R0 = 0, R1 = 0; // global rows
     int C0 = 0, C1 = 0;      // 64-row chunks
     int t0 = 0, T = 0;       // tiles in the global tile table
+    int n0 = 0, N = 0;       // pieces in the global piece table
     cudaGraphExec_t exec = nullptr;
 };
 
@@ -103,6 +104,12 @@ struct mexk_batch_s {
     int* d_tile_nrows = nullptr;
     int* d_ptile0 = nullptr;
     int* d_ptiles = nullptr;
+    int* d_piece_prob = nullptr;  // pieces of the streaming sweeps
+    long long* d_piece_row0 = nullptr;
+    int* d_piece_nrows = nullptr;
+    int* d_ppiece0 = nullptr;
+    int* d_ppieces = nullptr;
+    double* d_npart = nullptr;
     int tiles_total_cap = 0;
     std::vector<Wave> waves;
     std::vector<DevState> h_init;  // initial states
@@ -118,43 +125,58 @@ namespace {
 
 int P_of(mexk_batch_t b) { return static_cast<int>(b->probs.size()); }
 
-// Tile table of every wave for tile_rows; fills the device arrays.
-int build_tiles(mexk_batch_t b, int tile_rows) {
-    std::vector<int> tprob, tnr, pt0(P_of(b)), ptn(P_of(b));
-    std::vector<long long> trow0;
+// A table of row ranges (every problem cut into ranges of `rows` rows, wave
+// after wave) and where it lives on the device.
+struct RangeTable {
+    int *prob, *nrows, *first, *count;  // per range, per range, per problem, per problem
+    long long* row0;                    // per range
+};
+
+// Fills the device arrays; begin/size: a wave's first range and its ranges.
+int build_ranges(mexk_batch_t b, int rows, const RangeTable& t, int Wave::*begin, int Wave::*size, int cap_wave,
+                 int cap_total) {
+    std::vector<int> prob, nr, first(P_of(b)), count(P_of(b));
+    std::vector<long long> row0;
     for (auto& w : b->waves) {
-        w.t0 = static_cast<int>(tprob.size());
+        w.*begin = static_cast<int>(prob.size());
         for (int p = w.p0; p < w.p1; ++p) {
-            pt0[p] = static_cast<int>(tprob.size()) - w.t0;
+            first[p] = static_cast<int>(prob.size()) - w.*begin;
             const long long r0 = b->prow0[p];
             const long long rp = b->prow0[p + 1] - r0;
             int cnt = 0;
-            for (long long r = 0; r < rp; r += tile_rows) {
-                tprob.push_back(p);
-                trow0.push_back(r0 + r);
-                tnr.push_back(static_cast<int>(std::min<long long>(tile_rows, rp - r)));
+            for (long long r = 0; r < rp; r += rows) {
+                prob.push_back(p);
+                row0.push_back(r0 + r);
+                nr.push_back(static_cast<int>(std::min<long long>(rows, rp - r)));
                 ++cnt;
             }
-            ptn[p] = cnt;
+            count[p] = cnt;
         }
-        w.T = static_cast<int>(tprob.size()) - w.t0;
+        w.*size = static_cast<int>(prob.size()) - w.*begin;
+        if (w.*size > cap_wave) return MEXK_ERR_DEVICE;
     }
-    if (static_cast<int>(tprob.size()) > b->tiles_total_cap) return MEXK_ERR_DEVICE;
-    for (auto& w : b->waves)
-        if (w.T > b->tiles_cap) return MEXK_ERR_DEVICE;
-    MEXK_CK(cudaMemcpy(b->d_tile_prob, tprob.data(), sizeof(int) * tprob.size(), cudaMemcpyHostToDevice));
-    MEXK_CK(cudaMemcpy(b->d_tile_row0, trow0.data(), sizeof(long long) * trow0.size(), cudaMemcpyHostToDevice));
-    MEXK_CK(cudaMemcpy(b->d_tile_nrows, tnr.data(), sizeof(int) * tnr.size(), cudaMemcpyHostToDevice));
-    MEXK_CK(cudaMemcpy(b->d_ptile0, pt0.data(), sizeof(int) * pt0.size(), cudaMemcpyHostToDevice));
-    MEXK_CK(cudaMemcpy(b->d_ptiles, ptn.data(), sizeof(int) * ptn.size(), cudaMemcpyHostToDevice));
-    b->tile_rows = tile_rows;
+    if (static_cast<int>(prob.size()) > cap_total) return MEXK_ERR_DEVICE;
+    MEXK_CK(cudaMemcpy(t.prob, prob.data(), sizeof(int) * prob.size(), cudaMemcpyHostToDevice));
+    MEXK_CK(cudaMemcpy(t.row0, row0.data(), sizeof(long long) * row0.size(), cudaMemcpyHostToDevice));
+    MEXK_CK(cudaMemcpy(t.nrows, nr.data(), sizeof(int) * nr.size(), cudaMemcpyHostToDevice));
+    MEXK_CK(cudaMemcpy(t.first, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice));
+    MEXK_CK(cudaMemcpy(t.count, count.data(), sizeof(int) * count.size(), cudaMemcpyHostToDevice));
     return MEXK_OK;
+}
+
+// Tile table of every wave for tile_rows.
+int build_tiles(mexk_batch_t b, int tile_rows) {
+    const RangeTable t = {b->d_tile_prob, b->d_tile_nrows, b->d_ptile0, b->d_ptiles, b->d_tile_row0};
+    const int rc = build_ranges(b, tile_rows, t, &Wave::t0, &Wave::T, b->tiles_cap, b->tiles_total_cap);
+    if (rc == MEXK_OK) b->tile_rows = tile_rows;
+    return rc;
 }
 
 Layout layout(mexk_batch_t b, const Wave& w) {
     Layout L;
     L.P = w.p1 - w.p0;
     L.T = w.T;
+    L.N = w.N;
     L.C0 = w.C0;
     L.C1 = w.C1;
     L.R0 = w.R0;
@@ -163,6 +185,11 @@ Layout layout(mexk_batch_t b, const Wave& w) {
     L.tile_nrows = b->d_tile_nrows + w.t0;
     L.ptile0 = b->d_ptile0;
     L.ptiles = b->d_ptiles;
+    L.piece_prob = b->d_piece_prob + w.n0;
+    L.piece_row0 = b->d_piece_row0 + w.n0;
+    L.piece_nrows = b->d_piece_nrows + w.n0;
+    L.ppiece0 = b->d_ppiece0;
+    L.ppieces = b->d_ppieces;
     L.chunk_prob = b->d_chunk_prob;
     L.prow0 = b->d_prow0;
     L.row_ptr = b->d_row_ptr;
@@ -183,6 +210,7 @@ Layout layout(mexk_batch_t b, const Wave& w) {
     L.psc = b->d_psc;
     L.coefl = b->d_coefl;
     L.part = b->d_part;
+    L.npart = b->d_npart;
     L.pcount = b->d_pcount;
     L.pdone = b->d_pdone;
     L.active = b->d_active;
@@ -553,18 +581,22 @@ int mexk_batch_upload(mexk_batch_t b) {
     w.p1 = P;
     b->waves.push_back(w);
     long long wave_rows = 0;
-    int tiles_cap = 0, tiles_total = 0;
+    int tiles_cap = 0, tiles_total = 0, pieces_cap = 0, pieces_total = 0;
     for (auto& x : b->waves) {
         x.R0 = b->prow0[x.p0];
         x.R1 = b->prow0[x.p1];
         x.C0 = static_cast<int>(x.R0 / BROWS);
         x.C1 = static_cast<int>(x.R1 / BROWS);
         wave_rows = std::max(wave_rows, x.R1 - x.R0);
-        int tw = 0;  // tiles at the smallest candidate tile size
-        for (int p = x.p0; p < x.p1; ++p)
+        int tw = 0, nw = 0;  // tiles at the smallest candidate tile size, pieces
+        for (int p = x.p0; p < x.p1; ++p) {
             tw += static_cast<int>((b->prow0[p + 1] - b->prow0[p] + TILE_CANDIDATES[0] - 1) / TILE_CANDIDATES[0]);
+            nw += static_cast<int>((b->prow0[p + 1] - b->prow0[p] + PIECE_ROWS - 1) / PIECE_ROWS);
+        }
         tiles_cap = std::max(tiles_cap, tw);
         tiles_total += tw;
+        pieces_cap = std::max(pieces_cap, nw);
+        pieces_total += nw;
     }
     b->wave_rows_cap = wave_rows;
     b->tiles_cap = tiles_cap;
@@ -573,11 +605,16 @@ int mexk_batch_upload(mexk_batch_t b) {
         (rc = dalloc(&b->d_W, static_cast<size_t>(wave_rows) * BR)) ||
         (rc = dalloc(&b->d_part, static_cast<size_t>(tiles_cap) * BPS)) ||
         (rc = dalloc(&b->d_tile_prob, tiles_total)) || (rc = dalloc(&b->d_tile_row0, tiles_total)) ||
-        (rc = dalloc(&b->d_tile_nrows, tiles_total)))
+        (rc = dalloc(&b->d_tile_nrows, tiles_total)) || (rc = dalloc(&b->d_piece_prob, pieces_total)) ||
+        (rc = dalloc(&b->d_piece_row0, pieces_total)) || (rc = dalloc(&b->d_piece_nrows, pieces_total)) ||
+        (rc = dalloc(&b->d_ppiece0, P)) || (rc = dalloc(&b->d_ppieces, P)) ||
+        (rc = dalloc(&b->d_npart, static_cast<size_t>(pieces_cap) * BR)))
         return rc;
     MEXK_CK(cudaMemset(b->d_U, 0, sizeof(float) * static_cast<size_t>(m + 1) * wave_rows * BR));
     MEXK_CK(cudaMemset(b->d_W, 0, sizeof(float) * static_cast<size_t>(wave_rows) * BR));
     if ((rc = build_tiles(b, DEFAULT_TILE_ROWS))) return rc;
+    const RangeTable pieces = {b->d_piece_prob, b->d_piece_nrows, b->d_ppiece0, b->d_ppieces, b->d_piece_row0};
+    if ((rc = build_ranges(b, PIECE_ROWS, pieces, &Wave::n0, &Wave::N, pieces_cap, pieces_total))) return rc;
     b->uploaded = true;
     return MEXK_OK;
 }
@@ -730,6 +767,12 @@ int mexk_batch_destroy(mexk_batch_t b) {
     dfree(b->d_tile_nrows);
     dfree(b->d_ptile0);
     dfree(b->d_ptiles);
+    dfree(b->d_piece_prob);
+    dfree(b->d_piece_row0);
+    dfree(b->d_piece_nrows);
+    dfree(b->d_ppiece0);
+    dfree(b->d_ppieces);
+    dfree(b->d_npart);
     if (b->h_active) cudaFreeHost(b->h_active);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;

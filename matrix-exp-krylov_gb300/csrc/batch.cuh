@@ -32,9 +32,17 @@ constexpr int B_OFF = BR * BM_MAX;         //                     b[c][r]
 constexpr int W_OFF = 2 * BR * BM_MAX;     //                     |w|^2[r] (or |y|^2[r])
 constexpr int BPS = 2 * BR * BM_MAX + BR;  // doubles per tile partial (1040)
 
+// Rows per piece of the streaming sweeps (update, lift, last norms, restart),
+// whatever tile the dot sweep's autotuner picked: with its 16384-row tiles a
+// 380,000-row batch gave those sweeps 30 blocks on 152 SMs (update 255 us a
+// step, 62 us in pieces of 512 rows; the lift 780 and 150 us). A constant, so
+// that the norms' sums do not depend on the wave or the tuner.
+constexpr int PIECE_ROWS = 512;
+
 struct Layout {
     int P;                 // problems in the wave
     int T;                 // tiles of the wave
+    int N;                 // pieces of the wave
     int C0, C1;            // 64-row chunks [C0, C1) of the wave (global chunk index)
     long long R0;          // first global row of the wave (vectors U, W index row - R0)
     const int* tile_prob;  // [T] problem (global index)
@@ -42,6 +50,11 @@ struct Layout {
     const int* tile_nrows;       // [T] rows (multiple of 64)
     const int* ptile0;     // [global problem] first tile of the problem in this wave
     const int* ptiles;     // [global problem] tiles of the problem in this wave
+    const int* piece_prob;        // [N] the pieces, as the tiles
+    const long long* piece_row0;
+    const int* piece_nrows;
+    const int* ppiece0;    // [global problem] first piece of the problem in this wave
+    const int* ppieces;    // [global problem] pieces of the problem
     const int* chunk_prob; // [global chunk] problem
     const long long* prow0;     // [global problem] first global row
     const long long* row_ptr;   // [global rows + 1] CSR over all problems, local columns
@@ -62,6 +75,7 @@ struct Layout {
     float* psc;            // per state
     double* coefl;         // per state BLD lift coefficients (from the controller)
     double* part;          // [T][BPS]
+    double* npart;         // [N][16] the pieces' sums of squares
     unsigned int* pcount;  // [global problem] arrival counters
     int* pdone;            // [global problem] every state of the problem finished
     int* active;           // states still running after the cycle (one int)

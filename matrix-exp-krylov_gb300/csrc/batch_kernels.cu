@@ -328,8 +328,8 @@ __global__ void __launch_bounds__(BT) update_kernel(Layout L, int j) {
     __shared__ float4 ssc[2][4];
     const float4* __restrict__ W4 = reinterpret_cast<const float4*>(L.W);
     float4* __restrict__ Out = reinterpret_cast<float4*>(L.U + static_cast<size_t>(j + 1) * L.ldu);
-    for (int tile = blockIdx.x; tile < L.T; tile += gridDim.x) {
-        const int p = L.tile_prob[tile];
+    for (int piece = blockIdx.x; piece < L.N; piece += gridDim.x) {
+        const int p = L.piece_prob[piece];
         if (L.pdone[p]) continue;
         __syncthreads();
         for (int v = threadIdx.x; v < BM_MAX * BR; v += BT) {
@@ -344,8 +344,8 @@ __global__ void __launch_bounds__(BT) update_kernel(Layout L, int j) {
         __syncthreads();
         const float4 wsc = ssc[0][q];
         const float4 psc = ssc[1][q];
-        const long long base = L.tile_row0[tile] - L.R0;
-        const int nr = L.tile_nrows[tile];
+        const long long base = L.piece_row0[piece] - L.R0;
+        const int nr = L.piece_nrows[piece];
         for (int r = rl; r < nr; r += BROWS) {
             const size_t i = static_cast<size_t>(base + r) * 4 + q;
             const float4 x = __ldg(W4 + i);
@@ -371,9 +371,9 @@ __global__ void __launch_bounds__(BT) update_kernel(Layout L, int j) {
 }
 
 // ---------------------------------------------------------------- per-RHS norms
-// Writes the 16 per-RHS sums of a block (acc per thread, FP64) to slot
-// W_OFF of the tile partial.
-__device__ __forceinline__ void tile_rhs_partial(const Layout& L, int tile, const double (&acc)[4]) {
+// Writes the 16 per-RHS sums of a block (acc per thread, FP64) to the
+// piece's partial.
+__device__ __forceinline__ void piece_rhs_partial(const Layout& L, int piece, const double (&acc)[4]) {
     __shared__ double red[BT / 32][BR];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -389,19 +389,31 @@ __device__ __forceinline__ void tile_rhs_partial(const Layout& L, int tile, cons
         double s = 0.0;
 #pragma unroll
         for (int w = 0; w < BT / 32; ++w) s += red[w][threadIdx.x];
-        L.part[static_cast<size_t>(tile) * BPS + W_OFF + threadIdx.x] = s;
+        L.npart[static_cast<size_t>(piece) * BR + threadIdx.x] = s;
     }
+}
+
+// Sum of right-hand side r's partials over the pieces of problem p: the 16
+// lanes of a half warp take every 16th piece, then a butterfly. (Half warp r
+// of the block's 16; every thread calls it; the sum is in all 16 lanes.)
+__device__ __forceinline__ double pieces_sum(const Layout& L, int p) {
+    const int r = threadIdx.x >> 4, l = threadIdx.x & 15;
+    const int t0 = L.ppiece0[p], nt = L.ppieces[p];
+    double t = 0.0;
+    for (int tt = l; tt < nt; tt += 16) t += __ldcg(&L.npart[static_cast<size_t>(t0 + tt) * BR + r]);
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(FULL, t, o);
+    return t;
 }
 
 // |u_{j+1}|^2 per state after the last step: H(j+1, j), s_{j+1}, breakdown.
 __global__ void __launch_bounds__(BT) norm_last_kernel(Layout L, int j) {
-    const int tile = blockIdx.x;
-    const int p = L.tile_prob[tile];
+    const int piece = blockIdx.x;
+    const int p = L.piece_prob[piece];
     if (L.pdone[p]) return;
     const int q = threadIdx.x & 3;
     const int rl = threadIdx.x >> 2;
-    const long long base = L.tile_row0[tile] - L.R0;
-    const int nr = L.tile_nrows[tile];
+    const long long base = L.piece_row0[piece] - L.R0;
+    const int nr = L.piece_nrows[piece];
     const float4* __restrict__ Un = col4(L, j + 1);
     float4 a = zero4();
     for (int r = rl; r < nr; r += BROWS) {
@@ -409,14 +421,15 @@ __global__ void __launch_bounds__(BT) norm_last_kernel(Layout L, int j) {
         fma4(a, u, u);
     }
     const double acc[4] = {a.x, a.y, a.z, a.w};
-    tile_rhs_partial(L, tile, acc);
+    piece_rhs_partial(L, piece, acc);
     __shared__ int s_flag;
-    if (!problem_last(L.pcount + p, static_cast<unsigned>(L.ptiles[p]), &s_flag)) return;
-    if (threadIdx.x < BR) {
-        const int b = p * BR + threadIdx.x;
+    if (!problem_last(L.pcount + p, static_cast<unsigned>(L.ppieces[p]), &s_flag)) return;
+    static_assert(BT == 16 * BR, "a half warp per right-hand side");
+    const double nb = pieces_sum(L, p);
+    if ((threadIdx.x & 15) == 0) {
+        const int b = p * BR + (threadIdx.x >> 4);
         DevState* st = L.st + b;
         if (st->done || st->breakdown) return;
-        const double nb = tiles_sum(L, p, W_OFF + threadIdx.x);
         double* pv = L.pre + static_cast<size_t>(b) * (BLD + 1);
         const double beta = sqrt(nb) / pv[j + 1];
         const bool bad = !(beta >= 1e-14) || isinf(beta);
@@ -435,8 +448,8 @@ __global__ void __launch_bounds__(BT) norm_last_kernel(Layout L, int j) {
 // products, compensated FP32 sums, FP64 result), and |y|.
 // Then, per state, the restart scale 1/|y| (main.cu:2023-2073).
 __global__ void __launch_bounds__(BT) lift_kernel(Layout L, int kmax, int start) {
-    const int tile = blockIdx.x;
-    const int p = L.tile_prob[tile];
+    const int piece = blockIdx.x;
+    const int p = L.piece_prob[piece];
     if (L.pdone[p]) return;
     __shared__ float4 scl[BM_MAX][4];
     __shared__ int smask[BR];
@@ -462,9 +475,9 @@ __global__ void __launch_bounds__(BT) lift_kernel(Layout L, int kmax, int start)
     const int rl = threadIdx.x >> 2;
     const bool m0 = smask[4 * q] != 0, m1 = smask[4 * q + 1] != 0, m2 = smask[4 * q + 2] != 0,
                m3 = smask[4 * q + 3] != 0;
-    const long long grow = L.tile_row0[tile];
+    const long long grow = L.piece_row0[piece];
     const long long base = grow - L.R0;
-    const int nr = L.tile_nrows[tile];
+    const int nr = L.piece_nrows[piece];
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (int r = rl; r < nr; r += BROWS) {
         double2* y2 = reinterpret_cast<double2*>(L.Y + static_cast<size_t>(grow + r) * BR + 4 * q);
@@ -510,12 +523,13 @@ __global__ void __launch_bounds__(BT) lift_kernel(Layout L, int kmax, int start)
         if (m2) acc[2] = fma(y[2], y[2], acc[2]);
         if (m3) acc[3] = fma(y[3], y[3], acc[3]);
     }
-    tile_rhs_partial(L, tile, acc);
+    piece_rhs_partial(L, piece, acc);
     __shared__ int s_flag;
-    if (!problem_last(L.pcount + p, static_cast<unsigned>(L.ptiles[p]), &s_flag)) return;
-    if (threadIdx.x < BR && smask[threadIdx.x]) {
-        DevState* st = L.st + p * BR + threadIdx.x;
-        const double nrm = sqrt(tiles_sum(L, p, W_OFF + threadIdx.x));
+    if (!problem_last(L.pcount + p, static_cast<unsigned>(L.ppieces[p]), &s_flag)) return;
+    const double n2 = pieces_sum(L, p);
+    if ((threadIdx.x & 15) == 0 && smask[threadIdx.x >> 4]) {
+        DevState* st = L.st + p * BR + (threadIdx.x >> 4);
+        const double nrm = sqrt(n2);
         st->restart_scale = nrm > 1e-14 ? 1.0 / nrm : 1.0;
         // FP32 bases do not resolve errors below their rounding of the iterate:
         // a step also passes below it while the accepted errors stay within
@@ -539,8 +553,8 @@ __global__ void __launch_bounds__(BT) restart_kernel(Layout L, int from_start) {
     const int q = threadIdx.x & 3;
     const int rl = threadIdx.x >> 2;
     float4* __restrict__ U0 = reinterpret_cast<float4*>(L.U);
-    for (int tile = blockIdx.x; tile < L.T; tile += gridDim.x) {
-        const int p = L.tile_prob[tile];
+    for (int piece = blockIdx.x; piece < L.N; piece += gridDim.x) {
+        const int p = L.piece_prob[piece];
         if (L.pdone[p]) continue;
         __syncthreads();
         if (threadIdx.x < BR) {
@@ -549,9 +563,9 @@ __global__ void __launch_bounds__(BT) restart_kernel(Layout L, int from_start) {
         }
         __syncthreads();
         const float4 sc = *reinterpret_cast<const float4*>(&ssc[4 * q]);
-        const long long grow = L.tile_row0[tile];
+        const long long grow = L.piece_row0[piece];
         const long long base = grow - L.R0;
-        const int nr = L.tile_nrows[tile];
+        const int nr = L.piece_nrows[piece];
         for (int r = rl; r < nr; r += BROWS) {
             const double* src = from_start ? L.V0 : L.Y;
             const double2* y2 = reinterpret_cast<const double2*>(src + static_cast<size_t>(grow + r) * BR + 4 * q);
@@ -599,7 +613,7 @@ int launch_dot(const Layout& L, int j, int reortho, int gg, int tune, cudaStream
 
 int launch_update(const Layout& L, int j, cudaStream_t s) {
     if (j < 0 || j >= BM_MAX || L.T <= 0) return L.T <= 0 ? MEXK_OK : MEXK_ERR_INVALID;
-    const int grid = L.T < sm_blocks(4) ? L.T : sm_blocks(4);
+    const int grid = L.N < sm_blocks(4) ? L.N : sm_blocks(4);
     update_kernel<<<grid, BT, 0, s>>>(L, j);
     MEXK_CK_LAUNCH("batch update_kernel");
     return MEXK_OK;
@@ -607,7 +621,7 @@ int launch_update(const Layout& L, int j, cudaStream_t s) {
 
 int launch_norm_last(const Layout& L, int j, cudaStream_t s) {
     if (j < 0 || j >= BM_MAX || L.T <= 0) return L.T <= 0 ? MEXK_OK : MEXK_ERR_INVALID;
-    norm_last_kernel<<<L.T, BT, 0, s>>>(L, j);
+    norm_last_kernel<<<L.N, BT, 0, s>>>(L, j);
     MEXK_CK_LAUNCH("batch norm_last_kernel");
     return MEXK_OK;
 }
@@ -615,14 +629,14 @@ int launch_norm_last(const Layout& L, int j, cudaStream_t s) {
 int launch_lift(const Layout& L, int k_max, int start, cudaStream_t s) {
     if (L.T <= 0) return MEXK_OK;
     if (k_max < 0 || k_max > BM_MAX) return MEXK_ERR_INVALID;
-    lift_kernel<<<L.T, BT, 0, s>>>(L, k_max, start);
+    lift_kernel<<<L.N, BT, 0, s>>>(L, k_max, start);
     MEXK_CK_LAUNCH("batch lift_kernel");
     return MEXK_OK;
 }
 
 int launch_restart(const Layout& L, int from_start, cudaStream_t s) {
     if (L.T <= 0) return MEXK_OK;
-    const int grid = L.T < sm_blocks(4) ? L.T : sm_blocks(4);
+    const int grid = L.N < sm_blocks(4) ? L.N : sm_blocks(4);
     restart_kernel<<<grid, BT, 0, s>>>(L, from_start);
     MEXK_CK_LAUNCH("batch restart_kernel");
     return MEXK_OK;
