@@ -357,6 +357,9 @@ int mexk_batch_upload(mexk_batch_t b);
 int mexk_batch_run(mexk_batch_t b);
 /* Y: rows x nrhs row-major; results: nrhs entries (may be null). */
 int mexk_batch_result(mexk_batch_t b, int problem, double* Y, mexk_result_t* results);
+/* The same with Y nrhs x rows, row-major (one right-hand side after another):
+ * transposed on the device and copied straight into Y. */
+int mexk_batch_result_columns(mexk_batch_t b, int problem, double* Y, mexk_result_t* results);
 int mexk_batch_info(mexk_batch_t b, mexk_batch_info_t* info);
 /* Times `iters` launches of one per-step kernel of the first wave at step j
  * with the schedule in use (after a run): kind 0 SpMM, 1 dot sweep (timing

@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -110,6 +111,9 @@ struct mexk_batch_s {
     int* d_ppiece0 = nullptr;
     int* d_ppieces = nullptr;
     double* d_npart = nullptr;
+    double* d_cols = nullptr;  // a problem's results transposed (mexk_batch_result_columns), once asked for
+    size_t cols_cap = 0;
+    std::mutex cols_mutex;  // results of one batch may be fetched by several threads
     int tiles_total_cap = 0;
     std::vector<Wave> waves;
     std::vector<DevState> h_init;  // initial states
@@ -663,30 +667,58 @@ int mexk_batch_run(mexk_batch_t b) {
     return MEXK_OK;
 }
 
+static void fill_results(mexk_batch_t b, int problem, mexk_result_t* results) {
+    for (int r = 0; r < b->probs[problem].nrhs; ++r) {
+        const DevState& st = b->h_final[static_cast<size_t>(problem) * BR + r];
+        mexk_result_t& o = results[r];
+        o.converged = st.converged;
+        o.restarts_done = st.accepted;
+        o.last_residual = st.last_residual;
+        o.attempts = st.attempts;
+        o.cycles = st.cycles;
+        o.spmv_count = st.spmv_count;
+        o.t_done = st.t_done;
+        o.status = st.status;
+    }
+}
+
 int mexk_batch_result(mexk_batch_t b, int problem, double* Y, mexk_result_t* results) {
     if (!b || !b->uploaded || problem < 0 || problem >= P_of(b) || !Y) return MEXK_ERR_INVALID;
     if (!b->have_final) return MEXK_ERR_NOT_READY;
     MEXK_CK(cudaSetDevice(b->device));
     const HostProblem& q = b->probs[problem];
-    std::vector<double> tmp(static_cast<size_t>(q.rows) * BR);
-    MEXK_CK(cudaMemcpy(tmp.data(), b->d_Y + b->prow0[problem] * BR, sizeof(double) * tmp.size(),
-                       cudaMemcpyDeviceToHost));
-    for (int i = 0; i < q.rows; ++i)
-        for (int r = 0; r < q.nrhs; ++r) Y[static_cast<size_t>(i) * q.nrhs + r] = tmp[static_cast<size_t>(i) * BR + r];
-    if (results) {
-        for (int r = 0; r < q.nrhs; ++r) {
-            const DevState& st = b->h_final[static_cast<size_t>(problem) * BR + r];
-            mexk_result_t& o = results[r];
-            o.converged = st.converged;
-            o.restarts_done = st.accepted;
-            o.last_residual = st.last_residual;
-            o.attempts = st.attempts;
-            o.cycles = st.cycles;
-            o.spmv_count = st.spmv_count;
-            o.t_done = st.t_done;
-            o.status = st.status;
-        }
+    const double* src = b->d_Y + b->prow0[problem] * BR;
+    if (q.nrhs == BR) {  // the device layout is Y's
+        MEXK_CK(cudaMemcpy(Y, src, sizeof(double) * static_cast<size_t>(q.rows) * BR, cudaMemcpyDeviceToHost));
+    } else {
+        std::vector<double> tmp(static_cast<size_t>(q.rows) * BR);
+        MEXK_CK(cudaMemcpy(tmp.data(), src, sizeof(double) * tmp.size(), cudaMemcpyDeviceToHost));
+        for (int i = 0; i < q.rows; ++i)
+            for (int r = 0; r < q.nrhs; ++r)
+                Y[static_cast<size_t>(i) * q.nrhs + r] = tmp[static_cast<size_t>(i) * BR + r];
     }
+    if (results) fill_results(b, problem, results);
+    return MEXK_OK;
+}
+
+int mexk_batch_result_columns(mexk_batch_t b, int problem, double* Y, mexk_result_t* results) {
+    if (!b || !b->uploaded || problem < 0 || problem >= P_of(b) || !Y) return MEXK_ERR_INVALID;
+    if (!b->have_final) return MEXK_ERR_NOT_READY;
+    MEXK_CK(cudaSetDevice(b->device));
+    const HostProblem& q = b->probs[problem];
+    const size_t count = static_cast<size_t>(q.rows) * q.nrhs;
+    const std::lock_guard<std::mutex> lock(b->cols_mutex);
+    int rc;
+    if (count > b->cols_cap) {
+        dfree(b->d_cols);
+        b->cols_cap = 0;
+        if ((rc = dalloc(&b->d_cols, count))) return rc;
+        b->cols_cap = count;
+    }
+    if ((rc = launch_columns(b->d_Y + b->prow0[problem] * BR, q.rows, q.nrhs, b->d_cols, b->stream))) return rc;
+    MEXK_CK(cudaMemcpyAsync(Y, b->d_cols, sizeof(double) * count, cudaMemcpyDeviceToHost, b->stream));
+    MEXK_CK(cudaStreamSynchronize(b->stream));
+    if (results) fill_results(b, problem, results);
     return MEXK_OK;
 }
 
@@ -773,6 +805,7 @@ int mexk_batch_destroy(mexk_batch_t b) {
     dfree(b->d_ppiece0);
     dfree(b->d_ppieces);
     dfree(b->d_npart);
+    dfree(b->d_cols);
     if (b->h_active) cudaFreeHost(b->h_active);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;

@@ -92,6 +92,8 @@ int launch_lift(const Layout& L, int k_max, int start, cudaStream_t s);
 // from_start: u_0 from the start vectors V0, else from the lifted Y.
 int launch_restart(const Layout& L, int from_start, cudaStream_t s);
 int launch_status(const Layout& L, int p0, int p1, cudaStream_t s);
+// out[r * rows + i] = Y[i * 16 + r] for r < nrhs, i < rows.
+int launch_columns(const double* Y, long long rows, int nrhs, double* out, cudaStream_t s);
 
 }  // namespace batch
 }  // namespace mexk

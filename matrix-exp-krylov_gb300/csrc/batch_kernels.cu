@@ -588,6 +588,23 @@ __global__ void status_kernel(Layout L, int p0, int p1) {
     if (running) atomicAdd(L.active, running);
 }
 
+// 64 rows x 16 right-hand sides per block through shared memory: 128-byte
+// rows in, runs of 64 rows out.
+__global__ void __launch_bounds__(BT) columns_kernel(const double* __restrict__ Y, long long rows, int nrhs,
+                                                     double* __restrict__ out) {
+    __shared__ double t[BROWS][BR + 1];
+    const long long r0 = static_cast<long long>(blockIdx.x) * BROWS;
+    for (int e = threadIdx.x; e < BROWS * BR; e += BT) {
+        const long long i = r0 + e / BR;
+        t[e / BR][e % BR] = i < rows ? __ldcs(Y + i * BR + e % BR) : 0.0;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < BROWS * nrhs; e += BT) {
+        const long long i = r0 + e % BROWS;
+        if (i < rows) out[static_cast<long long>(e / BROWS) * rows + i] = t[e % BROWS][e / BROWS];
+    }
+}
+
 int sm_blocks(int per_sm) { return device_sm_count() * per_sm; }
 
 }  // namespace
@@ -646,6 +663,13 @@ int launch_status(const Layout& L, int p0, int p1, cudaStream_t s) {
     if (p1 <= p0) return MEXK_OK;
     status_kernel<<<(p1 - p0 + 255) / 256, 256, 0, s>>>(L, p0, p1);
     MEXK_CK_LAUNCH("batch status_kernel");
+    return MEXK_OK;
+}
+
+int launch_columns(const double* Y, long long rows, int nrhs, double* out, cudaStream_t s) {
+    if (rows <= 0 || nrhs < 1 || nrhs > BR) return MEXK_ERR_INVALID;
+    columns_kernel<<<static_cast<unsigned>((rows + BROWS - 1) / BROWS), BT, 0, s>>>(Y, rows, nrhs, out);
+    MEXK_CK_LAUNCH("batch columns_kernel");
     return MEXK_OK;
 }
 

@@ -331,6 +331,21 @@ struct ClusterExpm {
             }
         }
         __syncthreads();
+        if (nj > 8) {
+            // many own columns (a small cluster): row by row, each row's
+            // divisions in one warp's lanes -- a division costs a warp the
+            // same with one lane active as with 32
+            for (int i = k - 1; i >= 0; --i) {
+                for (int q = threadIdx.x; q < nj; q += blockDim.x) B[i + q * k] /= L[i + i * k];
+                __syncthreads();
+                for (int e = threadIdx.x; e < i * nj; e += blockDim.x) {
+                    const int l = e % i, q = e / i;
+                    B[l + q * k] -= L[l + i * k] * B[i + q * k];
+                }
+                __syncthreads();
+            }
+            return;
+        }
         for (int q = warp; q < nj; q += nw) {
             double* col = B + static_cast<size_t>(q) * k;
             double x[U];

@@ -103,6 +103,7 @@ _PROTOS = {
     "mexk_batch_upload": ([C.c_void_p], C.c_int),
     "mexk_batch_run": ([C.c_void_p], C.c_int),
     "mexk_batch_result": ([C.c_void_p, C.c_int, C.POINTER(C.c_double), C.POINTER(Result)], C.c_int),
+    "mexk_batch_result_columns": ([C.c_void_p, C.c_int, C.POINTER(C.c_double), C.POINTER(Result)], C.c_int),
     "mexk_batch_info": ([C.c_void_p, C.POINTER(BatchInfo)], C.c_int),
     "mexk_batch_destroy": ([C.c_void_p], C.c_int),
     "mexk_batch_profile": ([C.c_void_p, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_double),

@@ -58,10 +58,10 @@ class Batch:
 
     def result(self, index: int):
         n, nrhs = self._shapes[index]
-        Y = np.zeros((n, nrhs))
+        Y = np.empty((nrhs, n))
         res = (Result * nrhs)()
-        check(lib().mexk_batch_result(self._h, index, _ptr(Y, C.c_double), res), "mexk_batch_result")
-        return np.ascontiguousarray(Y.T), [r.as_dict() for r in res]
+        check(lib().mexk_batch_result_columns(self._h, index, _ptr(Y, C.c_double), res), "mexk_batch_result_columns")
+        return Y, [r.as_dict() for r in res]
 
     def info(self) -> dict:
         i = BatchInfo()
