@@ -442,11 +442,13 @@ int mexk_context_set_lanczos_form(mexk_context_t ctx, int form);
 /* enable != 0: from now on, thread block 0 of the staged CSR SpMV also waits
  * (1 ms limit) on a barrier that nothing arrives at, so its bounded wait runs
  * out: it drains its bulk copies in flight and sets the timeout status bit;
- * and thread block 0 of the fused Lanczos cycle leaves before its first grid
- * barrier, so the other blocks' bounded waits (1 s) run out. Either way the
- * solve returns MEXK_ERR_DEVICE and the context stays usable. enable = 0
+ * thread block 0 of an FP64 basis built by a cooperative grid (more than 4096
+ * rows) waits 1 ms for an arrival that never comes, raises the status bit and
+ * the abort word, and the others leave; and thread block 0 of the fused
+ * Lanczos cycle leaves before its first grid barrier, so the other blocks'
+ * bounded waits (1 s) run out. Each way the solve returns MEXK_ERR_DEVICE and the context stays usable. enable = 0
  * restores normal operation. For failure-path tests only: it changes no
- * result of a solve that uses neither form. No reference counterpart (the
+ * result of a solve that uses none of them. No reference counterpart (the
  * reference has no bounded device waits). */
 int mexk_test_force_wait_timeout(int device, int enable);
 

@@ -388,6 +388,49 @@ template <typename TV>
 int launch_normalize(int n, int j, int ldv, const TV* w, TV* V, const DevState* st,
                      const double* inv_beta, cudaStream_t s);
 
+// All m steps of an FP64 basis in one launch (arnoldi_cycle.cu): V[:,0] given,
+// columns 1..m, H and the breakdown state written as launch_gs_step and
+// launch_normalize leave them. x: n doubles of scratch; bar: four words, and
+// words: CYCLE_WORDS, zero before a context's first launch (and after one
+// that gave up). scale: 2^scale bounds |A x| for |x| = 1. Steps j0..j1-1 run,
+// with their products (product != 0) or, for one step, from x = A v_j0.
+// rows, scale_gather: set by the launch.
+constexpr int CYCLE_DIGITS = 8;        // words per column of an exchange
+constexpr int CYCLE_EXCHANGE = MEXK_M_MAX * CYCLE_DIGITS + 2;
+constexpr int CYCLE_MAX_BLOCKS = 256;
+constexpr int CYCLE_WORDS = 4 * CYCLE_EXCHANGE + CYCLE_MAX_BLOCKS;
+constexpr int CYCLE_ROWS_MAX = 2000000;
+struct CycleArgs {
+    int n, m, ldv, ldh, reortho, window;
+    int j0, j1, product;
+    int rows = 0, scale_gather = 0;
+    int scale;
+    int max_len;         // of the row patterns
+    long long nnz;
+    const int* row_ptr;
+    const int* col_idx;
+    const double* values;
+    const uint8_t* pid;  // the row-pattern form, or null: the CSR arrays
+    const RowPatterns* T;
+    double* V;
+    double* x;
+    double* H;
+    DevState* st;
+    unsigned* bar;
+    unsigned long long* words;
+};
+// out (device, zero before the call): the bits of a bound of the largest row
+// sum of |values|, and the entries of the longest row.
+int launch_row_bounds(int n, const int* row_ptr, const double* values, unsigned long long* out, cudaStream_t s);
+bool arnoldi_cycle_fits(int n);
+// Whether the launch also takes the products (else one launch per step after
+// the context's SpMV).
+bool arnoldi_cycle_product(int n, long long nnz, int max_row, bool pattern);
+int arnoldi_cycle_prepare();
+int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s);
+// mexk_test_force_wait_timeout's part (current device).
+int arnoldi_cycle_test_hook(int enable);
+
 // ------------------------------------------------------------ Gram-corrected sweeps (FP32 basis)
 // Column c of the FP32 basis stores u_c; the basis vector is v_c = s[c] * u_c.
 constexpr int GRAM_M = MEXK_M_MAX_MIXED;    // largest Krylov dimension of the FP32 basis

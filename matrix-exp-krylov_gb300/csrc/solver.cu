@@ -32,6 +32,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -58,6 +59,8 @@ struct NvtxRange {
 };
 
 constexpr int PARTIAL_BLOCKS = 4096;
+constexpr int BAR_WORDS = 4;  // grid-barrier words; the one-launch basis's sums follow them
+constexpr size_t BAR_BYTES = sizeof(unsigned int) * BAR_WORDS + sizeof(unsigned long long) * CYCLE_WORDS;
 constexpr int LOG_CAP = 8192;
 
 }  // namespace mexk
@@ -89,6 +92,8 @@ struct mexk_context_s {
     int4* d_tiles = nullptr;
     uint16_t* d_col16 = nullptr;
     bool spmv_narrow = false;  // every staged SpMV row block has 16-bit columns
+    int max_row = 0;           // entries of the longest row
+    int cycle_scale = 0;       // 2^cycle_scale bounds |A x|, |x| = 1 (INT_MAX: no finite bound)
     // The SpMV form per precision (MEXK_SPMV_*): the row-pattern form when
     // every row is one of at most PAT_MAX patterns, else direct (one block per
     // row block) when some row block's columns span 65,536 or more, else staged.
@@ -462,6 +467,48 @@ int enqueue_lanczos_cycle(mexk_context_t ctx, int m, int reortho, cudaStream_t s
     return launch_lanczos_cycle(a, s);
 }
 
+// Whether an FP64 basis is built by arnoldi_cycle.cu: in one launch with its
+// products, or in one launch per step after the SpMV.
+bool use_arnoldi_cycle(mexk_context_t ctx) {
+    return ctx->cycle_scale != INT_MAX && arnoldi_cycle_fits(ctx->n);
+}
+
+int enqueue_arnoldi_cycle(mexk_context_t ctx, int m, int reortho, int window, cudaStream_t s) {
+    CycleArgs a;
+    a.n = ctx->n;
+    a.m = m;
+    a.ldv = ctx->ldv;
+    a.ldh = ctx->ldh;
+    a.reortho = reortho ? 1 : 0;
+    a.window = window;
+    a.nnz = ctx->nnz;
+    a.row_ptr = ctx->d_row_ptr;
+    a.col_idx = ctx->d_col;
+    a.values = ctx->d_val;
+    a.pid = ctx->spmv_form64 == MEXK_SPMV_PATTERN ? ctx->d_pid : nullptr;
+    a.T = ctx->d_pat;
+    a.V = ctx->d_V;
+    a.x = ctx->d_w;
+    a.H = ctx->d_H;
+    a.st = ctx->d_state;
+    a.bar = ctx->d_bar;
+    a.words = reinterpret_cast<unsigned long long*>(ctx->d_bar + BAR_WORDS);
+    a.scale = ctx->cycle_scale;
+    a.max_len = ctx->pat_max_len;
+    a.product = arnoldi_cycle_product(ctx->n, ctx->nnz, ctx->max_row, a.pid != nullptr) ? 1 : 0;
+    a.j0 = 0;
+    a.j1 = m;
+    if (a.product) return launch_arnoldi_cycle(a, s);
+    for (int j = 0; j < m; ++j) {
+        int rc;
+        if ((rc = context_spmv(ctx, j, false, &ctx->d_state->breakdown, s))) return rc;
+        a.j0 = j;
+        a.j1 = j + 1;
+        if ((rc = launch_arnoldi_cycle(a, s))) return rc;
+    }
+    return MEXK_OK;
+}
+
 // One Krylov cycle: the unit that is captured into a graph.
 template <typename TV>
 int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, cudaStream_t s) {
@@ -472,7 +519,9 @@ int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, 
     if (!fp32 && window > 0)
         MEXK_CK(cudaMemsetAsync(ctx->d_H, 0, sizeof(double) * static_cast<size_t>(ctx->ldh) * m, s));
     const bool fused = use_lanczos_cycle(ctx, m, fp32, window);
-    if (fused) {
+    if (!fp32 && use_arnoldi_cycle(ctx)) {
+        if ((rc = enqueue_arnoldi_cycle(ctx, m, reortho, window, s))) return rc;
+    } else if (fused) {
         // step 0 as two kernels (its update writes step 1's b and a_0 partials), then the rest in one launch
         if ((rc = enqueue_step(ctx, 0, reortho, fp32, s, window, m))) return rc;
         if ((rc = enqueue_lanczos_cycle(ctx, m, reortho, s))) return rc;
@@ -596,7 +645,7 @@ int solve(mexk_context_t ctx, const mexk_params_t* p, const double* v_dev, doubl
     ctx->last_controller = p->controller;
     init_state(ctx->h_state, p, LOG_CAP);
     MEXK_CK(cudaMemcpyAsync(ctx->d_state, ctx->h_state, sizeof(DevState), cudaMemcpyHostToDevice, s));
-    MEXK_CK(cudaMemsetAsync(ctx->d_bar, 0, sizeof(unsigned int) * 4, s));
+    MEXK_CK(cudaMemsetAsync(ctx->d_bar, 0, BAR_BYTES, s));
     if (ctx->h_state->done) {
         // The reference never lifts when no step runs: y stays zero (main_cpu.cpp:467).
         MEXK_CK(cudaMemsetAsync(ctx->d_y, 0, sizeof(double) * ctx->n, s));
@@ -743,8 +792,14 @@ int context_csr_finish(mexk_context_t ctx, const int* row_ptr) {
     if ((rc = dalloc(&ctx->d_partials, static_cast<size_t>(PARTIAL_BLOCKS) * RED_STRIDE))) return rc;
     if ((rc = dalloc(&ctx->d_counter, 4))) return rc;
     MEXK_CK(cudaMemset(ctx->d_counter, 0, sizeof(unsigned int) * 4));
-    if ((rc = dalloc(&ctx->d_bar, 4))) return rc;
-    MEXK_CK(cudaMemset(ctx->d_bar, 0, sizeof(unsigned int) * 4));
+    if ((rc = dalloc(&ctx->d_bar, BAR_BYTES / sizeof(unsigned int)))) return rc;
+    MEXK_CK(cudaMemsetAsync(ctx->d_bar, 0, BAR_BYTES, ctx->stream));
+    // bounds of A's rows, read back with the pattern detection's flags (the
+    // words are cleared again before each solve)
+    unsigned long long* const d_bounds = reinterpret_cast<unsigned long long*>(ctx->d_bar + BAR_WORDS);
+    if ((rc = launch_row_bounds(ctx->n, ctx->d_row_ptr, ctx->d_val, d_bounds, ctx->stream))) return rc;
+    unsigned long long bounds[2] = {0, 0};
+    MEXK_CK(cudaMemcpyAsync(bounds, d_bounds, sizeof(bounds), cudaMemcpyDeviceToHost, ctx->stream));
     if ((rc = dalloc(&ctx->d_state, 1))) return rc;
     if ((rc = dalloc(&ctx->d_log, LOG_CAP))) return rc;
     cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&ctx->h_state), sizeof(DevState));
@@ -769,6 +824,18 @@ int context_csr_finish(mexk_context_t ctx, const int* row_ptr) {
         return rc;
     MEXK_CK(cudaMemsetAsync(&ctx->d_state->status, 0, sizeof(int), ctx->stream));
     MEXK_CK(cudaStreamSynchronize(ctx->stream));
+    {
+        // |A x|_2 <= sqrt(n) |A x|_inf <= sqrt(n) |A|_inf for |x|_2 = 1
+        double norm;
+        memcpy(&norm, &bounds[0], sizeof(norm));
+        ctx->max_row = static_cast<int>(bounds[1]);
+        ctx->cycle_scale = INT_MAX;
+        if (norm <= 1e300) {
+            int e = 0;
+            (void)frexp(std::max(norm, 1e-300) * std::sqrt(static_cast<double>(ctx->n)), &e);
+            ctx->cycle_scale = e + 1;  // and w - V h1 stays within twice |w|
+        }
+    }
     if (pat_ok) {
         ctx->spmv_form64 = MEXK_SPMV_PATTERN;
     } else {
@@ -828,6 +895,7 @@ int mexk_context_create(int device, mexk_context_t* out) {
     int rc = expm_init_attributes();
     // without its shared memory the fused Lanczos form stays off (lanczos_cycle_fits says no)
     if (rc == MEXK_OK && lanczos_cycle_prepare() != MEXK_OK) (void)cudaGetLastError();
+    if (rc == MEXK_OK) rc = arnoldi_cycle_prepare();
     gs_prepare();
     if (rc) {
         cudaStreamDestroy(c->stream);

@@ -857,6 +857,42 @@ __global__ void symmetric_check_kernel(int n, const int* __restrict__ row_ptr, c
     }
 }
 
+// out[0]: the largest row sum of magnitudes, as the bits of a non-negative
+// double (whose order is the integers'); a row with a NaN counts as infinite.
+// out[1]: the longest row. Four lanes per row.
+__global__ void row_bounds_kernel(int n, const int* __restrict__ row_ptr, const double* __restrict__ values,
+                                  unsigned long long* out) {
+    const int sub = threadIdx.x & 3;
+    double m = 0.0;
+    int len = 0;
+    const int nw = (n + 7) & ~7;  // whole warps run every iteration
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; r < nw; r += (gridDim.x * blockDim.x) >> 2) {
+        const int e0 = r < n ? row_ptr[r] : 0, e1 = r < n ? row_ptr[r + 1] : 0;
+        len = max(len, e1 - e0);
+        float s = 0.f;  // rounded up: a bound is wanted, and FP32 adds are cheap here
+        for (int e = e0 + sub; e < e1; e += 4) s = __fadd_ru(s, __double2float_ru(fabs(values[e])));
+        s = __fadd_ru(s, __shfl_xor_sync(0xffffffffu, s, 1));
+        s = __fadd_ru(s, __shfl_xor_sync(0xffffffffu, s, 2));
+        const double d = s == s ? static_cast<double>(s) : static_cast<double>(INFINITY);
+        if (d > m) m = d;
+    }
+    unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(m));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) u = max(u, __shfl_xor_sync(0xffffffffu, u, o));
+    len = __reduce_max_sync(0xffffffffu, len);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(out, u);
+        atomicMax(out + 1, static_cast<unsigned long long>(len));
+    }
+}
+
+int launch_row_bounds(int n, const int* row_ptr, const double* values, unsigned long long* out, cudaStream_t s) {
+    const int grid = std::min((n + 63) / 64, 1216);
+    row_bounds_kernel<<<grid, 256, 0, s>>>(n, row_ptr, values, out);
+    MEXK_CK_LAUNCH("row_bounds_kernel");
+    return MEXK_OK;
+}
+
 __global__ void set_one_kernel(int* p) { *p = 1; }
 
 int launch_symmetric_check(int n, const int* row_ptr, const int* col_idx, const double* values, int* ok,
@@ -923,7 +959,8 @@ extern "C" int mexk_test_force_wait_timeout(int device, int enable) {
     MEXK_CK(cudaSetDevice(device));
     const int v = enable ? 1 : 0;
     MEXK_CK(cudaMemcpyToSymbol(mexk::g_test_dead_wait, &v, sizeof(int)));
-    const int rc = mexk::lanczos_cycle_test_hook(enable);
+    int rc = mexk::lanczos_cycle_test_hook(enable);
+    if (rc == MEXK_OK) rc = mexk::arnoldi_cycle_test_hook(enable);
     if (rc != MEXK_OK) return rc;
     MEXK_CK(cudaDeviceSynchronize());
     return MEXK_OK;
