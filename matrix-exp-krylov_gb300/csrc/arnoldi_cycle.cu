@@ -39,6 +39,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <climits>
 
 namespace mexk {
 
@@ -220,16 +221,128 @@ __device__ __forceinline__ void ac_place(int lane, int* column, int* copy) {
 extern __shared__ double ac_smem[];  // w (the block's rows); a cluster: then the exchanges' partials
 
 constexpr int AC_TILE = 2048;  // products staged at a time
+constexpr int AC_SMEM_DOUBLES = 22528;  // rows of w, and of its digits, that a block keeps in shared memory (176 KB)
 
 struct AcShared {
     double h[MEXK_M_MAX];               // the second pass's coefficients
     double h1[MEXK_M_MAX];              // the first pass's
     double red[AC_NW][MEXK_M_MAX + 1];  // row slices' dots, then the partial sums' slices
     double prod[AC_TILE];
+    int4 hd[MEXK_M_MAX + 8];            // digits of the update's coefficients, zero past the last
+    int vexp[MEXK_M_MAX + 1];           // exponents of the block's digit columns
     double inv;
+    unsigned mag[3];                    // largest high words, by turns
+    int escale;
     int ok, nlong;
     int rows_long[AC_THREADS];
 };
+
+// ---- 61-bit fixed point in three digits ---------------------------------------
+// This GPU issues about 1.7 FP64 FMAs per clock and SM, where memory delivers
+// 2.1 (from L2) to 2.6 (HBM, long columns) doubles; integer multiply-adds of
+// 32 bits into 64 run at 60. So a wide basis also keeps its columns as
+// X = v 2^(61-E), |X| < 2^61 rounded to nearest, with one exponent E per
+// block and column, packed as three balanced 21-bit digits (d2 2^42 + d1 2^21
+// + d0), and w and h are taken to the same form: a product's six leading
+// digit products are exact in three 64-bit sums, what is dropped is below
+// 2^-60 of the largest product. The quantum, 2^-62 of the block's largest
+// entry, keeps a dot or update at least as close to exact as FP64's rounding
+// of 2^-53 per entry: by 2^6 for entries of similar size, and for one large
+// entry among 27,000 small ones in every block by sqrt(27000) 2^-62 = 2^-54.6
+// against 2^-53. An element costs about 20 integer instructions (2.4 elements
+// per clock alone), so of each eight columns three stay on the FP64 units,
+// which work beside the integer ones. Sweeps of heat 2048^2 (27,600 rows a
+// block): 249,000 / 298,000 clocks a dot / update sweep in FP64, 228,000 /
+// 217,000 so.
+constexpr int AC_FRAC = 61;
+constexpr int AC_FP64_COLS = 3;  // of eight columns, those left to the FP64 units, which work beside the integer ones
+constexpr unsigned long long AC_BIAS = (1ull << 20) | (1ull << 41);
+struct Digits {
+    int d2, d1, d0;
+};
+__device__ __forceinline__ unsigned long long ac_pack(double v, int E) {
+    const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v));
+    const int e = static_cast<int>((u >> 52) & 0x7ff);
+    const unsigned long long m = e ? (u & 0xfffffffffffffull) | 0x10000000000000ull : 0ull;
+    const int sh = e - 1075 - (E - AC_FRAC);
+    unsigned long long x;
+    if (sh >= 0) x = m << sh;  // |v| < 2^E: sh <= 8
+    else x = sh > -55 ? (m + (1ull << (-sh - 1))) >> -sh : 0ull;
+    if (u >> 63) x = 0ull - x;
+    return (x + AC_BIAS) ^ AC_BIAS;  // balanced digits in two's complement fields
+}
+__device__ __forceinline__ Digits ac_digits(unsigned long long p) {
+    const unsigned lo = static_cast<unsigned>(p), hi = static_cast<unsigned>(p >> 32);
+    Digits d;
+    d.d2 = static_cast<int>(hi) >> 10;
+    d.d1 = static_cast<int>(__funnelshift_l(lo, hi, 22)) >> 11;
+    d.d0 = static_cast<int>(lo << 11) >> 11;
+    return d;
+}
+// s + a b in one integer instruction
+__device__ __forceinline__ void ac_mad(long long& s, int a, int b) {
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(s) : "r"(a), "r"(b));
+}
+struct DigitSum {
+    long long s4, s3, s2;  // weights 2^84, 2^63, 2^42
+    __device__ __forceinline__ void zero() { s4 = s3 = s2 = 0; }
+    __device__ __forceinline__ void add(const Digits& a, const Digits& b) {
+        ac_mad(s4, a.d2, b.d2);
+        ac_mad(s3, a.d2, b.d1);
+        ac_mad(s2, a.d2, b.d0);
+        ac_mad(s3, a.d1, b.d2);
+        ac_mad(s2, a.d1, b.d1);
+        ac_mad(s2, a.d0, b.d2);
+    }
+    // the sum times 2^E as a double, rounded once (integer arithmetic: a
+    // conversion would cost an FP64 instruction per part)
+    __device__ __forceinline__ double value(int E) const {
+        __int128 t = (static_cast<__int128>(s4) << 42) + (static_cast<__int128>(s3) << 21) + s2;
+        const bool neg = t < 0;
+        if (neg) t = -t;
+        const unsigned long long hi = static_cast<unsigned long long>(t >> 64), lo = static_cast<unsigned long long>(t);
+        if ((hi | lo) == 0ull) return 0.0;
+        const int lz = hi ? __clzll(static_cast<long long>(hi)) : 64 + __clzll(static_cast<long long>(lo));
+        const unsigned __int128 n = static_cast<unsigned __int128>(t) << lz;  // leading one at bit 127
+        const unsigned long long top = static_cast<unsigned long long>(n >> 64);
+        const int e = 127 - lz + 42 + E + 1023;  // biased exponent of the leading one
+        if (e <= 0 || e >= 2046) return ldexp(neg ? -static_cast<double>(top) : static_cast<double>(top), e - 1023 - 63);
+        unsigned long long b = (static_cast<unsigned long long>(e) << 52) + ((top >> 11) & 0xfffffffffffffull);
+        b += (top >> 10) & 1ull;  // to nearest, ties away (the bits below are not looked at)
+        return __longlong_as_double(static_cast<long long>(b | (neg ? 1ull << 63 : 0ull)));
+    }
+};
+// The same for one row of an update, whose coefficients have AC_HFRAC bits:
+// (s4 2^21 + s3 + s2 / 2^21) stays inside 64 bits for 128 columns.
+constexpr int AC_HFRAC = 57;
+__device__ __forceinline__ double ac_row_value(const DigitSum& s, int E) {
+    long long hi = (s.s4 << 21) + s.s3 + (s.s2 >> 21);
+    unsigned lo = static_cast<unsigned>(s.s2) & 0x1fffffu;
+    const bool neg = hi < 0;
+    if (neg) {  // -(hi 2^21 + lo)
+        hi = lo ? ~hi : -hi;
+        lo = (0u - lo) & 0x1fffffu;
+    }
+    unsigned long long u = static_cast<unsigned long long>(hi);
+    int shift = 63;  // weight 2^63 per unit of u
+    if (u >> 32 == 0ull) {  // fewer than 53 bits above lo: bring it in
+        u = (u << 21) | lo;
+        lo = 0u;
+        shift = 42;
+    }
+    if (u == 0ull) return 0.0;
+    const int lz = __clzll(static_cast<long long>(u));
+    u = (u << lz) | (lz <= 21 ? lo >> (21 - lz) : static_cast<unsigned long long>(lo) << (lz - 21));
+    const int e = 63 - lz + shift + E + 1023;
+    if (e <= 0 || e >= 2046) return ldexp(neg ? -static_cast<double>(u) : static_cast<double>(u), e - 1023 - 63);
+    const unsigned long long b =
+        (static_cast<unsigned long long>(e) << 52) + ((u >> 11) & 0xfffffffffffffull) + ((u >> 10) & 1ull);
+    return __longlong_as_double(static_cast<long long>(b | (neg ? 1ull << 63 : 0ull)));
+}
+// E with |v| < 2^E from the high word of |v| (0 for a zero or subnormal v)
+__device__ __forceinline__ int ac_exponent(unsigned hi) { return static_cast<int>(hi >> 20) - 1022; }
+__device__ __forceinline__ unsigned ac_mag(double v) { return static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu; }
+constexpr unsigned AC_INF = 0x7ff00000u;
 
 // One exchange: where the partial sums go. EXACT: part (in every block's
 // shared memory), column c's sub-block b at part[c * AC_PS + b]. Else the
@@ -244,7 +357,7 @@ struct AcExchange {
 // The dots of CN columns (kc of them real) with w over sub-blocks s0..s1-1.
 template <int WIDTH, bool EXACT, int CN>
 __device__ __forceinline__ void ac_dot_task(const double* V, size_t ldv, int c0, int kc, int r0, int s0, int s1, int sl,
-                                            const AcExchange& ex, AcShared& sh) {
+                                            const double* wv, const AcExchange& ex, AcShared& sh) {
     constexpr int SU = EXACT ? 1 : (CN == 8 ? 2 : 4);  // sub-blocks whose loads are in flight together
     const int lane = threadIdx.x & 31;
     double acc[CN];
@@ -263,7 +376,7 @@ __device__ __forceinline__ void ac_dot_task(const double* V, size_t ldv, int c0,
 #pragma unroll
         for (int u = 0; u < SU; ++u) {
             if (u > 0 && s + u >= s1) break;
-            const double2 w = *reinterpret_cast<const double2*>(ac_smem + lr + u * AC_SUB);
+            const double2 w = *reinterpret_cast<const double2*>(wv + lr + u * AC_SUB);
 #pragma unroll
             for (int c = 0; c < CN; ++c) {
                 acc[c] = fma(v[u][c].x, w.x, acc[c]);
@@ -311,7 +424,7 @@ __device__ __forceinline__ void ac_publish(const AcExchange& ex, int k, int slic
 // Warps take (group of up to eight columns, sub-block or row slice).
 template <int WIDTH, bool EXACT>
 __device__ __forceinline__ void ac_dots(const CycleArgs& g, const double* V, int k, int r0, int nsub,
-                                        const AcExchange& ex, AcShared& sh) {
+                                        const double* wv, const AcExchange& ex, AcShared& sh) {
     const int warp = threadIdx.x >> 5;
     const size_t ldv = static_cast<size_t>(g.ldv);
     const int cgs = (k + 7) >> 3;
@@ -320,10 +433,10 @@ __device__ __forceinline__ void ac_dots(const CycleArgs& g, const double* V, int
         const int cg = t % cgs, sl = t / cgs;
         const int c0 = cg * 8, kc = min(8, k - c0);
         const int s0 = EXACT ? sl : sl * nsub / slices, s1 = EXACT ? sl + 1 : (sl + 1) * nsub / slices;
-        if (kc > 4) ac_dot_task<WIDTH, EXACT, 8>(V, ldv, c0, kc, r0, s0, s1, sl, ex, sh);
-        else if (kc > 2) ac_dot_task<WIDTH, EXACT, 4>(V, ldv, c0, kc, r0, s0, s1, sl, ex, sh);
-        else if (kc > 1) ac_dot_task<WIDTH, EXACT, 2>(V, ldv, c0, kc, r0, s0, s1, sl, ex, sh);
-        else ac_dot_task<WIDTH, EXACT, 1>(V, ldv, c0, kc, r0, s0, s1, sl, ex, sh);
+        if (kc > 4) ac_dot_task<WIDTH, EXACT, 8>(V, ldv, c0, kc, r0, s0, s1, sl, wv, ex, sh);
+        else if (kc > 2) ac_dot_task<WIDTH, EXACT, 4>(V, ldv, c0, kc, r0, s0, s1, sl, wv, ex, sh);
+        else if (kc > 1) ac_dot_task<WIDTH, EXACT, 2>(V, ldv, c0, kc, r0, s0, s1, sl, wv, ex, sh);
+        else ac_dot_task<WIDTH, EXACT, 1>(V, ldv, c0, kc, r0, s0, s1, sl, wv, ex, sh);
     }
     if (!EXACT) {
         __syncthreads();
@@ -375,7 +488,8 @@ __device__ __forceinline__ void ac_sums(const AcExchange& ex, int k, int np, int
 // w -= V h over the block's rows (one FMA chain per row, in column order);
 // RU rows of a thread and CH columns in flight.
 template <int RU, int CH>
-__device__ __forceinline__ void ac_update_rows(const double* V, size_t ldv, int k, int r0, int rows, const double* h) {
+__device__ __forceinline__ void ac_update_rows(const double* V, size_t ldv, int k, int r0, int rows, const double* h,
+                                               double* w) {
     for (int r = threadIdx.x; r < rows; r += RU * AC_THREADS) {
         double s[RU];
 #pragma unroll
@@ -397,14 +511,291 @@ __device__ __forceinline__ void ac_update_rows(const double* V, size_t ldv, int 
         }
 #pragma unroll
         for (int i = 0; i < RU; ++i)
-            if (r + i * AC_THREADS < rows) ac_smem[r + i * AC_THREADS] -= s[i];
+            if (r + i * AC_THREADS < rows) w[r + i * AC_THREADS] -= s[i];
     }
 }
 __device__ __forceinline__ void ac_update(const CycleArgs& g, const double* V, int k, int r0, int rows,
-                                          const double* h) {
+                                          const double* h, double* w) {
     const size_t ldv = static_cast<size_t>(g.ldv);
-    if (k <= 2 && rows > AC_THREADS) ac_update_rows<4, 2>(V, ldv, k, r0, rows, h);
-    else ac_update_rows<1, 8>(V, ldv, k, r0, rows, h);
+    if (k <= 2 && rows > AC_THREADS) ac_update_rows<4, 2>(V, ldv, k, r0, rows, h, w);
+    else ac_update_rows<1, 8>(V, ldv, k, r0, rows, h, w);
+}
+
+// ---- the sweeps over the digit columns ---------------------------------------
+// Largest high word over the block of m (every thread calls it); the three
+// slots are used by turns.
+__device__ __forceinline__ unsigned ac_block_mag(unsigned m, int& turn, AcShared& sh) {
+    const int slot = turn;
+    turn = slot == 2 ? 0 : slot + 1;
+    m = __reduce_max_sync(AC_FULL, m);
+    if ((threadIdx.x & 31) == 0 && m != 0u) atomicMax(&sh.mag[slot], m);
+    __syncthreads();
+    const unsigned r = sh.mag[slot];
+    if (threadIdx.x == 0) sh.mag[slot == 0 ? 2 : slot - 1] = 0u;  // the last turn's: read by all before this barrier
+    return r;
+}
+
+// Digits of the update's coefficients: h_c 2^(E_c) relative to the largest
+// (E_c: the exponent of column lo + c in this block); sh.escale its exponent,
+// INT_MAX when a coefficient is not finite.
+__device__ __forceinline__ void ac_coefficients(int lo, int k, const double* h, AcShared& sh) {
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int E[MEXK_M_MAX / 32], best = INT_MIN;
+        bool finite = true;
+#pragma unroll
+        for (int i = 0; i < MEXK_M_MAX / 32; ++i) {
+            const int c = lane + 32 * i;
+            E[i] = INT_MIN;
+            if (c < k && (ac_mag(h[c]) >> 20) != 0u) {
+                finite = finite && ac_mag(h[c]) < AC_INF;
+                E[i] = sh.vexp[lo + c];
+                best = max(best, E[i] + ac_exponent(ac_mag(h[c])));
+            }
+        }
+        best = __reduce_max_sync(AC_FULL, best);
+        if (best == INT_MIN) best = 0;
+#pragma unroll
+        for (int i = 0; i < MEXK_M_MAX / 32; ++i) {
+            const int c = lane + 32 * i;
+            if (c < 8) sh.hd[k + c] = make_int4(0, 0, 0, 0);
+            if (c < k) {
+                const Digits d = E[i] == INT_MIN ? Digits{0, 0, 0} : ac_digits(ac_pack(h[c], best - E[i] + AC_FRAC - AC_HFRAC));
+                sh.hd[c] = make_int4(d.d2, d.d1, d.d0, 0);
+            }
+        }
+        finite = __all_sync(AC_FULL, finite);
+        if (lane == 0) sh.escale = finite ? best : INT_MAX;
+    }
+    __syncthreads();
+}
+
+// w -= V h over the block's rows (columns lo..lo+k-1), RP rows per thread and
+// eight columns in flight, three of each eight in FP64 and five in digits;
+// returns the thread's largest high word of |w|. Coefficients that are not
+// finite make w NaN, which ends the basis.
+template <int RP>
+__device__ __forceinline__ unsigned ac_update_digit_rows(const CycleArgs& g, int lo, int k, int r0, int rows, double* w,
+                                                         const double* hc, const AcShared& sh) {
+    constexpr int CH = 8;
+    const size_t ldv = static_cast<size_t>(g.ldv);
+    const bool finite = sh.escale != INT_MAX;
+    const int E = sh.escale - AC_HFRAC - AC_FRAC;
+    const ptrdiff_t qoff = reinterpret_cast<const char*>(g.vq) - reinterpret_cast<const char*>(g.V);
+    unsigned mag = 0u;
+    unsigned long long v[CH][RP];
+    // each column's registers are reloaded, for the next eight columns or the
+    // next rows, as soon as they are used: the loads stay in flight
+    const char* next = reinterpret_cast<const char*>(g.V + static_cast<size_t>(lo) * ldv + r0 +
+                                                     RP * static_cast<int>(threadIdx.x));
+    auto load = [&](int u, bool on) {  // column u of the eight at next
+        const char* p = next + static_cast<size_t>(u) * ldv * 8 + (u < AC_FP64_COLS ? 0 : qoff);
+        if constexpr (RP == 2) {
+            const ulonglong2 t = on ? *reinterpret_cast<const ulonglong2*>(p) : make_ulonglong2(0ull, 0ull);
+            v[u][0] = t.x;
+            v[u][1] = t.y;
+        } else {
+            v[u][0] = on ? *reinterpret_cast<const unsigned long long*>(p) : 0ull;
+        }
+    };
+    int r = RP * static_cast<int>(threadIdx.x);
+#pragma unroll
+    for (int u = 0; u < CH; ++u) load(u, r < rows && u < k);
+    for (; r < rows; r += RP * AC_THREADS) {
+        DigitSum a[RP];
+        double f[RP];
+#pragma unroll
+        for (int i = 0; i < RP; ++i) {
+            a[i].zero();
+            f[i] = 0.0;
+        }
+        const char* const here = next;
+        const char* p = here;
+        for (int c = 0; c < k; c += CH) {
+            const bool more = c + CH < k;
+            p += CH * ldv * 8;
+            if (!more) p = here + RP * AC_THREADS * 8;
+            next = p;
+            const bool on = more || r + RP * AC_THREADS < rows;
+            const int left = more ? k - c - CH : k;
+#pragma unroll
+            for (int u = 0; u < CH; ++u) {
+                if (u < AC_FP64_COLS) {
+                    const double h = c + u < k ? hc[c + u] : 0.0;
+#pragma unroll
+                    for (int i = 0; i < RP; ++i) f[i] = fma(__longlong_as_double(static_cast<long long>(v[u][i])), h, f[i]);
+                    load(u, on && u < left);
+                } else {
+                    const int4 h4 = sh.hd[c + u];  // zero past column k
+                    const Digits h = {h4.x, h4.y, h4.z};
+                    Digits d[RP];
+#pragma unroll
+                    for (int i = 0; i < RP; ++i) d[i] = ac_digits(v[u][i]);
+                    load(u, on && u < left);
+#pragma unroll
+                    for (int i = 0; i < RP; ++i) a[i].add(d[i], h);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < RP; ++i) {
+            const double x =
+                finite ? w[r + i] - (f[i] + ac_row_value(a[i], E)) : __longlong_as_double(0x7ff8000000000000ll);
+            w[r + i] = x;
+            mag = max(mag, ac_mag(x));
+        }
+    }
+    return mag;
+}
+__device__ __forceinline__ unsigned ac_update_digits(const CycleArgs& g, int lo, int k, int r0, int rows, double* w,
+                                                     const double* hc, const AcShared& sh) {
+    // pairs of rows where they leave no larger share of the threads idle in the last round
+    const bool pairs = 2 * ((rows + 2 * AC_THREADS - 1) / (2 * AC_THREADS)) <= (rows + AC_THREADS - 1) / AC_THREADS;
+    return pairs ? ac_update_digit_rows<2>(g, lo, k, r0, rows, w, hc, sh)
+                 : ac_update_digit_rows<1>(g, lo, k, r0, rows, w, hc, sh);
+}
+
+// The warp's dots of CN columns from c0 (kc of them real) with w over
+// sub-blocks s0..s1-1, into red[sl]: the first ND in FP64, the rest in digits.
+template <int CN>
+__device__ __forceinline__ void ac_digit_task(const CycleArgs& g, int lo, int c0, int kc, int r0, int s0, int s1, int sl,
+                                              const double* w, const unsigned long long* wq, int E, bool finite,
+                                              AcShared& sh) {
+    constexpr int ND = CN == 8 ? AC_FP64_COLS : CN >= 4 ? 2 : CN / 2;
+    const int lane = threadIdx.x & 31;
+    const size_t ldv = static_cast<size_t>(g.ldv);
+    DigitSum acc[CN - ND];
+    double f[ND > 0 ? ND : 1];
+#pragma unroll
+    for (int c = 0; c < CN - ND; ++c) acc[c].zero();
+#pragma unroll
+    for (int c = 0; c < ND; ++c) f[c] = 0.0;
+    const size_t off = static_cast<size_t>(lo + c0) * ldv + (r0 + s0 * AC_SUB + 2 * lane);
+    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(g.V + off);
+    const ulonglong2* pq = reinterpret_cast<const ulonglong2*>(g.vq + off);
+    const size_t ld2 = ldv / 2;
+    ulonglong2 v[CN];
+    auto load = [&](int c, bool on) {
+        v[c] = (c < kc && on) ? (c < ND ? p : pq)[c * ld2] : make_ulonglong2(0ull, 0ull);
+    };
+#pragma unroll
+    for (int c = 0; c < CN; ++c) load(c, s0 < s1);
+    for (int s = s0; s < s1; ++s) {
+        p += AC_SUB / 2;
+        pq += AC_SUB / 2;
+        const int lr = s * AC_SUB + 2 * lane;
+        const double2 x = *reinterpret_cast<const double2*>(w + lr);
+        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(wq + lr);
+        const Digits x0 = ac_digits(q.x), x1 = ac_digits(q.y);
+        const bool more = s + 1 < s1;
+        // a column's registers are reloaded as soon as it is used: the loads stay in flight
+#pragma unroll
+        for (int c = 0; c < ND; ++c) {
+            f[c] = fma(__longlong_as_double(static_cast<long long>(v[c].x)), x.x, f[c]);
+            f[c] = fma(__longlong_as_double(static_cast<long long>(v[c].y)), x.y, f[c]);
+            load(c, more);
+        }
+#pragma unroll
+        for (int c = ND; c < CN; ++c) {
+            const Digits d0 = ac_digits(v[c].x), d1 = ac_digits(v[c].y);
+            load(c, more);
+            acc[c - ND].add(d0, x0);
+            acc[c - ND].add(d1, x1);
+        }
+    }
+    if constexpr (ND > 0) {
+        constexpr int NP = ND > 2 ? 4 : ND;
+        double t[NP];
+#pragma unroll
+        for (int c = 0; c < NP; ++c) t[c] = c < ND ? f[c < ND ? c : 0] : 0.0;
+        const double tot = ac_reduce<2, NP>(t, lane);
+        int c, copy;
+        ac_place<2, NP>(lane, &c, &copy);
+        if (copy == 0 && c < ND && c < kc) sh.red[sl][c0 + c] = tot;
+    }
+    // the warp's totals, the columns transposed over the lanes
+    constexpr int CQ = CN - ND, CP = CQ > 4 ? 8 : CQ > 2 ? 4 : CQ;  // a power of two
+    DigitSum sum[CP];
+#pragma unroll
+    for (int c = 0; c < CP; ++c) {
+        if (c < CQ) sum[c] = acc[c < CQ ? c : 0];
+        else sum[c].zero();
+    }
+    auto swap_add = [&](long long& keep_lo, long long hi, bool up, int b) {
+        const long long send = up ? keep_lo : hi, keep = up ? hi : keep_lo;
+        keep_lo = keep + __shfl_xor_sync(AC_FULL, send, b);
+    };
+    int b = 16, cc = 0;
+#pragma unroll
+    for (int h = CP / 2; h >= 1; h >>= 1, b >>= 1) {
+        const bool up = (lane & b) != 0;
+        if (up) cc += h;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            swap_add(sum[i].s4, sum[i + h].s4, up, b);
+            swap_add(sum[i].s3, sum[i + h].s3, up, b);
+            swap_add(sum[i].s2, sum[i + h].s2, up, b);
+        }
+    }
+    const int rest = 2 * b - 1;  // the lane bits that name copies
+    for (; b >= 1; b >>= 1) {
+        sum[0].s4 += __shfl_xor_sync(AC_FULL, sum[0].s4, b);
+        sum[0].s3 += __shfl_xor_sync(AC_FULL, sum[0].s3, b);
+        sum[0].s2 += __shfl_xor_sync(AC_FULL, sum[0].s2, b);
+    }
+    cc += ND;
+    if ((lane & rest) == 0 && cc < kc) {
+        const double t = sum[0].value(E + sh.vexp[lo + c0 + cc] - 2 * AC_FRAC);
+        sh.red[sl][c0 + cc] = finite ? t : __longlong_as_double(0x7ff8000000000000ll);
+    }
+}
+
+// Dots of all k columns with w over the block's rows into the exchange: w's
+// digits first (relative to its largest entry in the block, whose high word
+// is mag), then every warp its (group of columns, row slice) without meeting.
+__device__ __forceinline__ void ac_dots_digits(const CycleArgs& g, int lo, int k, int r0, int nsub, const double* w,
+                                               unsigned mag, unsigned long long* wq, const AcExchange& ex,
+                                               AcShared& sh) {
+    const int warp = threadIdx.x >> 5;
+    const bool finite = mag < AC_INF;
+    const int E = ac_exponent(min(mag, AC_INF - 1u));
+    for (int r = 2 * static_cast<int>(threadIdx.x); r < nsub * AC_SUB; r += 2 * AC_THREADS) {
+        const double2 x = *reinterpret_cast<const double2*>(w + r);
+        *reinterpret_cast<ulonglong2*>(wq + r) = finite ? make_ulonglong2(ac_pack(x.x, E), ac_pack(x.y, E))
+                                                        : make_ulonglong2(0ull, 0ull);
+    }
+    __syncthreads();
+    const int cgs = (k + 7) >> 3;  // groups of columns as even as they come
+    const int slices = max(1, min(nsub, AC_NW / cgs));
+    const int cg = warp % cgs, sl = warp / cgs;  // at most one task per warp: cgs <= AC_NW
+    if (sl < slices) {
+        const int c0 = cg * k / cgs, kc = (cg + 1) * k / cgs - c0;
+        const int s0 = sl * nsub / slices, s1 = (sl + 1) * nsub / slices;
+        if (kc > 6) ac_digit_task<8>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
+        else if (kc > 4) ac_digit_task<6>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
+        else if (kc > 2) ac_digit_task<4>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
+        else if (kc > 1) ac_digit_task<2>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
+        else ac_digit_task<1>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
+    }
+    __syncthreads();
+    ac_publish(ex, k, slices, g.scale, sh);
+}
+
+// Column c of the basis into digits from the block's rows of the FP64 column
+// (the cycle's first column).
+__device__ __forceinline__ void ac_pack_column(const CycleArgs& g, int c, int r0, int rows, AcShared& sh, int& turn) {
+    const double* v = g.V + static_cast<size_t>(c) * g.ldv + r0;
+    unsigned long long* q = g.vq + static_cast<size_t>(c) * g.ldv + r0;
+    unsigned mag = 0u;
+    for (int r = threadIdx.x; r < rows; r += AC_THREADS) mag = max(mag, ac_mag(v[r]));
+    mag = ac_block_mag(mag, turn, sh);
+    const int E = ac_exponent(min(mag, AC_INF - 1u));  // non-finite columns are caught by w
+    for (int r = threadIdx.x; r < rows; r += AC_THREADS) q[r] = ac_pack(v[r], E);
+    if (threadIdx.x == 0) {
+        sh.vexp[c] = E;
+        g.vexp[c * CYCLE_MAX_BLOCKS + blockIdx.x] = E;
+    }
+    __syncthreads();
 }
 
 // The block's rows of w = A x in the row-pattern form, patterns of at most LM
@@ -412,7 +803,7 @@ __device__ __forceinline__ void ac_update(const CycleArgs& g, const double* V, i
 // entries times inv (scaled) or as they are.
 template <int LM>
 __device__ __forceinline__ void ac_product_pattern(const CycleArgs& g, const double* gx, double inv, bool scaled,
-                                                   int r0, int rows, int n_rows) {
+                                                   int r0, int rows, int n_rows, double* w) {
     const RowPatterns* __restrict__ T = g.T;
     for (int r = threadIdx.x; r < rows; r += AC_THREADS) {
         double s = 0.0;
@@ -432,7 +823,7 @@ __device__ __forceinline__ void ac_product_pattern(const CycleArgs& g, const dou
             for (int q = 0; q < LM; ++q)
                 if (q < len) s = __dadd_rn(s, __dmul_rn(a[q], scaled ? __dmul_rn(x[q], inv) : x[q]));
         }
-        ac_smem[r] = s;
+        w[r] = s;
     }
 }
 
@@ -441,7 +832,7 @@ __device__ __forceinline__ void ac_product_pattern(const CycleArgs& g, const dou
 // entries summed in order by its thread, a longer one by a warp, lanes
 // strided, from the arrays.
 __device__ __forceinline__ void ac_product_csr(const CycleArgs& g, const double* gx, double inv, bool scaled, int r0,
-                                               int rows, int n_rows, AcShared& sh) {
+                                               int rows, int n_rows, double* w, AcShared& sh) {
     constexpr int EU = AC_TILE / AC_THREADS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto entry = [&](int e) {
@@ -485,7 +876,7 @@ __device__ __forceinline__ void ac_product_csr(const CycleArgs& g, const double*
             for (; e < min(e1, te); ++e) s = __dadd_rn(s, sh.prod[e - tb]);
             __syncthreads();
         }
-        if (r < rows) ac_smem[r] = s;
+        if (r < rows) w[r] = s;
         __syncthreads();
         for (int i = warp; i < sh.nlong; i += AC_NW) {
             const int q = sh.rows_long[i];
@@ -493,28 +884,28 @@ __device__ __forceinline__ void ac_product_csr(const CycleArgs& g, const double*
             double t = 0.0;
             for (int i2 = a0 + lane; i2 < a1; i2 += 32) t = __dadd_rn(t, entry(i2));
             t = warp_sum(t);
-            if (lane == 0) ac_smem[q] = t;
+            if (lane == 0) w[q] = t;
         }
         __syncthreads();
     }
 }
 
 __device__ __forceinline__ void ac_product(const CycleArgs& g, const double* gx, double inv, bool scaled, int r0,
-                                           int rows, int n_rows, AcShared& sh) {
-    if (g.pid == nullptr) ac_product_csr(g, gx, inv, scaled, r0, rows, n_rows, sh);
-    else if (g.max_len <= 5) ac_product_pattern<5>(g, gx, inv, scaled, r0, rows, n_rows);
-    else if (g.max_len <= 7) ac_product_pattern<7>(g, gx, inv, scaled, r0, rows, n_rows);
-    else ac_product_pattern<PAT_LEN>(g, gx, inv, scaled, r0, rows, n_rows);
+                                           int rows, int n_rows, double* w, AcShared& sh) {
+    if (g.pid == nullptr) ac_product_csr(g, gx, inv, scaled, r0, rows, n_rows, w, sh);
+    else if (g.max_len <= 5) ac_product_pattern<5>(g, gx, inv, scaled, r0, rows, n_rows, w);
+    else if (g.max_len <= 7) ac_product_pattern<7>(g, gx, inv, scaled, r0, rows, n_rows, w);
+    else ac_product_pattern<PAT_LEN>(g, gx, inv, scaled, r0, rows, n_rows, w);
 }
 
 // |w|^2 over the block's rows into the exchange. EXACT per sub-block (pairs,
 // then the plain butterfly).
 template <bool EXACT>
-__device__ __forceinline__ void ac_norm(int r0, int nsub, const AcExchange& ex, AcShared& sh) {
+__device__ __forceinline__ void ac_norm(int r0, int nsub, const double* wv, const AcExchange& ex, AcShared& sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double acc = 0.0;
     for (int s = warp; s < nsub; s += AC_NW) {
-        const double2 w = *reinterpret_cast<const double2*>(ac_smem + s * AC_SUB + 2 * lane);
+        const double2 w = *reinterpret_cast<const double2*>(wv + s * AC_SUB + 2 * lane);
         if (EXACT) acc = 0.0;
         acc = fma(w.x, w.x, acc);
         acc = fma(w.y, w.y, acc);
@@ -573,7 +964,10 @@ __device__ __forceinline__ double ac_norm_sum(const AcExchange& ex, int np) {
     return s;
 }
 
-template <bool CLUSTER>
+// CLUSTER: one cluster, the separate kernels' sums. DIGITS: the sweeps over
+// the digit columns. WSMEM: the block's rows of w fit in shared memory (else
+// they stay in x).
+template <bool CLUSTER, bool DIGITS, bool WSMEM>
 __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs g) {
     constexpr bool EXACT = CLUSTER;
     __shared__ AcShared sh;
@@ -589,6 +983,15 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
     const bool lead = blockIdx.x == 0;
     unsigned target = 0;
     double inv = 1.0;
+    double* const w = WSMEM ? ac_smem : g.x + r0;
+    unsigned long long* const wq = WSMEM ? reinterpret_cast<unsigned long long*>(ac_smem + g.rows) : g.wq + r0;
+    int turn = 0;
+    if (DIGITS) {
+        if (threadIdx.x < 3) sh.mag[threadIdx.x] = 0u;
+        for (int c = threadIdx.x; c <= g.j0; c += AC_THREADS) sh.vexp[c] = g.vexp[c * CYCLE_MAX_BLOCKS + blockIdx.x];
+        __syncthreads();
+        if (g.j0 == 0) ac_pack_column(g, 0, r0, rows, sh, turn);
+    }
     // the exchanges of a step: first dots, second dots, norm; a grid's words
     // alternate by step parity, so that one set is cleared while the other is
     // in use
@@ -619,17 +1022,27 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         const bool scaled = j > g.j0 && g.scale_gather;
         if (!EXACT) exchanges(j & 1);
         if (g.product) {
-            ac_product(g, scaled ? g.x : g.V + static_cast<size_t>(j) * ldv, inv, scaled, r0, rows, n_rows, sh);
-        } else {
-            for (int r = threadIdx.x; r < rows; r += AC_THREADS) ac_smem[r] = r < n_rows ? __ldg(g.x + r0 + r) : 0.0;
+            ac_product(g, scaled ? g.x : g.V + static_cast<size_t>(j) * ldv, inv, scaled, r0, rows, n_rows, w, sh);
+        } else if (WSMEM) {
+            for (int r = threadIdx.x; r < rows; r += AC_THREADS) w[r] = r < n_rows ? __ldg(g.x + r0 + r) : 0.0;
         }
         __syncthreads();
         auto dots = [&](const AcExchange& e) {
-            if (k <= 8) ac_dots<0, EXACT>(g, V, k, r0, nsub, e, sh);
-            else if (k <= 16) ac_dots<1, EXACT>(g, V, k, r0, nsub, e, sh);
-            else ac_dots<2, EXACT>(g, V, k, r0, nsub, e, sh);
+            if (k <= 8) ac_dots<0, EXACT>(g, V, k, r0, nsub, w, e, sh);
+            else if (k <= 16) ac_dots<1, EXACT>(g, V, k, r0, nsub, w, e, sh);
+            else ac_dots<2, EXACT>(g, V, k, r0, nsub, w, e, sh);
         };
-        dots(ex[0]);
+        unsigned mag = 0u;
+        if (DIGITS) {
+            for (int r = 2 * static_cast<int>(threadIdx.x); r < rows; r += 2 * AC_THREADS) {
+                const double2 x = *reinterpret_cast<const double2*>(w + r);
+                mag = max(mag, max(ac_mag(x.x), ac_mag(x.y)));
+            }
+            mag = ac_block_mag(mag, turn, sh);
+            ac_dots_digits(g, lo, k, r0, nsub, w, mag, wq, ex[0], sh);
+        } else {
+            dots(ex[0]);
+        }
         if (!ac_meet<CLUSTER>(g.bar, target, &st->status, &sh.ok)) return;
         // every block has read the other parity's sums: clear them for the next step
         if (!EXACT && lead) {
@@ -637,21 +1050,32 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
             for (int i = threadIdx.x; i < 2 * CYCLE_EXCHANGE; i += AC_THREADS) __stcg(w + i, 0ull);
         }
         ac_sums<EXACT>(ex[0], k, np, g.scale, sh.h1, sh);
-        ac_update(g, V, k, r0, rows, sh.h1);
-        __syncthreads();
+        if (DIGITS) {
+            ac_coefficients(lo, k, sh.h1, sh);
+            mag = ac_block_mag(ac_update_digits(g, lo, k, r0, rows, w, sh.h1, sh), turn, sh);
+        } else {
+            ac_update(g, V, k, r0, rows, sh.h1, w);
+            __syncthreads();
+        }
         if (g.reortho) {
-            dots(ex[1]);
+            if (DIGITS) ac_dots_digits(g, lo, k, r0, nsub, w, mag, wq, ex[1], sh);
+            else dots(ex[1]);
             if (!ac_meet<CLUSTER>(g.bar, target, &st->status, &sh.ok)) return;
             ac_sums<EXACT>(ex[1], k, np, g.scale, sh.h, sh);
-            ac_update(g, V, k, r0, rows, sh.h);
+            if (DIGITS) {
+                ac_coefficients(lo, k, sh.h, sh);
+                mag = ac_block_mag(ac_update_digits(g, lo, k, r0, rows, w, sh.h, sh), turn, sh);
+            } else {
+                ac_update(g, V, k, r0, rows, sh.h, w);
+            }
         }
         if (lead)
             for (int c = threadIdx.x; c < k; c += AC_THREADS)
                 g.H[(lo + c) + j * ldh] = g.reortho ? sh.h1[c] + sh.h[c] : sh.h1[c];
         __syncthreads();
-        ac_norm<EXACT>(r0, nsub, ex[2], sh);
-        if (g.scale_gather)
-            for (int r = threadIdx.x; r < n_rows; r += AC_THREADS) __stcg(g.x + r0 + r, ac_smem[r]);
+        ac_norm<EXACT>(r0, nsub, w, ex[2], sh);
+        if (WSMEM && g.scale_gather)
+            for (int r = threadIdx.x; r < n_rows; r += AC_THREADS) __stcg(g.x + r0 + r, w[r]);
         if (!ac_meet<CLUSTER>(g.bar, target, &st->status, &sh.ok)) return;
         const double w2 = ac_norm_sum<EXACT>(ex[2], np);
         // one thread: a square root and a division by every warp would queue on the FP64 units
@@ -672,7 +1096,22 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         if (!sh.ok) break;  // the same sums in every block
         inv = sh.inv;
         double* q = g.V + static_cast<size_t>(j + 1) * ldv + r0;
-        for (int r = threadIdx.x; r < n_rows; r += AC_THREADS) __stcg(q + r, ac_smem[r] * inv);
+        if (DIGITS) {
+            // |w| < 2^a, 1/|w| < 2^b: every entry of the new column below 2^(a+b)
+            const int E = ac_exponent(min(mag, AC_INF - 1u)) + ac_exponent(ac_mag(inv));
+            unsigned long long* vq = g.vq + static_cast<size_t>(j + 1) * ldv + r0;
+            for (int r = threadIdx.x; r < n_rows; r += AC_THREADS) {
+                const double v = w[r] * inv;
+                __stcg(q + r, v);
+                __stcg(vq + r, ac_pack(v, E));
+            }
+            if (threadIdx.x == 0) {
+                sh.vexp[j + 1] = E;
+                g.vexp[(j + 1) * CYCLE_MAX_BLOCKS + blockIdx.x] = E;
+            }
+        } else {
+            for (int r = threadIdx.x; r < n_rows; r += AC_THREADS) __stcg(q + r, w[r] * inv);
+        }
         if (!g.scale_gather && j + 1 < g.j1 && !ac_meet<CLUSTER>(g.bar, target, &st->status, &sh.ok)) return;
         __syncthreads();
     }
@@ -702,6 +1141,16 @@ int sm_total() { return std::min(device_sm_count(), CYCLE_MAX_BLOCKS); }
 
 bool arnoldi_cycle_fits(int n) { return n <= CYCLE_ROWS_MAX; }
 
+// Digits pay from about 20,000 entries per block and sweep. FP64 sweeps against
+// them, by rows x allocated columns: 8,000 x 100 19.4 / 19.7 ms, 50,000 x 30
+// 1008 / 1032 us, 100,000 x 30 1365 / 1349 us, 50,021 x 100 32.7 / 29.7 ms,
+// 604,000 x 30 16.3 / 14.4 ms, 4,194,304 x 30 247 / 209 ms. The allocation
+// decides (not the step), so that a solve's sums do not depend on the ones
+// before it. A window of up to four columns has next to no sweeps.
+bool arnoldi_cycle_digits(int n, int m_alloc, int window) {
+    return n > EXACT_ROWS && static_cast<long long>(n) * m_alloc >= 3000000 && (window == 0 || window > 4);
+}
+
 // Measured on random rows (degree 10, m = 30, one cycle): own product against
 // the context's SpMV and a launch per step, 661 / 871 us at 5,000 rows, 997 /
 // 1108 at 50,000, 1367 / 1382 at 100,000, 1971 / 1957 at 200,000 (2.2 million
@@ -715,12 +1164,13 @@ bool arnoldi_cycle_product(int n, long long nnz, int max_row, bool pattern) {
 }
 
 int arnoldi_cycle_prepare() {
-    const int rows = (CYCLE_ROWS_MAX + sm_total() - 1) / sm_total() + 2 * AC_SUB;
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(sizeof(double)) * (EXACT_ROWS / AC_CLUSTER + (2 * MEXK_M_MAX + 1) * AC_PS)));
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(sizeof(double)) * rows));
+    const int cl = static_cast<int>(sizeof(double)) * (EXACT_ROWS / AC_CLUSTER + (2 * MEXK_M_MAX + 1) * AC_PS);
+    const int ws = static_cast<int>(sizeof(double)) * AC_SMEM_DOUBLES;
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cl));
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true>,
+                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
     return MEXK_OK;
 }
 
@@ -749,7 +1199,11 @@ int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(AC_THREADS);
-    cfg.dynamicSmemBytes = sizeof(double) * (static_cast<size_t>(a.rows) + (cluster ? (2 * static_cast<size_t>(a.m) + 1) * AC_PS : 0));
+    const bool digits = !cluster && a.vq != nullptr;
+    const bool wsmem = a.rows * (digits ? 2 : 1) <= AC_SMEM_DOUBLES;
+    if (!wsmem) a.scale_gather = 0;  // x holds w
+    cfg.dynamicSmemBytes = sizeof(double) * ((wsmem ? static_cast<size_t>(a.rows) * (digits ? 2 : 1) : 0) +
+                                             (cluster ? (2 * static_cast<size_t>(a.m) + 1) * AC_PS : 0));
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     if (cluster) {
@@ -766,8 +1220,11 @@ int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s) {
         cfg.numAttrs = 1;
     }
     cfg.attrs = attr;
-    const cudaError_t e = cluster ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true>, a)
-                                  : cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false>, a);
+    const cudaError_t e = cluster           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true, false, true>, a)
+                          : digits && wsmem ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true, true>, a)
+                          : digits          ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true, false>, a)
+                          : wsmem           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, true>, a)
+                                            : cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, false>, a);
     if (e != cudaSuccess) {
         set_cuda_error(e, "arnoldi_cycle_kernel", __FILE__, __LINE__);
         return MEXK_ERR_CUDA;

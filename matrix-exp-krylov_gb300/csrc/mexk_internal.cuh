@@ -399,7 +399,7 @@ constexpr int CYCLE_DIGITS = 8;        // words per column of an exchange
 constexpr int CYCLE_EXCHANGE = MEXK_M_MAX * CYCLE_DIGITS + 2;
 constexpr int CYCLE_MAX_BLOCKS = 256;
 constexpr int CYCLE_WORDS = 4 * CYCLE_EXCHANGE + CYCLE_MAX_BLOCKS;
-constexpr int CYCLE_ROWS_MAX = 2000000;
+constexpr int CYCLE_ROWS_MAX = 16000000;
 struct CycleArgs {
     int n, m, ldv, ldh, reortho, window;
     int j0, j1, product;
@@ -413,6 +413,9 @@ struct CycleArgs {
     const uint8_t* pid;  // the row-pattern form, or null: the CSR arrays
     const RowPatterns* T;
     double* V;
+    unsigned long long* vq = nullptr;  // the basis in digits, as V (arnoldi_cycle_digits), or null
+    int* vexp = nullptr;               // its exponents, column c's at c * CYCLE_MAX_BLOCKS
+    unsigned long long* wq = nullptr;  // ldv words: w in digits, where it does not fit on chip
     double* x;
     double* H;
     DevState* st;
@@ -423,6 +426,8 @@ struct CycleArgs {
 // sum of |values|, and the entries of the longest row.
 int launch_row_bounds(int n, const int* row_ptr, const double* values, unsigned long long* out, cudaStream_t s);
 bool arnoldi_cycle_fits(int n);
+// Whether a basis runs its sweeps on digit columns (vq, vexp, wq).
+bool arnoldi_cycle_digits(int n, int m_alloc, int window);
 // Whether the launch also takes the products (else one launch per step after
 // the context's SpMV).
 bool arnoldi_cycle_product(int n, long long nnz, int max_row, bool pattern);

@@ -35,6 +35,11 @@ CASES += [("random", 2000, 32, 1, 0), ("random", 2000, 64, 1, 0), ("random", 600
           ("powerlaw", 2048, 20, 1, 0), ("powerlaw", 12345, 20, 1, 0), ("longrow", 3000, 8, 1, 0),
           ("longrow", 6000, 8, 1, 0), ("heat", 40, 30, 1, 0), ("heat", 64, 30, 1, 2), ("heat", 64, 20, 0, 3),
           ("heat", 131, 17, 1, 0), ("heat", 131, 30, 1, 2), ("heat", 301, 30, 1, 4)]
+# sweeps on digit columns (rows x allocated columns >= 3 million): full and window, one and two rows per thread,
+# own product and the SpMV's, every group size
+CASES += [("random", 300011, 10, 1, 0), ("random", 150003, 23, 1, 0), ("random", 40007, 75, 1, 0),
+          ("random", 150003, 20, 0, 0), ("powerlaw", 160001, 19, 1, 0), ("heat", 601, 17, 1, 0),
+          ("heat", 601, 30, 1, 6)]
 
 
 @pytest.mark.parametrize("kind,n,m,reortho,window", CASES)
@@ -85,3 +90,39 @@ def test_basis_matches_stepwise(kind, n, m, reortho, window):
             term = (t / i) * (M @ term)
             ref += term
         assert np.linalg.norm(y - ref) <= 1e-12 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("n,m", [(150001, 21), (40007, 80)])
+def test_localised_vector_keeps_fp64_orthogonality(n, m):
+    """One large entry and a tail 1e-9 of it: digits share an exponent over a
+    block's rows, and the basis stays orthonormal to the bound FP64 is held to."""
+    from mexk import synthetic as S
+    from mexk.api import Context
+
+    A = S.random_diag_dominant(n, 8, seed=3)
+    v = 1e-9 * np.random.default_rng(4).standard_normal(n)
+    v[n // 3] = 1.0
+    with Context(A, m_alloc=m) as ctx:
+        _, res = ctx.expmv(v, 1e-3 / A.max_abs(), m)
+        assert res["cycles"] == 1
+        V = ctx.get_basis(m)
+    assert np.abs(V @ V.T - np.eye(m)).max() < 1e-13
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("n,m", [(6000, 20), (150001, 21)])
+def test_non_finite_vector_breaks_down_at_once(n, m, bad):
+    from mexk import synthetic as S
+    from mexk.api import Context
+
+    A = S.random_diag_dominant(n, 8, seed=5)
+    v = np.random.default_rng(6).standard_normal(n)
+    with Context(A, m_alloc=m) as ctx:
+        y_ok, _ = ctx.expmv(v, 0.1, m)
+        w = v.copy()
+        w[n - 3] = bad
+        y, res = ctx.expmv(w, 0.1, m)
+        steps = ctx.steps()
+        y2, _ = ctx.expmv(v, 0.1, m)
+    assert not y.any() and res["converged"] == 1 and res["cycles"] == 1 and steps[0][3] == 1
+    assert np.array_equal(y_ok, y2)  # nothing of the failed solve is left behind
