@@ -34,9 +34,7 @@
 // shared memory; beyond, a cooperative grid with bounded waits (1.5 us) and
 // exact integer sums. A matrix whose products do not suit the kernel (long
 // rows, many entries) keeps the context's SpMV and takes one launch per step.
-#include "gram_step.cuh"
-
-#include <cooperative_groups.h>
+#include "cycle.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -53,128 +51,7 @@ constexpr int AC_CLUSTER = 16;
 // takes 17 us at 9,216 rows, where the cluster's FP64 work has doubled).
 constexpr int EXACT_ROWS = 4096;
 constexpr int AC_LONG_MAX = 2048;    // longest row (the product's block-wide rows are not built here)
-constexpr unsigned AC_FULL = 0xffffffffu;
-constexpr unsigned long long AC_WAIT_NS = 1000000000ull;
 constexpr int AC_PS = EXACT_ROWS / AC_SUB;  // a cluster's partials of one column
-
-// Testing hook (mexk_test_force_wait_timeout): when set, block 0 of a grid
-// waits 1 ms for an arrival that never comes before its first meeting, then
-// raises the abort word.
-__device__ int g_test_ac_dead_wait = 0;
-
-__device__ __forceinline__ unsigned long long ac_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// The blocks' meeting. A cluster: the hardware barrier (cluster-scope
-// release/acquire). A grid: an arrival counter that only grows (bar[0], the
-// next target in `target`), polled with a bounded wait; bar[1] is the abort
-// word. False when a wait gave up.
-template <bool CLUSTER>
-__device__ __forceinline__ bool ac_meet(unsigned* bar, unsigned& target, int* status, int* s_ok) {
-    if constexpr (CLUSTER) {
-        cooperative_groups::this_cluster().sync();
-        return true;
-    } else {
-        target += gridDim.x;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-            int ok = 1;
-            unsigned seen;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-            if (static_cast<int>(seen - target) < 0) {
-                const unsigned long long t0 = ac_ns();
-                do {
-                    unsigned aborted;
-                    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(aborted) : "l"(bar + 1) : "memory");
-                    if (aborted != 0u) {
-                        ok = 0;
-                        break;
-                    }
-                    if (ac_ns() - t0 > AC_WAIT_NS) {
-                        atomicExch(&bar[1], 1u);
-                        atomicOr(status, ST_TIMEOUT);
-                        ok = 0;
-                        break;
-                    }
-                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-                } while (static_cast<int>(seen - target) < 0);
-            }
-            *s_ok = ok;
-        }
-        __syncthreads();
-        return *s_ok != 0;
-    }
-}
-
-// ---- exact sums over the blocks of a grid -----------------------------------
-// A partial sum x becomes up to three 40-bit digits of the integer
-// x / 2^(scale - AC_TOP), added to three of its column's eight 64-bit words
-// by integer atomics: the words hold the exact sum of up to 2^23 blocks
-// whatever the order of arrival, and every block reads 8 words per column
-// instead of one partial per block and column (152 FP64 adds per column cost
-// more than the dots themselves). 2^scale bounds every |x|; what lies below
-// the last digit, 2^-318 of that bound, rounds off.
-constexpr int AC_DIGIT = 40;
-constexpr int AC_DIGITS = CYCLE_DIGITS;
-constexpr int AC_TOP = AC_DIGIT * AC_DIGITS - 2;
-constexpr long long AC_MASK = (1ll << AC_DIGIT) - 1;
-// The q-th (0..2) of x's digits, signed; *index its place.
-__device__ __forceinline__ long long ac_digit(double x, int scale, int q, int* index) {
-    const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(x));
-    const int e = static_cast<int>((u >> 52) & 0x7ff);
-    *index = 0;
-    if (e == 0) return 0;  // zero and subnormals
-    unsigned long long m = (u & 0xfffffffffffffull) | 0x10000000000000ull;
-    int p = e - 1075 - (scale - AC_TOP);  // bit position of m's last bit
-    if (p < 0) {
-        m = p > -54 ? (m + (1ull << (-p - 1))) >> -p : 0ull;
-        p = 0;
-    }
-    const int base = p / AC_DIGIT, off = p - base * AC_DIGIT;
-    *index = min(base + q, AC_DIGITS - 1);
-    const unsigned long long v = q == 0   ? (m << off) & AC_MASK
-                                 : q == 1 ? (m >> (AC_DIGIT - off)) & AC_MASK
-                                          : (off > 2 * AC_DIGIT - 54 ? m >> (2 * AC_DIGIT - off) : 0ull);
-    const long long sv = static_cast<long long>(v);
-    return (u >> 63) ? -sv : sv;
-}
-// The double of a column's digits: carries propagated and the sign taken out
-// first, then the three digits from the highest nonzero one (the roundings
-// are of non-negative terms).
-__device__ __forceinline__ double ac_value(long long (&d)[AC_DIGITS], int scale) {
-#pragma unroll
-    for (int i = 0; i + 1 < AC_DIGITS; ++i) {
-        d[i + 1] += d[i] >> AC_DIGIT;
-        d[i] &= AC_MASK;
-    }
-    const bool neg = d[AC_DIGITS - 1] < 0;
-    if (neg) {
-#pragma unroll
-        for (int i = 0; i < AC_DIGITS; ++i) d[i] = -d[i];
-#pragma unroll
-        for (int i = 0; i + 1 < AC_DIGITS; ++i) {
-            d[i + 1] += d[i] >> AC_DIGIT;
-            d[i] &= AC_MASK;
-        }
-    }
-    long long h2 = 0, h1 = 0, h0 = 0;
-    int top = 0;
-#pragma unroll
-    for (int i = 0; i < AC_DIGITS; ++i)
-        if (d[i] != 0) {
-            h2 = d[i];
-            h1 = i >= 1 ? d[i >= 1 ? i - 1 : 0] : 0;
-            h0 = i >= 2 ? d[i >= 2 ? i - 2 : 0] : 0;
-            top = i;
-        }
-    const double v = (static_cast<double>(h0) * 0x1p-80 + static_cast<double>(h1) * 0x1p-40) + static_cast<double>(h2);
-    const double r = ldexp(v, scale - AC_TOP + AC_DIGIT * top);
-    return neg ? -r : r;
-}
 
 // ---- warp reductions ---------------------------------------------------------
 // Lane-bit order of the separate sweeps of width 8, 16 or more columns.
@@ -398,28 +275,6 @@ __device__ __forceinline__ void ac_dot_task(const double* V, size_t ldv, int c0,
     }
 }
 
-// Adds column totals over the row slices (red[0..slices)) to the exchange's
-// words: four adjacent lanes per column.
-__device__ __forceinline__ void ac_publish(const AcExchange& ex, int k, int slices, int scale, AcShared& sh) {
-    for (int t = threadIdx.x; t < ((4 * k + 31) & ~31); t += AC_THREADS) {
-        const int c = min(t >> 2, k - 1), q = t & 3;
-        double s = q < slices ? sh.red[q][c] : 0.0;
-        for (int i = q + 4; i < slices; i += 4) s += sh.red[i][c];
-        s += __shfl_xor_sync(AC_FULL, s, 1);
-        s += __shfl_xor_sync(AC_FULL, s, 2);
-        if ((t >> 2) < k) {
-            const bool finite = (__double2hiint(s) & 0x7ff00000) != 0x7ff00000;
-            if (q < 3 && finite) {
-                int i;
-                const long long d = ac_digit(s, scale, q, &i);
-                if (d != 0) atomicAdd(ex.words + AC_DIGITS * c + i, static_cast<unsigned long long>(d));
-            } else if (q == 3 && !finite) {
-                atomicAdd(ex.words + AC_DIGITS * MEXK_M_MAX, 1ull);
-            }
-        }
-    }
-}
-
 // Dots of columns 0..k-1 of V with w over the block's rows into the exchange.
 // Warps take (group of up to eight columns, sub-block or row slice).
 template <int WIDTH, bool EXACT>
@@ -440,7 +295,7 @@ __device__ __forceinline__ void ac_dots(const CycleArgs& g, const double* V, int
     }
     if (!EXACT) {
         __syncthreads();
-        ac_publish(ex, k, slices, g.scale, sh);
+        ac_publish<AC_THREADS>(ex.words, &sh.red[0][0], MEXK_M_MAX + 1, k, slices, g.scale);
     }
 }
 
@@ -469,17 +324,7 @@ __device__ __forceinline__ void ac_sums(const AcExchange& ex, int k, int np, int
         }
     } else {
         for (int c = threadIdx.x; c < k; c += AC_THREADS) {
-            const ulonglong2* w = reinterpret_cast<const ulonglong2*>(ex.words + AC_DIGITS * c);
-            long long d[AC_DIGITS];
-#pragma unroll
-            for (int i = 0; i < AC_DIGITS; i += 2) {
-                const ulonglong2 p = __ldcg(w + i / 2);
-                d[i] = static_cast<long long>(p.x);
-                d[i + 1] = static_cast<long long>(p.y);
-            }
-            const bool finite = __ldcg(ex.words + AC_DIGITS * MEXK_M_MAX) == 0ull;
-            const double v = ac_value(d, scale);
-            out[c] = finite ? v : __longlong_as_double(0x7ff8000000000000ll);
+            out[c] = ac_collect(ex.words, c, scale);
         }
     }
     __syncthreads();
@@ -778,7 +623,7 @@ __device__ __forceinline__ void ac_dots_digits(const CycleArgs& g, int lo, int k
         else ac_digit_task<1>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
     }
     __syncthreads();
-    ac_publish(ex, k, slices, g.scale, sh);
+    ac_publish<AC_THREADS>(ex.words, &sh.red[0][0], MEXK_M_MAX + 1, k, slices, g.scale);
 }
 
 // Column c of the basis into digits from the block's rows of the FP64 column
@@ -1005,16 +850,7 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
     };
     exchanges(0);
     if (CLUSTER) cooperative_groups::this_cluster().sync();  // every block runs before another writes to its memory
-    if (!CLUSTER && lead && g_test_ac_dead_wait != 0) {
-        if (threadIdx.x == 0) {
-            const unsigned long long t0 = ac_ns();
-            while (ac_ns() - t0 < 1000000ull) {
-            }
-            atomicOr(&st->status, ST_TIMEOUT);
-            atomicExch(&g.bar[1], 1u);
-        }
-        return;
-    }
+    if (!CLUSTER && lead && ac_test_dead_wait(&st->status, g.bar)) return;
     for (int j = g.j0; j < g.j1; ++j) {
         const int lo = g.window > 0 ? max(0, j + 1 - g.window) : 0;
         const int k = j + 1 - lo;

@@ -478,6 +478,32 @@ struct GramArgs {
     int sym = 0;
     DevState* st;
 };
+// All m steps of an FP32 basis in one launch (gram_cycle.cu): V[:,0] given,
+// V, H, the Gram state and the solver state written as the stepwise kernels
+// do, H(m, m-1) included. scale, bar, words: as CycleArgs. The products come
+// from the row patterns (pid, T) or the FP32 CSR arrays.
+struct GramCycleArgs {
+    int n, m, ldv, ldh, reortho, window;
+    int rows = 0, on = 0;  // rows per block, columns held on chip (the launch's)
+    int scale;
+    int max_len;           // of the row patterns
+    int long_rows;         // whether a CSR row has more than SEQ_ROW_MAX entries
+    const int* row_ptr;
+    const int* col_idx;
+    const float* values;
+    const uint8_t* pid;
+    const RowPatterns* T;
+    float* V;
+    double* H;
+    GramState* gs;
+    DevState* st;
+    unsigned* bar;
+    unsigned long long* words;
+};
+bool gram_cycle_fits(int n, long long nnz, int m, int max_row, bool pattern, int window);
+int gram_cycle_prepare();
+int launch_gram_cycle(GramCycleArgs a, cudaStream_t s);
+int gram_cycle_test_hook(int enable);  // as arnoldi_cycle_test_hook
 int device_sm_count();
 int launch_gram_dot(const GramArgs& a, cudaStream_t s);
 int launch_gram_update(const GramArgs& a, cudaStream_t s);

@@ -536,6 +536,37 @@ int enqueue_arnoldi_cycle(mexk_context_t ctx, int m, int reortho, int window, cu
     return MEXK_OK;
 }
 
+// Whether an FP32 basis is built in one launch by gram_cycle.cu.
+bool use_gram_cycle(mexk_context_t ctx, int m, int window) {
+    return ctx->cycle_scale != INT_MAX && !use_lanczos_cycle(ctx, m, true, window) &&
+           gram_cycle_fits(ctx->n, ctx->nnz, m, ctx->max_row, ctx->spmv_form32 == MEXK_SPMV_PATTERN, window);
+}
+
+int enqueue_gram_cycle(mexk_context_t ctx, int m, int reortho, int window, cudaStream_t s) {
+    GramCycleArgs a;
+    a.n = ctx->n;
+    a.m = m;
+    a.ldv = ctx->ldv;
+    a.ldh = ctx->ldh;
+    a.reortho = reortho ? 1 : 0;
+    a.window = window;
+    a.scale = ctx->cycle_scale;
+    a.max_len = ctx->pat_max_len;
+    a.long_rows = ctx->max_row > SEQ_ROW_MAX ? 1 : 0;
+    a.row_ptr = ctx->d_row_ptr;
+    a.col_idx = ctx->d_col;
+    a.values = ctx->d_val32;
+    a.pid = ctx->spmv_form32 == MEXK_SPMV_PATTERN ? ctx->d_pid : nullptr;
+    a.T = ctx->d_pat;
+    a.V = ctx->d_V32;
+    a.H = ctx->d_H;
+    a.gs = ctx->d_gram;
+    a.st = ctx->d_state;
+    a.bar = ctx->d_bar;
+    a.words = reinterpret_cast<unsigned long long*>(ctx->d_bar + BAR_WORDS);
+    return launch_gram_cycle(a, s);
+}
+
 // One Krylov cycle: the unit that is captured into a graph.
 template <typename TV>
 int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, cudaStream_t s) {
@@ -546,8 +577,11 @@ int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, 
     if (!fp32 && window > 0)
         MEXK_CK(cudaMemsetAsync(ctx->d_H, 0, sizeof(double) * static_cast<size_t>(ctx->ldh) * m, s));
     const bool fused = use_lanczos_cycle(ctx, m, fp32, window);
+    const bool onchip = fp32 && use_gram_cycle(ctx, m, window);
     if (!fp32 && use_arnoldi_cycle(ctx)) {
         if ((rc = enqueue_arnoldi_cycle(ctx, m, reortho, window, s))) return rc;
+    } else if (onchip) {
+        if ((rc = enqueue_gram_cycle(ctx, m, reortho, window, s))) return rc;
     } else if (fused) {
         // step 0 as two kernels (its update writes step 1's b and a_0 partials), then the rest in one launch
         if ((rc = enqueue_step(ctx, 0, reortho, fp32, s, window, m))) return rc;
@@ -557,7 +591,7 @@ int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, 
             if ((rc = enqueue_step(ctx, j, reortho, fp32, s, window, m))) return rc;
     }
     // the stepwise basis's last update left |u_m|^2 as partials where it could
-    if ((rc = finish_basis(ctx, m - 1, fp32, s, !fused && fp32 && norm_from_update(m, window)))) return rc;
+    if (!onchip && (rc = finish_basis(ctx, m - 1, fp32, s, !fused && fp32 && norm_from_update(m, window)))) return rc;
     if ((rc = enqueue_controller(ctx, m, ctrl, ctx->d_log, s, window))) return rc;
     const LiftArgs l = lift_args(ctx, fp32);
     if ((rc = launch_lift<TV>(l, gs_grid_size(ctx->n, 1), s))) return rc;
@@ -924,6 +958,7 @@ int mexk_context_create(int device, mexk_context_t* out) {
     // without its shared memory the fused Lanczos form stays off (lanczos_cycle_fits says no)
     if (rc == MEXK_OK && lanczos_cycle_prepare() != MEXK_OK) (void)cudaGetLastError();
     if (rc == MEXK_OK) rc = arnoldi_cycle_prepare();
+    if (rc == MEXK_OK) rc = gram_cycle_prepare();
     gs_prepare();
     if (rc) {
         cudaStreamDestroy(c->stream);

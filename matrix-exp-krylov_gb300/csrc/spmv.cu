@@ -961,6 +961,7 @@ extern "C" int mexk_test_force_wait_timeout(int device, int enable) {
     MEXK_CK(cudaMemcpyToSymbol(mexk::g_test_dead_wait, &v, sizeof(int)));
     int rc = mexk::lanczos_cycle_test_hook(enable);
     if (rc == MEXK_OK) rc = mexk::arnoldi_cycle_test_hook(enable);
+    if (rc == MEXK_OK) rc = mexk::gram_cycle_test_hook(enable);
     if (rc != MEXK_OK) return rc;
     MEXK_CK(cudaDeviceSynchronize());
     return MEXK_OK;

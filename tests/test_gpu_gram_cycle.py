@@ -1,0 +1,112 @@
+"""The one-launch FP32 basis (rows on chip, Gram-corrected steps) around the
+edges of its sub-blocks (128 rows), blocks (32), the cluster (4096 rows) and
+the grid, with columns on and off chip, for each form of the product, with and
+without reorthogonalisation and with a window.
+
+With u = 2^-24, rows of at most 64 entries and at most 64 columns, one step's
+rounding is bounded by (64 + 64 + 4) u ||A||v_j||: the product's and the
+update's sums. That bounds A v_j's distance from the span of the columns; the
+loss of orthogonality is the same divided by what the projection leaves of
+A v_j."""
+import numpy as np
+import pytest
+
+from test_gpu_arnoldi_cycle import make
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -24
+
+CASES = [("random", n, 12, 1, 0) for n in (14, 64, 129, 511, 512, 513, 2000, 2047, 4095, 4096, 4097, 4865, 9729, 20011)]
+CASES += [("random", 2000, 1, 1, 0), ("random", 2000, 33, 1, 0), ("random", 2000, 64, 1, 0), ("random", 9000, 64, 1, 0),
+          ("random", 2000, 20, 0, 0), ("random", 30000, 9, 0, 0), ("random", 120001, 30, 1, 0),
+          ("random", 300007, 40, 1, 0), ("powerlaw", 2048, 20, 1, 0), ("powerlaw", 12345, 20, 1, 0),
+          ("longrow", 2000, 8, 1, 0), ("longrow", 6000, 8, 1, 0), ("heat", 7, 30, 1, 0), ("heat", 64, 30, 1, 3),
+          ("heat", 64, 20, 0, 3), ("heat", 131, 17, 1, 0), ("heat", 131, 30, 1, 5), ("heat", 401, 40, 1, 0)]
+
+
+@pytest.mark.parametrize("kind,n,m,reortho,window", CASES)
+def test_basis(kind, n, m, reortho, window):
+    import scipy.sparse as sp
+
+    from mexk.api import Context
+
+    A = make(kind, n)
+    n = A.n
+    v = np.random.default_rng(n).standard_normal(n)
+    t = 1e-3 / A.max_abs()  # one accepted step: the context keeps that cycle's basis
+    with Context(A, m_alloc=m) as ctx:
+        y, res = ctx.expmv(v, t, m, precision="mixed", controller="search", reorthogonalize=bool(reortho),
+                           window=window)
+        assert res["cycles"] == 1
+        V = ctx.get_basis(m + 1, "mixed")
+        y2, _ = ctx.expmv(v, t, m, precision="mixed", controller="search", reorthogonalize=bool(reortho),
+                          window=window)
+    assert np.array_equal(y, y2)
+    M = sp.csr_matrix((A.values, A.col_idx, A.row_ptr), shape=(n, n))
+    longest = int(np.diff(A.row_ptr).max())
+    step = (min(longest, 64) + longest // 32 + m + 4) * U
+    for j in range(m):
+        lo = max(0, j + 1 - window) if window else 0
+        B = V[lo:j + 2]
+        w = M @ V[j]
+        size = np.linalg.norm(abs(M) @ np.abs(V[j]))
+        coef = np.linalg.lstsq(B.T, w, rcond=None)[0]
+        assert np.linalg.norm(w - B.T @ coef) <= step * size
+        left = abs(coef[-1])
+        loss = np.abs(B @ B.T - np.eye(len(B)))[-1].max()
+        if reortho:
+            assert loss <= 4 * U + step * size / left, j
+    if m == 1:
+        return  # one column does not reach the bound below
+    ref, term = v.copy(), v.copy()
+    for i in range(1, 12):  # |tA| < 0.1
+        term = (t / i) * (M @ term)
+        ref += term
+    assert np.linalg.norm(y - ref) <= 1e-6 * np.linalg.norm(ref)  # the mixed form's bound
+
+
+@pytest.mark.parametrize("n", [3000, 6000])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_vector_breaks_down_at_once(n, bad):
+    from mexk import synthetic as S
+    from mexk.api import Context
+
+    A = S.random_diag_dominant(n, 8, seed=5)
+    v = np.random.default_rng(6).standard_normal(n)
+    with Context(A, m_alloc=20) as ctx:
+        good, _ = ctx.expmv(v, 0.1, 20, precision="mixed", controller="search")
+        w = v.copy()
+        w[n // 2] = bad
+        try:
+            y, _ = ctx.expmv(w, 0.1, 20, precision="mixed", controller="search")
+            assert not np.isfinite(y).all()
+        except Exception:
+            pass
+        again, _ = ctx.expmv(v, 0.1, 20, precision="mixed", controller="search")
+    assert np.array_equal(good, again)
+
+
+@pytest.mark.parametrize("n", [2000, 6000])
+def test_invariant_subspace_breaks_down(n):
+    """A = diag + a cycle of five rows; a start vector inside them spans five columns."""
+    import scipy.sparse as sp
+
+    from mexk import synthetic as S
+    from mexk.api import Context
+
+    M = sp.lil_matrix((n, n))
+    M.setdiag(-1.0)
+    for i in range(5):
+        M[n // 2 + i, n // 2 + (i + 1) % 5] = 0.5
+    M = M.tocsr()
+    M.sort_indices()
+    A = S.CSR(n, M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data)
+    v = np.zeros(n)
+    v[n // 2] = 2.0
+    with Context(A, m_alloc=20) as ctx:
+        y, _ = ctx.expmv(v, 1.0, 20, precision="mixed", controller="search")
+    ref, term = v.copy(), v.copy()
+    for i in range(1, 40):
+        term = (1.0 / i) * (M @ term)
+        ref += term
+    assert np.linalg.norm(y - ref) <= 1e-6 * np.linalg.norm(ref)
