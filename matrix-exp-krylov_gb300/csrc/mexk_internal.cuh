@@ -503,6 +503,30 @@ struct GramCycleArgs {
 bool gram_cycle_fits(int n, long long nnz, int m, int max_row, bool pattern, int window);
 int gram_cycle_prepare();
 int launch_gram_cycle(GramCycleArgs a, cudaStream_t s);
+// The same for a window of 2 on a symmetric matrix in the row-pattern form
+// (stencil_cycle.cu): off, val: the len entries of the pattern with the most
+// rows; reach: the largest |offset| of any pattern.
+constexpr int STENCIL_LEN = 7;
+struct StencilArgs {
+    int n, m, ldv, ldh, reortho;
+    int rows = 0;
+    int scale;
+    int len, reach;
+    int off[STENCIL_LEN];
+    float val[STENCIL_LEN];
+    const uint8_t* pid;
+    const RowPatterns* T;
+    float* V;
+    double* H;
+    GramState* gs;
+    DevState* st;
+    unsigned* bar;
+    unsigned long long* words;
+};
+bool stencil_cycle_fits(int n, int m, int len, int reach);
+int stencil_cycle_prepare();
+int launch_stencil_cycle(StencilArgs a, cudaStream_t s);
+int stencil_cycle_test_hook(int enable);
 int gram_cycle_test_hook(int enable);  // as arnoldi_cycle_test_hook
 int device_sm_count();
 int launch_gram_dot(const GramArgs& a, cudaStream_t s);

@@ -104,6 +104,9 @@ struct mexk_context_s {
     int pat_major = 0;  // the pattern with the most rows, and its length
     int pat_major_len = 0;
     int pat_max_len = 0;
+    int pat_reach = 0;             // the largest |offset| of any pattern
+    int pat_off[PAT_LEN] = {};     // the major pattern's entries
+    float pat_val[PAT_LEN] = {};
     double* d_V = nullptr;
     float* d_V32 = nullptr;
     unsigned long long* d_vq = nullptr;  // the FP64 basis in digits (arnoldi_cycle.cu), and its exponents
@@ -536,9 +539,16 @@ int enqueue_arnoldi_cycle(mexk_context_t ctx, int m, int reortho, int window, cu
     return MEXK_OK;
 }
 
-// Whether an FP32 basis is built in one launch by gram_cycle.cu.
+// Whether an FP32 basis is built in one launch, by stencil_cycle.cu (a window
+// of 2) or gram_cycle.cu (up to 4096 rows, where its blocks are a cluster,
+// also for a window of 2).
+bool use_stencil_cycle(mexk_context_t ctx, int m, int window) {
+    return window == 2 && ctx->n > 4096 && ctx->spmv_form32 == MEXK_SPMV_PATTERN &&
+           stencil_cycle_fits(ctx->n, m, ctx->pat_major_len, ctx->pat_reach);
+}
 bool use_gram_cycle(mexk_context_t ctx, int m, int window) {
-    return ctx->cycle_scale != INT_MAX && !use_lanczos_cycle(ctx, m, true, window) &&
+    if (ctx->cycle_scale == INT_MAX || use_lanczos_cycle(ctx, m, true, window)) return false;
+    return use_stencil_cycle(ctx, m, window) ||
            gram_cycle_fits(ctx->n, ctx->nnz, m, ctx->max_row, ctx->spmv_form32 == MEXK_SPMV_PATTERN, window);
 }
 
@@ -567,6 +577,31 @@ int enqueue_gram_cycle(mexk_context_t ctx, int m, int reortho, int window, cudaS
     return launch_gram_cycle(a, s);
 }
 
+int enqueue_stencil_cycle(mexk_context_t ctx, int m, int reortho, cudaStream_t s) {
+    StencilArgs a;
+    a.n = ctx->n;
+    a.m = m;
+    a.ldv = ctx->ldv;
+    a.ldh = ctx->ldh;
+    a.reortho = reortho ? 1 : 0;
+    a.scale = ctx->cycle_scale;
+    a.len = ctx->pat_major_len;
+    a.reach = ctx->pat_reach;
+    for (int q = 0; q < STENCIL_LEN; ++q) {
+        a.off[q] = q < a.len ? ctx->pat_off[q] : 0;
+        a.val[q] = q < a.len ? ctx->pat_val[q] : 0.f;
+    }
+    a.pid = ctx->d_pid;
+    a.T = ctx->d_pat;
+    a.V = ctx->d_V32;
+    a.H = ctx->d_H;
+    a.gs = ctx->d_gram;
+    a.st = ctx->d_state;
+    a.bar = ctx->d_bar;
+    a.words = reinterpret_cast<unsigned long long*>(ctx->d_bar + BAR_WORDS);
+    return launch_stencil_cycle(a, s);
+}
+
 // One Krylov cycle: the unit that is captured into a graph.
 template <typename TV>
 int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, cudaStream_t s) {
@@ -581,7 +616,9 @@ int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, 
     if (!fp32 && use_arnoldi_cycle(ctx)) {
         if ((rc = enqueue_arnoldi_cycle(ctx, m, reortho, window, s))) return rc;
     } else if (onchip) {
-        if ((rc = enqueue_gram_cycle(ctx, m, reortho, window, s))) return rc;
+        rc = use_stencil_cycle(ctx, m, window) ? enqueue_stencil_cycle(ctx, m, reortho, s)
+                                               : enqueue_gram_cycle(ctx, m, reortho, window, s);
+        if (rc) return rc;
     } else if (fused) {
         // step 0 as two kernels (its update writes step 1's b and a_0 partials), then the rest in one launch
         if ((rc = enqueue_step(ctx, 0, reortho, fp32, s, window, m))) return rc;
@@ -885,7 +922,24 @@ int context_csr_finish(mexk_context_t ctx, const int* row_ptr) {
                                  &ctx->pat_max_len, ctx->stream)))
         return rc;
     MEXK_CK(cudaMemsetAsync(&ctx->d_state->status, 0, sizeof(int), ctx->stream));
+    std::vector<int> pat_len(PAT_MAX), pat_off(PAT_MAX * PAT_LEN);
+    int pat_count = 0;
+    if (pat_ok) {
+        const size_t at = static_cast<size_t>(ctx->pat_major) * PAT_LEN;
+        MEXK_CK(cudaMemcpyAsync(&pat_count, &ctx->d_pat->count, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        MEXK_CK(cudaMemcpyAsync(pat_len.data(), ctx->d_pat->len, sizeof(int) * PAT_MAX, cudaMemcpyDeviceToHost,
+                                ctx->stream));
+        MEXK_CK(cudaMemcpyAsync(pat_off.data(), ctx->d_pat->off, sizeof(int) * PAT_MAX * PAT_LEN,
+                                cudaMemcpyDeviceToHost, ctx->stream));
+        MEXK_CK(cudaMemcpyAsync(ctx->pat_val, ctx->d_pat->v32 + at, sizeof(float) * PAT_LEN, cudaMemcpyDeviceToHost,
+                                ctx->stream));
+    }
     MEXK_CK(cudaStreamSynchronize(ctx->stream));
+    ctx->pat_reach = 0;
+    for (int p = 0; p < std::min(pat_count, PAT_MAX); ++p)
+        for (int q = 0; q < std::min(pat_len[p], PAT_LEN); ++q)
+            ctx->pat_reach = std::max(ctx->pat_reach, std::abs(pat_off[p * PAT_LEN + q]));
+    for (int q = 0; pat_ok && q < PAT_LEN; ++q) ctx->pat_off[q] = pat_off[ctx->pat_major * PAT_LEN + q];
     {
         // |A x|_2 <= sqrt(n) |A x|_inf <= sqrt(n) |A|_inf for |x|_2 = 1
         double norm;
@@ -959,6 +1013,7 @@ int mexk_context_create(int device, mexk_context_t* out) {
     if (rc == MEXK_OK && lanczos_cycle_prepare() != MEXK_OK) (void)cudaGetLastError();
     if (rc == MEXK_OK) rc = arnoldi_cycle_prepare();
     if (rc == MEXK_OK) rc = gram_cycle_prepare();
+    if (rc == MEXK_OK) rc = stencil_cycle_prepare();
     gs_prepare();
     if (rc) {
         cudaStreamDestroy(c->stream);

@@ -962,6 +962,7 @@ extern "C" int mexk_test_force_wait_timeout(int device, int enable) {
     int rc = mexk::lanczos_cycle_test_hook(enable);
     if (rc == MEXK_OK) rc = mexk::arnoldi_cycle_test_hook(enable);
     if (rc == MEXK_OK) rc = mexk::gram_cycle_test_hook(enable);
+    if (rc == MEXK_OK) rc = mexk::stencil_cycle_test_hook(enable);
     if (rc != MEXK_OK) return rc;
     MEXK_CK(cudaDeviceSynchronize());
     return MEXK_OK;

@@ -11,10 +11,30 @@ A v_j."""
 import numpy as np
 import pytest
 
-from test_gpu_arnoldi_cycle import make
+from test_gpu_arnoldi_cycle import make as make_general
 
 pytestmark = pytest.mark.gpu
 U = 2.0 ** -24
+
+
+def make(kind, n):
+    """heat3d: a 7-point stencil on n^3 points. patches: a 5-point one on n^2 with another
+    diagonal on some rows (patterns that are no part of the main one)."""
+    import scipy.sparse as sp
+
+    from mexk import synthetic as S
+
+    if kind not in ("heat3d", "patches"):
+        return make_general(kind, n)
+    T = sp.diags([np.ones(n - 1), np.full(n, -2.0), np.ones(n - 1)], [-1, 0, 1])
+    one = sp.identity(n)
+    if kind == "heat3d":
+        M = sp.kron(sp.kron(T, one), one) + sp.kron(sp.kron(one, T), one) + sp.kron(sp.kron(one, one), T)
+    else:
+        M = sp.kron(T, one) + sp.kron(one, T) - sp.diags(np.random.default_rng(n).integers(0, 12, n * n) // 11 * 0.5)
+    M = sp.csr_matrix(M)
+    M.sort_indices()
+    return S.CSR(M.shape[0], M.indptr.astype(np.int32), M.indices.astype(np.int32), M.data)
 
 CASES = [("random", n, 12, 1, 0) for n in (14, 64, 129, 511, 512, 513, 2000, 2047, 4095, 4096, 4097, 4865, 9729, 20011)]
 CASES += [("random", 2000, 1, 1, 0), ("random", 2000, 33, 1, 0), ("random", 2000, 64, 1, 0), ("random", 9000, 64, 1, 0),
@@ -22,6 +42,11 @@ CASES += [("random", 2000, 1, 1, 0), ("random", 2000, 33, 1, 0), ("random", 2000
           ("random", 300007, 40, 1, 0), ("powerlaw", 2048, 20, 1, 0), ("powerlaw", 12345, 20, 1, 0),
           ("longrow", 2000, 8, 1, 0), ("longrow", 6000, 8, 1, 0), ("heat", 7, 30, 1, 0), ("heat", 64, 30, 1, 3),
           ("heat", 64, 20, 0, 3), ("heat", 131, 17, 1, 0), ("heat", 131, 30, 1, 5), ("heat", 401, 40, 1, 0)]
+# a window of 2 in the row-pattern form: the recurrence on chip past 4096 rows (blocks of one edge, of two, with
+# row groups between them; a stencil that reaches past the edges)
+CASES += [("heat", N, 30, 1, 2) for N in (64, 65, 97, 131, 556, 700, 801, 1303)]
+CASES += [("heat", 300, 2, 1, 2), ("heat", 300, 64, 1, 2), ("heat", 801, 20, 0, 2), ("heat3d", 31, 20, 1, 2),
+          ("heat3d", 40, 20, 1, 2), ("heat3d", 100, 20, 1, 2), ("patches", 150, 20, 1, 2), ("patches", 801, 20, 1, 2)]
 
 
 @pytest.mark.parametrize("kind,n,m,reortho,window", CASES)
@@ -56,8 +81,8 @@ def test_basis(kind, n, m, reortho, window):
         loss = np.abs(B @ B.T - np.eye(len(B)))[-1].max()
         if reortho:
             assert loss <= 4 * U + step * size / left, j
-    if m == 1:
-        return  # one column does not reach the bound below
+    if m <= 2:
+        return  # one or two columns do not reach the bound below
     ref, term = v.copy(), v.copy()
     for i in range(1, 12):  # |tA| < 0.1
         term = (t / i) * (M @ term)
@@ -110,3 +135,25 @@ def test_invariant_subspace_breaks_down(n):
         term = (1.0 / i) * (M @ term)
         ref += term
     assert np.linalg.norm(y - ref) <= 1e-6 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("kind,window", [("random", 0), ("heat", 2)])
+def test_wait_that_runs_out_reports_and_the_context_survives(kind, window):
+    """Block 0 leaves before the first meeting: the others' waits end, the solve
+    reports it, and the same context then solves as before."""
+    from mexk._lib import MexkError, check, lib
+    from mexk.api import Context
+
+    A = make(kind, 300 if kind == "heat" else 20000)
+    v = np.random.default_rng(8).standard_normal(A.n)
+    t = 1.0 / A.max_abs()
+    with Context(A, m_alloc=20) as ctx:
+        good, _ = ctx.expmv(v, t, 20, precision="mixed", controller="search", window=window)
+        check(lib().mexk_test_force_wait_timeout(0, 1))
+        try:
+            with pytest.raises(MexkError, match="device wait gave up"):
+                ctx.expmv(v, t, 20, precision="mixed", controller="search", window=window)
+        finally:
+            check(lib().mexk_test_force_wait_timeout(0, 0))
+        again, _ = ctx.expmv(v, t, 20, precision="mixed", controller="search", window=window)
+    assert np.array_equal(good, again)
