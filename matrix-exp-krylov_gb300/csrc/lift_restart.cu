@@ -97,7 +97,6 @@ __global__ void __launch_bounds__(LIFT_THREADS, LIFT_BLOCKS_PER_SM) lift_kernel(
     __shared__ double s_coef[MEXK_M_MAX + 1];
     __shared__ float s_coef32[MEXK_M_MAX + 1];
     __shared__ double s_red[32];
-    __shared__ double s_out[1];
     __shared__ double s_scratch[LIFT_THREADS];
     __shared__ int s_flag;
     // launched as a dependent of the controller: its state and coefficients
@@ -151,9 +150,9 @@ __global__ void __launch_bounds__(LIFT_THREADS, LIFT_BLOCKS_PER_SM) lift_kernel(
         a.partials[static_cast<size_t>(blockIdx.x) * RED_STRIDE] = t;
     }
     if (!grid_last_block(a.counter, &s_flag)) return;
-    reduce_partials(a.partials, gridDim.x, 1, s_out, s_scratch);
+    const double y2 = reduce_column(a.partials, gridDim.x, s_scratch);
     if (threadIdx.x == 0) {
-        const double nrm = sqrt(s_out[0]);
+        const double nrm = sqrt(y2);
         st->restart_scale = nrm > 1e-14 ? 1.0 / nrm : 1.0;
         if (st->restart) st->v_norm = nrm;
         st->lift = 0;
@@ -165,7 +164,6 @@ __global__ void __launch_bounds__(LIFT_THREADS)
     start_norm_kernel(int n, const double* __restrict__ x, double* partials, unsigned int* counter,
                       DevState* st) {
     __shared__ double s_red[32];
-    __shared__ double s_out[1];
     __shared__ double s_scratch[LIFT_THREADS];
     __shared__ int s_flag;
     double nacc = 0.0;
@@ -180,9 +178,9 @@ __global__ void __launch_bounds__(LIFT_THREADS)
         partials[static_cast<size_t>(blockIdx.x) * RED_STRIDE] = t;
     }
     if (!grid_last_block(counter, &s_flag)) return;
-    reduce_partials(partials, gridDim.x, 1, s_out, s_scratch);
+    const double x2 = reduce_column(partials, gridDim.x, s_scratch);
     if (threadIdx.x == 0) {
-        const double nrm = sqrt(s_out[0]);
+        const double nrm = sqrt(x2);
         st->v_norm = nrm;
         st->restart_scale = nrm > 1e-14 ? 1.0 / nrm : 1.0;
     }

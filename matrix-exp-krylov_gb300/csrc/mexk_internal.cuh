@@ -265,6 +265,35 @@ __device__ __forceinline__ void reduce_partials(const double* partials, int nblo
     __syncthreads();
 }
 
+// The same for one column in every thread's loads and a tree (an FP64 add
+// takes 64 cycles: one thread over 256 running sums took 8 us). Up to 32
+// blocks, whose sums are those of reduce_partials bit for bit, one thread adds
+// them in order.
+__device__ __forceinline__ double reduce_column(const double* partials, int nblocks, double* scratch) {
+    const int t = threadIdx.x, nt = static_cast<int>(blockDim.x);
+    double s = 0.0;
+    {
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+        int b = t;
+        for (; b + 3 * nt < nblocks; b += 4 * nt) {
+            s0 += __ldcg(&partials[(size_t)b * RED_STRIDE]);
+            s1 += __ldcg(&partials[(size_t)(b + nt) * RED_STRIDE]);
+            s2 += __ldcg(&partials[(size_t)(b + 2 * nt) * RED_STRIDE]);
+            s3 += __ldcg(&partials[(size_t)(b + 3 * nt) * RED_STRIDE]);
+        }
+        for (; b < nblocks; b += nt) s0 += __ldcg(&partials[(size_t)b * RED_STRIDE]);
+        s = (s0 + s1) + (s2 + s3);
+    }
+    if (nblocks > 32) s = warp_sum(s);
+    if (nblocks <= 32 || (t & 31) == 0) scratch[nblocks <= 32 ? t : t >> 5] = s;
+    __syncthreads();
+    double tot = 0.0;
+    if (t == 0)
+        for (int q = 0; q < min(nblocks, 32) && q < (nblocks <= 32 ? nt : nt >> 5); ++q) tot += scratch[q];
+    __syncthreads();
+    return tot;  // thread 0's
+}
+
 // ------------------------------------------------------------ SpMV
 // Row-block schedule: rows [blocks[b], blocks[b+1]) form block b. A block
 // holds <= tile nonzeros and <= tile_rows rows, or one longer row.
