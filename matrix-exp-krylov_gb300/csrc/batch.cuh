@@ -32,11 +32,11 @@ constexpr int B_OFF = BR * BM_MAX;         //                     b[c][r]
 constexpr int W_OFF = 2 * BR * BM_MAX;     //                     |w|^2[r] (or |y|^2[r])
 constexpr int BPS = 2 * BR * BM_MAX + BR;  // doubles per tile partial (1040)
 
-// Rows per piece of the streaming sweeps (update, lift, last norms, restart),
+// Rows per piece of the streaming sweeps (lift, last norms, restart),
 // whatever tile the dot sweep's autotuner picked: with its 16384-row tiles a
-// 380,000-row batch gave those sweeps 30 blocks on 152 SMs (update 255 us a
-// step, 62 us in pieces of 512 rows; the lift 780 and 150 us). A constant, so
-// that the norms' sums do not depend on the wave or the tuner.
+// 380,000-row batch gave those sweeps 30 blocks on 152 SMs (the lift 780 us,
+// 150 us in pieces of 512 rows). A constant, so that the norms' sums do not
+// depend on the wave or the tuner.
 constexpr int PIECE_ROWS = 512;
 
 struct Layout {

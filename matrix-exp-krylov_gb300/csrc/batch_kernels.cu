@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(BT, 3) dot_kernel(Layout L, int j, int reortho
 // ---------------------------------------------------------------- update sweep
 constexpr int UCH = 8;
 
-__global__ void __launch_bounds__(BT) update_kernel(Layout L, int j) {
+__global__ void __launch_bounds__(BT, 4) update_kernel(Layout L, int j) {
     const int k = j + 1;
     const int q = threadIdx.x & 3;
     const int rl = threadIdx.x >> 2;
@@ -328,45 +328,52 @@ __global__ void __launch_bounds__(BT) update_kernel(Layout L, int j) {
     __shared__ float4 ssc[2][4];
     const float4* __restrict__ W4 = reinterpret_cast<const float4*>(L.W);
     float4* __restrict__ Out = reinterpret_cast<float4*>(L.U + static_cast<size_t>(j + 1) * L.ldu);
-    for (int piece = blockIdx.x; piece < L.N; piece += gridDim.x) {
-        const int p = L.piece_prob[piece];
+    // a contiguous share of the wave's 64-row chunks per block, in one wave of
+    // blocks (660 pieces of 512 rows on 608 resident blocks ran as two: 85 us a
+    // step, now 55)
+    const int chunks = L.C1 - L.C0;
+    const int ch0 = L.C0 + static_cast<int>(static_cast<long long>(chunks) * blockIdx.x / gridDim.x);
+    const int ch1 = L.C0 + static_cast<int>(static_cast<long long>(chunks) * (blockIdx.x + 1) / gridDim.x);
+    int cur = -1;
+    float4 wsc = zero4(), psc = zero4();
+    for (int ch = ch0; ch < ch1; ++ch) {
+        const int p = L.chunk_prob[ch];
         if (L.pdone[p]) continue;
-        __syncthreads();
-        for (int v = threadIdx.x; v < BM_MAX * BR; v += BT) {
-            const int c = v / BR;
-            const int r = v - c * BR;
-            reinterpret_cast<float*>(sco)[v] = (c < k) ? L.coef[static_cast<size_t>(p * BR + r) * BLD + c] : 0.f;
-        }
-        if (threadIdx.x < BR) {
-            reinterpret_cast<float*>(ssc)[threadIdx.x] = L.wsc[p * BR + threadIdx.x];
-            reinterpret_cast<float*>(ssc)[BR + threadIdx.x] = L.psc[p * BR + threadIdx.x];
-        }
-        __syncthreads();
-        const float4 wsc = ssc[0][q];
-        const float4 psc = ssc[1][q];
-        const long long base = L.piece_row0[piece] - L.R0;
-        const int nr = L.piece_nrows[piece];
-        for (int r = rl; r < nr; r += BROWS) {
-            const size_t i = static_cast<size_t>(base + r) * 4 + q;
-            const float4 x = __ldg(W4 + i);
-            float4 s = zero4();
-#pragma unroll
-            for (int cb = 0; cb < BM_MAX; cb += UCH) {
-                if (cb < k) {
-                    float4 v[UCH];
-#pragma unroll
-                    for (int c = 0; c < UCH; ++c) v[c] = (cb + c < k) ? __ldcs(col4(L, cb + c) + i) : zero4();
-#pragma unroll
-                    for (int c = 0; c < UCH; ++c) fma4(s, v[c], sco[cb + c][q]);
-                }
+        if (p != cur) {
+            cur = p;
+            __syncthreads();
+            for (int v = threadIdx.x; v < BM_MAX * BR; v += BT) {
+                const int c = v / BR;
+                const int r = v - c * BR;
+                reinterpret_cast<float*>(sco)[v] = (c < k) ? L.coef[static_cast<size_t>(p * BR + r) * BLD + c] : 0.f;
             }
-            float4 o;
-            o.x = fmaf(x.x, wsc.x, -s.x) * psc.x;
-            o.y = fmaf(x.y, wsc.y, -s.y) * psc.y;
-            o.z = fmaf(x.z, wsc.z, -s.z) * psc.z;
-            o.w = fmaf(x.w, wsc.w, -s.w) * psc.w;
-            Out[i] = o;
+            if (threadIdx.x < BR) {
+                reinterpret_cast<float*>(ssc)[threadIdx.x] = L.wsc[p * BR + threadIdx.x];
+                reinterpret_cast<float*>(ssc)[BR + threadIdx.x] = L.psc[p * BR + threadIdx.x];
+            }
+            __syncthreads();
+            wsc = ssc[0][q];
+            psc = ssc[1][q];
         }
+        const size_t i = static_cast<size_t>(static_cast<long long>(ch) * BROWS - L.R0 + rl) * 4 + q;
+        const float4 x = __ldg(W4 + i);
+        float4 s = zero4();
+#pragma unroll
+        for (int cb = 0; cb < BM_MAX; cb += UCH) {
+            if (cb < k) {
+                float4 v[UCH];
+#pragma unroll
+                for (int c = 0; c < UCH; ++c) v[c] = (cb + c < k) ? __ldcs(col4(L, cb + c) + i) : zero4();
+#pragma unroll
+                for (int c = 0; c < UCH; ++c) fma4(s, v[c], sco[cb + c][q]);
+            }
+        }
+        float4 o;
+        o.x = fmaf(x.x, wsc.x, -s.x) * psc.x;
+        o.y = fmaf(x.y, wsc.y, -s.y) * psc.y;
+        o.z = fmaf(x.z, wsc.z, -s.z) * psc.z;
+        o.w = fmaf(x.w, wsc.w, -s.w) * psc.w;
+        Out[i] = o;
     }
 }
 
@@ -630,7 +637,8 @@ int launch_dot(const Layout& L, int j, int reortho, int gg, int tune, cudaStream
 
 int launch_update(const Layout& L, int j, cudaStream_t s) {
     if (j < 0 || j >= BM_MAX || L.T <= 0) return L.T <= 0 ? MEXK_OK : MEXK_ERR_INVALID;
-    const int grid = L.N < sm_blocks(4) ? L.N : sm_blocks(4);
+    const int chunks = L.C1 - L.C0;
+    const int grid = chunks < sm_blocks(4) ? chunks : sm_blocks(4);
     update_kernel<<<grid, BT, 0, s>>>(L, j);
     MEXK_CK_LAUNCH("batch update_kernel");
     return MEXK_OK;
