@@ -366,6 +366,76 @@ __device__ __forceinline__ void ac_update(const CycleArgs& g, const double* V, i
     else ac_update_rows<1, 8>(V, ldv, k, r0, rows, h, w);
 }
 
+// ---- one or two columns --------------------------------------------------------
+// A short window's step in three passes instead of five, each reading the
+// columns once: the dots; the first update with the second dots; the second
+// update with the norm (a sweep of its own for each took 38 of a step's 85
+// thousand cycles at 777^2 rows, window 2). UPDATE: w -= h0 v0 + h1 v1.
+// The thread's sums of v0.w, v1.w (or |w|^2 in sum[0]) over its rows.
+enum AcPass { AC_PASS_DOTS, AC_PASS_NORM };
+template <bool UPDATE, AcPass PASS>
+__device__ __forceinline__ void ac_narrow_pass(const double* V, size_t ldv, int k, int r0, int rows, const double* h,
+                                               double* w, double (&sum)[2]) {
+    constexpr int UN = 4;
+    const bool two = k == 2;
+    const double* const p0 = V + r0;
+    const double* const p1 = p0 + ldv;
+    const double h0 = UPDATE ? -h[0] : 0.0, h1 = UPDATE && two ? -h[1] : 0.0;
+    sum[0] = sum[1] = 0.0;
+    for (int r = 2 * static_cast<int>(threadIdx.x); r < rows; r += 2 * UN * AC_THREADS) {
+        double2 x[UN], a[UN], b[UN];
+#pragma unroll
+        for (int u = 0; u < UN; ++u) {
+            const int q = r + 2 * u * AC_THREADS;
+            a[u] = b[u] = x[u] = make_double2(0.0, 0.0);
+            if (q < rows) {
+                a[u] = __ldcg(reinterpret_cast<const double2*>(p0 + q));
+                if (two) b[u] = __ldcg(reinterpret_cast<const double2*>(p1 + q));
+                x[u] = *reinterpret_cast<const double2*>(w + q);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < UN; ++u) {
+            const int q = r + 2 * u * AC_THREADS;
+            if (q >= rows) break;
+            if (UPDATE) {
+                x[u].x = fma(h0, a[u].x, x[u].x);
+                x[u].y = fma(h0, a[u].y, x[u].y);
+                if (two) {
+                    x[u].x = fma(h1, b[u].x, x[u].x);
+                    x[u].y = fma(h1, b[u].y, x[u].y);
+                }
+                *reinterpret_cast<double2*>(w + q) = x[u];
+            }
+            if (PASS == AC_PASS_DOTS) {
+                sum[0] = fma(a[u].x, x[u].x, sum[0]);
+                sum[0] = fma(a[u].y, x[u].y, sum[0]);
+                if (two) {
+                    sum[1] = fma(b[u].x, x[u].x, sum[1]);
+                    sum[1] = fma(b[u].y, x[u].y, sum[1]);
+                }
+            } else {
+                sum[0] = fma(x[u].x, x[u].x, sum[0]);
+                sum[0] = fma(x[u].y, x[u].y, sum[0]);
+            }
+        }
+    }
+}
+
+// The block's sums of two columns into the exchange.
+__device__ __forceinline__ void ac_narrow_publish(const CycleArgs& g, int k, double (&sum)[2], const AcExchange& ex,
+                                                  AcShared& sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // lanes 0..15 go on with column 0, the others with column 1
+    double t = (lane & 16) ? sum[1] : sum[0];
+    t += __shfl_xor_sync(AC_FULL, (lane & 16) ? sum[0] : sum[1], 16);
+#pragma unroll
+    for (int o = 8; o >= 1; o >>= 1) t += __shfl_xor_sync(AC_FULL, t, o);
+    if ((lane & 15) == 0) sh.red[warp][lane >> 4] = t;
+    __syncthreads();
+    ac_publish<AC_THREADS>(ex.words, &sh.red[0][0], MEXK_M_MAX + 1, k, AC_NW, g.scale);
+}
+
 // ---- the sweeps over the digit columns ---------------------------------------
 // Largest high word over the block of m (every thread calls it); the three
 // slots are used by turns.
@@ -743,6 +813,21 @@ __device__ __forceinline__ void ac_product(const CycleArgs& g, const double* gx,
     else ac_product_pattern<PAT_LEN>(g, gx, inv, scaled, r0, rows, n_rows, w);
 }
 
+// The block's |w|^2 from the first nw warps' sums into the exchange.
+__device__ __forceinline__ void ac_norm_publish(double acc, int nw, const AcExchange& ex, AcShared& sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < nw) {
+        const double t = warp_sum(acc);
+        if (lane == 0) sh.red[warp][0] = t;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double t = lane < nw ? sh.red[lane][0] : 0.0;
+        for (int o = 1; o < nw; o <<= 1) t += __shfl_xor_sync(AC_FULL, t, o);
+        if (lane == 0) __stcg(ex.part + blockIdx.x, t);
+    }
+}
+
 // |w|^2 over the block's rows into the exchange. EXACT per sub-block (pairs,
 // then the plain butterfly).
 template <bool EXACT>
@@ -760,19 +845,7 @@ __device__ __forceinline__ void ac_norm(int r0, int nsub, const double* wv, cons
             if (lane < AC_CLUSTER) *cl.map_shared_rank(ex.part + r0 / AC_SUB + s, lane) = t;
         }
     }
-    if (!EXACT) {
-        const int nw = min(AC_NW, nsub);
-        if (warp < nw) {
-            const double t = warp_sum(acc);
-            if (lane == 0) sh.red[warp][0] = t;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            double t = lane < nw ? sh.red[lane][0] : 0.0;
-            for (int o = 1; o < nw; o <<= 1) t += __shfl_xor_sync(AC_FULL, t, o);
-            if (lane == 0) __stcg(ex.part + blockIdx.x, t);
-        }
-    }
+    if (!EXACT) ac_norm_publish(acc, min(AC_NW, nsub), ex, sh);
 }
 
 // |w|^2 over all blocks, after the meeting, in thread 0. The dynamic range of
@@ -811,8 +884,8 @@ __device__ __forceinline__ double ac_norm_sum(const AcExchange& ex, int np) {
 
 // CLUSTER: one cluster, the separate kernels' sums. DIGITS: the sweeps over
 // the digit columns. WSMEM: the block's rows of w fit in shared memory (else
-// they stay in x).
-template <bool CLUSTER, bool DIGITS, bool WSMEM>
+// they stay in x). NARROW: a window of at most two columns.
+template <bool CLUSTER, bool DIGITS, bool WSMEM, bool NARROW = false>
 __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs g) {
     constexpr bool EXACT = CLUSTER;
     __shared__ AcShared sh;
@@ -868,8 +941,13 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
             else if (k <= 16) ac_dots<1, EXACT>(g, V, k, r0, nsub, w, e, sh);
             else ac_dots<2, EXACT>(g, V, k, r0, nsub, w, e, sh);
         };
+        constexpr bool narrow = NARROW;
+        double sum[2];
         unsigned mag = 0u;
-        if (DIGITS) {
+        if (narrow) {
+            ac_narrow_pass<false, AC_PASS_DOTS>(V, ldv, k, r0, rows, nullptr, w, sum);
+            ac_narrow_publish(g, k, sum, ex[0], sh);
+        } else if (DIGITS) {
             for (int r = 2 * static_cast<int>(threadIdx.x); r < rows; r += 2 * AC_THREADS) {
                 const double2 x = *reinterpret_cast<const double2*>(w + r);
                 mag = max(mag, max(ac_mag(x.x), ac_mag(x.y)));
@@ -886,7 +964,10 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
             for (int i = threadIdx.x; i < 2 * CYCLE_EXCHANGE; i += AC_THREADS) __stcg(w + i, 0ull);
         }
         ac_sums<EXACT>(ex[0], k, np, g.scale, sh.h1, sh);
-        if (DIGITS) {
+        if (narrow) {
+            if (g.reortho) ac_narrow_pass<true, AC_PASS_DOTS>(V, ldv, k, r0, rows, sh.h1, w, sum);
+            else ac_narrow_pass<true, AC_PASS_NORM>(V, ldv, k, r0, rows, sh.h1, w, sum);
+        } else if (DIGITS) {
             ac_coefficients(lo, k, sh.h1, sh);
             mag = ac_block_mag(ac_update_digits(g, lo, k, r0, rows, w, sh.h1, sh), turn, sh);
         } else {
@@ -894,11 +975,14 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
             __syncthreads();
         }
         if (g.reortho) {
-            if (DIGITS) ac_dots_digits(g, lo, k, r0, nsub, w, mag, wq, ex[1], sh);
+            if (narrow) ac_narrow_publish(g, k, sum, ex[1], sh);
+            else if (DIGITS) ac_dots_digits(g, lo, k, r0, nsub, w, mag, wq, ex[1], sh);
             else dots(ex[1]);
             if (!ac_meet<CLUSTER>(g.bar, target, &st->status, &sh.ok)) return;
             ac_sums<EXACT>(ex[1], k, np, g.scale, sh.h, sh);
-            if (DIGITS) {
+            if (narrow) {
+                ac_narrow_pass<true, AC_PASS_NORM>(V, ldv, k, r0, rows, sh.h, w, sum);
+            } else if (DIGITS) {
                 ac_coefficients(lo, k, sh.h, sh);
                 mag = ac_block_mag(ac_update_digits(g, lo, k, r0, rows, w, sh.h, sh), turn, sh);
             } else {
@@ -909,7 +993,8 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
             for (int c = threadIdx.x; c < k; c += AC_THREADS)
                 g.H[(lo + c) + j * ldh] = g.reortho ? sh.h1[c] + sh.h[c] : sh.h1[c];
         __syncthreads();
-        ac_norm<EXACT>(r0, nsub, w, ex[2], sh);
+        if (narrow) ac_norm_publish(sum[0], AC_NW, ex[2], sh);
+        else ac_norm<EXACT>(r0, nsub, w, ex[2], sh);
         if (WSMEM && g.scale_gather)
             for (int r = threadIdx.x; r < n_rows; r += AC_THREADS) __stcg(g.x + r0 + r, w[r]);
         if (!ac_meet<CLUSTER>(g.bar, target, &st->status, &sh.ok)) return;
@@ -1007,6 +1092,8 @@ int arnoldi_cycle_prepare() {
                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
     MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, false, true, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
     return MEXK_OK;
 }
 
@@ -1036,6 +1123,10 @@ int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s) {
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(AC_THREADS);
     const bool digits = !cluster && a.vq != nullptr;
+    // Three passes against five sweeps, heat grids, window 2, one solve: 200^2 (320 rows a block) 2911 / 2890 us,
+    // 300^2 3804 / 3302, 777^2 7271 / 6787, 1500^2 18442 / 16838; below 256 rows a block the sweeps share a column's
+    // few rows out better (131^2 2695 / 2763).
+    const bool narrow = !cluster && !digits && a.window > 0 && a.window <= 2 && a.rows >= 256;
     const bool wsmem = a.rows * (digits ? 2 : 1) <= AC_SMEM_DOUBLES;
     if (!wsmem) a.scale_gather = 0;  // x holds w
     cfg.dynamicSmemBytes = sizeof(double) * ((wsmem ? static_cast<size_t>(a.rows) * (digits ? 2 : 1) : 0) +
@@ -1057,6 +1148,8 @@ int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s) {
     }
     cfg.attrs = attr;
     const cudaError_t e = cluster           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true, false, true>, a)
+                          : narrow && wsmem ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, true, true>, a)
+                          : narrow          ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, false, true>, a)
                           : digits && wsmem ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true, true>, a)
                           : digits          ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true, false>, a)
                           : wsmem           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, true>, a)

@@ -40,6 +40,8 @@ CASES += [("random", 2000, 32, 1, 0), ("random", 2000, 64, 1, 0), ("random", 600
 CASES += [("random", 300011, 10, 1, 0), ("random", 150003, 23, 1, 0), ("random", 40007, 75, 1, 0),
           ("random", 150003, 20, 0, 0), ("powerlaw", 160001, 19, 1, 0), ("heat", 601, 17, 1, 0),
           ("heat", 601, 30, 1, 6)]
+# a window of 2 in three passes (256 rows a block or more), w on chip and not
+CASES += [("heat", 198, 30, 1, 2), ("heat", 301, 30, 1, 2), ("heat", 777, 20, 0, 2), ("heat", 1851, 6, 1, 2)]
 
 
 @pytest.mark.parametrize("kind,n,m,reortho,window", CASES)
