@@ -249,7 +249,9 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) stencil_cycle_kernel(StencilArgs 
             }
         };
         if (!scalar) halo_load(0);
-        // w = A u_j (added in entry order), u_j.w and |w|^2
+        // w = A u_j, rounded products added in entry order (the SpMV kernels' sums bit for bit:
+        // what a smooth vector's rounding leaves in w is part of what the learned controller was
+        // trained on; fused ones cost heat 2048^2 a fifth cycle), u_j.w and |w|^2
         float d0[2] = {0.f, 0.f}, d1[2] = {0.f, 0.f};
         auto product = [&](int c) {
             const int b = c * SC_CHUNK_ROWS + tid;
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) stencil_cycle_kernel(StencilArgs 
                     for (int e = 0; e < SC_CHUNK; ++e)
 #pragma unroll
                         for (int q = 0; q < L; ++q)
-                            w[e] = fmaf(g.val[q], xv[e][q], w[e]);
+                            w[e] = __fadd_rn(w[e], __fmul_rn(g.val[q], xv[e][q]));
                 } else {
                     int mk[SC_CHUNK];
 #pragma unroll
@@ -276,7 +278,7 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) stencil_cycle_kernel(StencilArgs 
                     for (int e = 0; e < SC_CHUNK; ++e)
 #pragma unroll
                         for (int q = 0; q < L; ++q)
-                            if ((mk[e] >> q) & 1) w[e] = fmaf(g.val[q], xv[e][q], w[e]);
+                            if ((mk[e] >> q) & 1) w[e] = __fadd_rn(w[e], __fmul_rn(g.val[q], xv[e][q]));
                 }
             } else {
                 // rows of patterns that are no part of the major one among them: from the table
@@ -287,7 +289,8 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) stencil_cycle_kernel(StencilArgs 
                     if (r >= nr) continue;
                     const int id = __ldg(g.pid + r0 + r), pl = __ldg(T->len + id);
                     for (int q = 0; q < pl; ++q)
-                        w[e] = fmaf(__ldg(T->v32 + id * PAT_LEN + q), u[r + __ldg(T->off + id * PAT_LEN + q)], w[e]);
+                        w[e] = __fadd_rn(w[e], __fmul_rn(__ldg(T->v32 + id * PAT_LEN + q),
+                                                         u[r + __ldg(T->off + id * PAT_LEN + q)]));
                 }
             }
             __syncwarp();
