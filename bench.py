@@ -164,6 +164,14 @@ def kernel_bytes(kind, n, nnz, k, fp32, window=0, form="staged"):
         # per step u_j (gathered once), u_{j-1} read and u_{j+1} written; w stays
         # on chip
         return n + (k - 1) * 3 * n * s
+    if kind == "basis":
+        # k steps in one launch. A window of 2 in mixed precision keeps the recurrence
+        # on chip: row ids, the first column and every column written once; else what
+        # the separate kernels of its steps would move
+        if fp32 and window == 2 and form == "pattern":
+            return n + (k + 1) * n * s
+        return sum(kernel_bytes(q, n, nnz, j + 1, fp32, window, form)
+                   for j in range(k) for q in STEP_KINDS["mixed" if fp32 else "fp64"])
     if kind == "spmv":
         return nnz * (s + 4) + 4 * (n + 1) + 2 * n * s  # values+cols, row_ptr, x once, y
     if kind == "spmv_dots":  # the SpMV, then u_{j-1} read for the dots (u_j is x)
@@ -251,6 +259,7 @@ def profile_cycle(ctx, m, n, nnz, precision, iters=8, window=0):
     form = ctx.spmv_form(precision)
     dots_in_spmv = form != "direct"
     fused = lanczos_fused(ctx, precision, window)
+    one_launch = ctx.basis_launches(m, precision, window) == 1
     per = {}
 
     def add(kind, j, k):
@@ -264,33 +273,44 @@ def profile_cycle(ctx, m, n, nnz, precision, iters=8, window=0):
 
     # The controller first: it runs on the Hessenberg matrix the last solve left.
     for kind in once:
-        add(kind, m - 1, m)
+        if not (one_launch and kind == "gram_norm"):  # part of the basis
+            add(kind, m - 1, m)
+    if one_launch:
+        add("basis", m - 1, m)
+        return per
     for j in range(m):
         for kind in step_kinds(precision, j, window, dots_in_spmv, fused):
             add(kind, j, j + 1)
     return per
 
 
+def spmv_profile(ctx, per, m, n, nnz, precision, iters=8):
+    """The SpMV kernel's time, bytes and launches over a cycle, whether or not
+    a solve's basis launches it."""
+    if "spmv" in per:
+        return per["spmv"]
+    steps = (0, m // 2, m - 1)
+    return {"ms": sum(ctx.profile_kernel("spmv", j, iters, precision) for j in steps),
+            "bytes": len(steps) * kernel_bytes("spmv", n, nnz, 1, precision == "mixed", 0, ctx.spmv_form(precision)),
+            "launches": len(steps)}
+
+
 def launches_per_solve(ctx, precision, res, m, window=0):
     """Kernels one solve launches: the start vector (2), then per cycle its
-    steps (SpMV + sweeps, step_kinds) and the cycle's controller, lift and
-    restart (+ the mixed form's last-column norm). Cycle sizes come from the
-    attempt log."""
+    basis, controller, lift and restart. Cycle sizes come from the attempt
+    log."""
     sizes = [int(s[3]) for s in ctx.steps()]
     if len(sizes) != res["cycles"]:  # rejects reuse their cycle's basis
         sizes = [m] * res["cycles"]
-    per_cycle = 4 if precision == "mixed" else 3
-    dots_in_spmv = ctx.spmv_form(precision) != "direct"
-    fused = lanczos_fused(ctx, precision, window)
-    return 2 + sum(sum(len(step_kinds(precision, j, window, dots_in_spmv, fused)) for j in range(k)) + per_cycle
-                   for k in sizes)
+    return 2 + sum(ctx.basis_launches(k, precision, window) + 3 for k in sizes)
 
 
 def gs_cgs2_equivalent(per, n, m, precision):
     """Gram-Schmidt of one cycle against the CGS2 byte count: all GS kernel
-    time of the cycle over sum_j cgs2_step_bytes."""
+    time of the cycle (a basis in one launch: with its products) over sum_j
+    cgs2_step_bytes."""
     fp32 = precision == "mixed"
-    gs = [k for k in per if k.startswith("gs_") or k.startswith("gram_") or k == "normalize"]
+    gs = [k for k in per if k.startswith("gs_") or k.startswith("gram_") or k in ("normalize", "basis")]
     ms = sum(per[k]["ms"] for k in gs)
     b = sum(cgs2_step_bytes(n, j + 1, fp32) for j in range(m))
     return {"ms_per_cycle": round(ms, 4), "cgs2_bytes": b, "gbs": round(b / (ms / 1e3) / 1e9, 1),
@@ -545,14 +565,14 @@ def run_ours(args, rank, world, local_rank):
             "traffic": traffic, "traffic_source": tsrc,
             "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
             "size_matched_copy": size_matched_copy(per[dom]["bytes"] / per[dom]["launches"], stream)}
-    sp = per["spmv"]
+    sp = spmv_profile(ctx, per, m, n, nnz, form)
     spmv_gbs = sp["bytes"] / (sp["ms"] / 1e3) / 1e9
     if form != "fp64":
         ctx.expmv_device(v_d.data_ptr(), y64.data_ptr(), P.t, m, precision="fp64")
         per64 = profile_cycle(ctx, m, n, nnz, "fp64")
     else:
         per64 = per
-    sp64 = per64["spmv"]
+    sp64 = spmv_profile(ctx, per64, m, n, nnz, "fp64")
 
     cpu = None
     if rank == 0 and not args.no_cpu:

@@ -382,7 +382,8 @@ int mexk_batch_destroy(mexk_batch_t b);
 #define MEXK_KERNEL_GRAM_NORM 9   /* mixed: norm of the last column (once per basis) */
 #define MEXK_KERNEL_SPMV_DOTS 10  /* mixed, steps j >= 1 over two columns: SpMV + the step's dots and finish */
 #define MEXK_KERNEL_LANCZOS_CYCLE 11 /* mixed, window 2, fused form: steps 1..j of a basis in one launch */
-#define MEXK_KERNEL_KINDS 12
+#define MEXK_KERNEL_BASIS 12 /* a basis of j + 1 columns from the first one, as a solve builds it */
+#define MEXK_KERNEL_KINDS 13
 
 /* Times `iters` launches of one solver kernel for Arnoldi step j (k = j+1
  * basis columns) on the context stream with CUDA events, on the context's
@@ -414,7 +415,9 @@ int mexk_profile_kernel(mexk_context_t ctx, int kind, int precision, int j, int 
  * for a matrix without one). All forms compute the same products and add
  * each row's in column order, so FP64 solves are bitwise equal under any;
  * mixed solves take the two-column steps' dots in a form-dependent order and
- * agree to rounding. No reference counterpart: the reference's SpMV is one
+ * agree to rounding. A basis built in one launch (mexk_context_basis_launches)
+ * takes its products itself: from the row patterns under the pattern form, else
+ * from the CSR arrays. No reference counterpart: the reference's SpMV is one
  * cuSPARSE call (main.cu:1743). */
 #define MEXK_SPMV_STAGED 0
 #define MEXK_SPMV_DIRECT 1
@@ -427,7 +430,9 @@ int mexk_context_set_spmv_form(mexk_context_t ctx, int precision, int form);
  * MEXK_LANCZOS_FUSED as one cooperative launch in which one thread block
  * per SM keeps its rows' ids and A u_j on chip and the blocks meet at two
  * bounded grid barriers per step; MEXK_LANCZOS_STEPWISE (the default) as two
- * launches per step (the SpMV with the step's dot products, the update).
+ * the library does by default: in one launch with the recurrence on chip
+ * where it fits (about 5 million rows), else as two launches per step (the
+ * SpMV with the step's dot products, the update).
  * The fused form applies when every block's rows fit its shared memory
  * (about 7 million rows on a 152-SM GB300); get reports the form a solve
  * would run. Both compute the same row sums and updates and sum the dot
@@ -437,6 +442,12 @@ int mexk_context_set_spmv_form(mexk_context_t ctx, int precision, int form);
 #define MEXK_LANCZOS_FUSED 1
 int mexk_context_get_lanczos_form(mexk_context_t ctx, int* form);
 int mexk_context_set_lanczos_form(mexk_context_t ctx, int form);
+
+/* Kernels a solve with this precision and ortho_window launches for a basis of
+ * m columns: 1 where one launch runs all its steps (and, but for FP64 matrices
+ * of long or very many rows, their products), else per step the SpMV and its
+ * sweeps. */
+int mexk_context_basis_launches(mexk_context_t ctx, int precision, int m, int ortho_window, int* launches);
 
 /* ---- testing hooks ------------------------------------------------------ */
 /* enable != 0: from now on, thread block 0 of the staged CSR SpMV also waits

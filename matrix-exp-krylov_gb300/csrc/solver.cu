@@ -4,13 +4,16 @@
 // ArnoldiRunner::compute_expmv (main.cu:1411-1571) for one device. The
 // reference drives every Arnoldi step from the host (about 10(j+1)+12
 // launches and 3 blocking syncs per step, H held on the host). Here a whole
-// Krylov cycle -- m x (SpMV, three Gram-Schmidt sweeps, normalise), the
-// exponential + controller, the lift and the restart -- is one CUDA graph
+// Krylov cycle -- the basis, the exponential + controller, the lift and the
+// restart -- is one CUDA graph
 // whose kernels read and write a device-resident state block, so the host
 // launches one graph per accepted step and syncs once to read `done`.
-// The FP64 form runs three CGS2 sweeps and a normalisation per step
-// (gram_schmidt.cu); the mixed form one reducing and one streaming sweep
-// over an FP32 basis with a device-resident Gram matrix (gram_mixed.cu).
+// A basis is one launch where it fits (arnoldi_cycle.cu in FP64, gram_cycle.cu
+// and, for a window of 2 on stencils, stencil_cycle.cu in mixed precision);
+// otherwise a step is the SpMV and, in FP64, three CGS2 sweeps and a
+// normalisation (gram_schmidt.cu), in mixed precision one reducing and one
+// streaming sweep over an FP32 basis with a device-resident Gram matrix
+// (gram_mixed.cu).
 //
 // HBM layout per context (n rows, m_alloc maximum Krylov dimension):
 //   CSR        row_ptr int32[n+1], col_idx int32[nnz], values f64[nnz]
@@ -20,9 +23,11 @@
 //   basis V    column-major, leading dimension ldv = n rounded up to 64,
 //              m_alloc+1 columns, f64 (+ f32 basis for the mixed form, whose
 //              columns carry f64 scales, with the Gram matrix, in GramState)
+//              wide FP64 bases also in 61-bit digits (d_vq) with their exponents
 //   w, y       work vector (basis precision) and result (f64)
 //   H          f64 (m_alloc+1) x m_alloc column-major; h1, h2, coef f64
 //   partials   f64[4096 x RED_STRIDE] grid-reduction scratch + counter
+//   bar        the one-launch bases' meeting words and exact sums
 //   state      DevState (device) mirrored into pinned host memory
 #include "mexk_internal.cuh"
 
@@ -602,24 +607,18 @@ int enqueue_stencil_cycle(mexk_context_t ctx, int m, int reortho, cudaStream_t s
     return launch_stencil_cycle(a, s);
 }
 
-// One Krylov cycle: the unit that is captured into a graph.
-template <typename TV>
-int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, cudaStream_t s) {
-    const bool fp32 = sizeof(TV) == 4;
-    TV* V = fp32 ? reinterpret_cast<TV*>(ctx->d_V32) : reinterpret_cast<TV*>(ctx->d_V);
+// A basis of m columns from V[:,0], H(m, m-1) included.
+int enqueue_basis(mexk_context_t ctx, int m, int reortho, int window, bool fp32, cudaStream_t s) {
     int rc;
     // a window's FP64 steps leave H(0:lo-1, j) alone: the cycle starts from zero
     if (!fp32 && window > 0)
         MEXK_CK(cudaMemsetAsync(ctx->d_H, 0, sizeof(double) * static_cast<size_t>(ctx->ldh) * m, s));
+    if (!fp32 && use_arnoldi_cycle(ctx)) return enqueue_arnoldi_cycle(ctx, m, reortho, window, s);
+    if (fp32 && use_gram_cycle(ctx, m, window))
+        return use_stencil_cycle(ctx, m, window) ? enqueue_stencil_cycle(ctx, m, reortho, s)
+                                                 : enqueue_gram_cycle(ctx, m, reortho, window, s);
     const bool fused = use_lanczos_cycle(ctx, m, fp32, window);
-    const bool onchip = fp32 && use_gram_cycle(ctx, m, window);
-    if (!fp32 && use_arnoldi_cycle(ctx)) {
-        if ((rc = enqueue_arnoldi_cycle(ctx, m, reortho, window, s))) return rc;
-    } else if (onchip) {
-        rc = use_stencil_cycle(ctx, m, window) ? enqueue_stencil_cycle(ctx, m, reortho, s)
-                                               : enqueue_gram_cycle(ctx, m, reortho, window, s);
-        if (rc) return rc;
-    } else if (fused) {
+    if (fused) {
         // step 0 as two kernels (its update writes step 1's b and a_0 partials), then the rest in one launch
         if ((rc = enqueue_step(ctx, 0, reortho, fp32, s, window, m))) return rc;
         if ((rc = enqueue_lanczos_cycle(ctx, m, reortho, s))) return rc;
@@ -628,7 +627,16 @@ int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, 
             if ((rc = enqueue_step(ctx, j, reortho, fp32, s, window, m))) return rc;
     }
     // the stepwise basis's last update left |u_m|^2 as partials where it could
-    if (!onchip && (rc = finish_basis(ctx, m - 1, fp32, s, !fused && fp32 && norm_from_update(m, window)))) return rc;
+    return finish_basis(ctx, m - 1, fp32, s, !fused && fp32 && norm_from_update(m, window));
+}
+
+// One Krylov cycle: the unit that is captured into a graph.
+template <typename TV>
+int enqueue_cycle(mexk_context_t ctx, int m, int reortho, int ctrl, int window, cudaStream_t s) {
+    const bool fp32 = sizeof(TV) == 4;
+    TV* V = fp32 ? reinterpret_cast<TV*>(ctx->d_V32) : reinterpret_cast<TV*>(ctx->d_V);
+    int rc;
+    if ((rc = enqueue_basis(ctx, m, reortho, window, fp32, s))) return rc;
     if ((rc = enqueue_controller(ctx, m, ctrl, ctx->d_log, s, window))) return rc;
     const LiftArgs l = lift_args(ctx, fp32);
     if ((rc = launch_lift<TV>(l, gs_grid_size(ctx->n, 1), s))) return rc;
@@ -1315,6 +1323,33 @@ int mexk_context_set_window_controller(mexk_context_t ctx, const float* weights,
     return MEXK_OK;
 }
 
+int mexk_context_basis_launches(mexk_context_t ctx, int precision, int m, int ortho_window, int* launches) {
+    if (!ctx || !ctx->uploaded || !launches || m < 1 || m > ctx->m_alloc || ortho_window < 0) return MEXK_ERR_INVALID;
+    if (precision != MEXK_PREC_FP64 && precision != MEXK_PREC_MIXED) return MEXK_ERR_INVALID;
+    MEXK_CK(cudaSetDevice(ctx->device));
+    int rc;
+    if (precision == MEXK_PREC_FP64) {
+        const bool product = arnoldi_cycle_product(ctx->n, ctx->nnz, ctx->max_row, ctx->spmv_form64 == MEXK_SPMV_PATTERN);
+        const int chunks = (m + GS_DOT_COLS - 1) / GS_DOT_COLS;  // of the separate sweeps' dots
+        *launches = use_arnoldi_cycle(ctx) ? (product ? 1 : 2 * m) : (chunks > 1 ? 7 : 5) * m;
+        return MEXK_OK;
+    }
+    if ((rc = ensure_mixed(ctx))) return rc;
+    if (use_gram_cycle(ctx, m, ortho_window)) {
+        *launches = 1;
+        return MEXK_OK;
+    }
+    if (use_lanczos_cycle(ctx, m, true, ortho_window)) {
+        *launches = 5;  // step 0's SpMV, dots and update, the rest, the last norm
+        return MEXK_OK;
+    }
+    int k = 1;  // the last column's norm
+    for (int j = 0; j < m; ++j)
+        k += ctx->spmv_form32 != MEXK_SPMV_DIRECT && fused_step(j, ortho_window) ? 2 : 3;
+    *launches = k;
+    return MEXK_OK;
+}
+
 int mexk_context_get_spmv_form(mexk_context_t ctx, int precision, int* form) {
     if (!ctx || !ctx->uploaded || !form) return MEXK_ERR_INVALID;
     if (precision != MEXK_PREC_FP64 && precision != MEXK_PREC_MIXED) return MEXK_ERR_INVALID;
@@ -1462,6 +1497,10 @@ int mexk_profile_kernel(mexk_context_t ctx, int kind, int precision, int j, int 
                         ? enqueue_lanczos_cycle(ctx, j + 1, 1, s)
                         : MEXK_ERR_UNSUPPORTED;
                 break;
+            case MEXK_KERNEL_BASIS:
+                // from column 0, which stays as it is: launches repeat the same work
+                r = enqueue_basis(ctx, j + 1, 1, ctx->last_window, fp32, s);
+                break;
             case MEXK_KERNEL_LIFT: {
                 const LiftArgs l = lift_args(ctx, fp32);
                 r = fp32 ? launch_lift<float>(l, gs_grid_size(ctx->n, 1), s)
@@ -1499,7 +1538,7 @@ int mexk_profile_kernel(mexk_context_t ctx, int kind, int precision, int j, int 
     const bool reset_each = !(kind == MEXK_KERNEL_SPMV || kind == MEXK_KERNEL_SPMV_DOTS ||
                               kind == MEXK_KERNEL_GRAM_DOT || kind == MEXK_KERNEL_GRAM_UPDATE ||
                               kind == MEXK_KERNEL_GRAM_NORM || kind == MEXK_KERNEL_GS_DOT ||
-                              kind == MEXK_KERNEL_LANCZOS_CYCLE);
+                              kind == MEXK_KERNEL_LANCZOS_CYCLE || kind == MEXK_KERNEL_BASIS);
     if (reset_each) {
         for (int it = 0; it < iters && rc == MEXK_OK; ++it) {
             cudaError_t ce = cudaMemcpyAsync(ctx->d_state, h_run, sizeof(DevState), cudaMemcpyHostToDevice, s);

@@ -208,8 +208,9 @@ class Context:
     LANCZOS_FORMS = ("stepwise", "fused")
 
     def lanczos_form(self) -> str:
-        """How window-2 bases run their steps: "stepwise" (two launches per
-        step, the default) or "fused" (one cooperative launch per basis, when
+        """How window-2 bases run their steps: "stepwise" (the default: in one
+        launch with the recurrence on chip where it fits, else two launches per
+        step) or "fused" (the cooperative launch that gathers from memory, when
         selected and the basis's rows fit)."""
         f = C.c_int(0)
         check(lib().mexk_context_get_lanczos_form(self._h, C.byref(f)), "mexk_context_get_lanczos_form")
@@ -218,6 +219,13 @@ class Context:
     def set_lanczos_form(self, form: str) -> None:
         check(lib().mexk_context_set_lanczos_form(self._h, self.LANCZOS_FORMS.index(form)),
               "mexk_context_set_lanczos_form")
+
+    def basis_launches(self, m: int, precision="fp64", window: int = 0) -> int:
+        """Kernels a solve launches for a basis of m columns (1: all steps in one launch)."""
+        k = C.c_int(0)
+        check(lib().mexk_context_basis_launches(self._h, PRECISIONS[precision], m, window, C.byref(k)),
+              "mexk_context_basis_launches")
+        return k.value
 
     def arnoldi_step(self, j: int, reorthogonalize=True, precision="fp64"):
         h = np.zeros(j + 1)

@@ -157,3 +157,20 @@ def test_wait_that_runs_out_reports_and_the_context_survives(kind, window):
             check(lib().mexk_test_force_wait_timeout(0, 0))
         again, _ = ctx.expmv(v, t, 20, precision="mixed", controller="search", window=window)
     assert np.array_equal(good, again)
+
+
+@pytest.mark.parametrize("kind,n,precision,window,one", [("random", 2000, "fp64", 0, True), ("random", 2000, "mixed", 0, True),
+                                                         ("heat", 300, "mixed", 2, True), ("random", 300007, "mixed", 0, False),
+                                                         ("random", 300007, "fp64", 0, False)])
+def test_basis_launches_and_profile(kind, n, precision, window, one):
+    from mexk.api import Context
+
+    A = make(kind, n)
+    v = np.random.default_rng(2).standard_normal(A.n)
+    ctrl = "reference" if precision == "fp64" else "search"
+    with Context(A, m_alloc=20) as ctx:
+        ctx.expmv(v, 1e-3 / A.max_abs(), 20, precision=precision, controller=ctrl, window=window)
+        assert (ctx.basis_launches(20, precision, window) == 1) == one
+        assert ctx.basis_launches(5, precision, window) <= ctx.basis_launches(20, precision, window)
+        t5, t20 = (ctx.profile_kernel("basis", j, 3, precision) for j in (4, 19))
+        assert 0.0 < t5 < t20 < 50.0
