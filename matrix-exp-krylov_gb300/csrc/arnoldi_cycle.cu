@@ -6,10 +6,11 @@
 // serial tails are what a step costs (about 40 us at 2,000 rows, 50 us at
 // 9,216, 100 us at 600,000 with a window of 2) while its FP64 arithmetic,
 // 8 n k flops at about two FMAs per clock per SM, would take 1 to 10 us.
-// Measured per step now: 15, 17 and 41 us; whole solves 1.2 to 2.7 times
-// faster from 2,000 to 2,000,000 rows. Here every thread block owns a contiguous range of rows for the whole basis,
-// keeps its part of w in shared memory, and the blocks meet three times a
-// step, each time to exchange k (or one) partial sums:
+// Measured per step now: 14, 16 and 38 us; whole solves 1.2 to 2.8 times
+// faster from 2,000 to 4,000,000 rows. Here every thread block owns a
+// contiguous range of rows for the whole basis, keeps its part of w in shared
+// memory, and the blocks meet three times a step, each time to exchange k (or
+// one) partial sums:
 //   w = A v_j; partial V^T w                                | meet
 //   h1 = sums; w -= V h1; partial V^T w                     | meet
 //   h2 = sums; H(:,j) = h1 + h2; w -= V h2; partial |w|^2   | meet

@@ -1,5 +1,6 @@
 // K2, mixed precision: Gram-Schmidt over an FP32 basis with one reducing
-// sweep and one streaming sweep per Arnoldi step.
+// sweep and one streaming sweep per Arnoldi step (bases that gram_cycle.cu and
+// stencil_cycle.cu do not take, and single steps).
 //
 // The reference orthogonalises with two MGS passes and normalises with a
 // separate norm (main.cu:1769-1942): on one GPU that is five passes over the
