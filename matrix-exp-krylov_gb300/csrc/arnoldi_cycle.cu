@@ -6,7 +6,7 @@
 // serial tails are what a step costs (about 40 us at 2,000 rows, 50 us at
 // 9,216, 100 us at 600,000 with a window of 2) while its FP64 arithmetic,
 // 8 n k flops at about two FMAs per clock per SM, would take 1 to 10 us.
-// Measured per step now: 14, 16 and 38 us; whole solves 1.2 to 2.8 times
+// Measured per step now: 13, 15 and 38 us; whole solves 1.2 to 2.8 times
 // faster from 2,000 to 4,000,000 rows. Here every thread block owns a
 // contiguous range of rows for the whole basis, keeps its part of w in shared
 // memory, and the blocks meet three times a step, each time to exchange k (or
@@ -232,7 +232,8 @@ struct AcExchange {
     unsigned long long* words;
 };
 
-// The dots of CN columns (kc of them real) with w over sub-blocks s0..s1-1.
+// The dots of CN columns (kc of them real) with w over sub-blocks s0..s1-1. V:
+// the block's first row of the first column, in memory or on chip.
 template <int WIDTH, bool EXACT, int CN>
 __device__ __forceinline__ void ac_dot_task(const double* V, size_t ldv, int c0, int kc, int r0, int s0, int s1, int sl,
                                             const double* wv, const AcExchange& ex, AcShared& sh) {
@@ -244,7 +245,7 @@ __device__ __forceinline__ void ac_dot_task(const double* V, size_t ldv, int c0,
     for (int s = s0; s < s1; s += SU) {
         double2 v[SU][CN];
         const int lr = s * AC_SUB + 2 * lane;
-        const double* p = V + static_cast<size_t>(c0) * ldv + (r0 + lr);
+        const double* p = V + static_cast<size_t>(c0) * ldv + lr;
 #pragma unroll
         for (int u = 0; u < SU; ++u)
 #pragma unroll
@@ -279,10 +280,9 @@ __device__ __forceinline__ void ac_dot_task(const double* V, size_t ldv, int c0,
 // Dots of columns 0..k-1 of V with w over the block's rows into the exchange.
 // Warps take (group of up to eight columns, sub-block or row slice).
 template <int WIDTH, bool EXACT>
-__device__ __forceinline__ void ac_dots(const CycleArgs& g, const double* V, int k, int r0, int nsub,
+__device__ __forceinline__ void ac_dots(const CycleArgs& g, const double* V, size_t ldv, int k, int r0, int nsub,
                                         const double* wv, const AcExchange& ex, AcShared& sh) {
     const int warp = threadIdx.x >> 5;
-    const size_t ldv = static_cast<size_t>(g.ldv);
     const int cgs = (k + 7) >> 3;
     const int slices = EXACT ? nsub : max(1, min(nsub, AC_NW / cgs));
     for (int t = warp; t < cgs * slices; t += AC_NW) {
@@ -334,13 +334,13 @@ __device__ __forceinline__ void ac_sums(const AcExchange& ex, int k, int np, int
 // w -= V h over the block's rows (one FMA chain per row, in column order);
 // RU rows of a thread and CH columns in flight.
 template <int RU, int CH>
-__device__ __forceinline__ void ac_update_rows(const double* V, size_t ldv, int k, int r0, int rows, const double* h,
+__device__ __forceinline__ void ac_update_rows(const double* V, size_t ldv, int k, int rows, const double* h,
                                                double* w) {
     for (int r = threadIdx.x; r < rows; r += RU * AC_THREADS) {
         double s[RU];
 #pragma unroll
         for (int i = 0; i < RU; ++i) s[i] = 0.0;
-        const double* p = V + (r0 + r);
+        const double* p = V + r;
         for (int c = 0; c < k; c += CH, p += CH * ldv) {
             double v[RU][CH];
 #pragma unroll
@@ -360,11 +360,9 @@ __device__ __forceinline__ void ac_update_rows(const double* V, size_t ldv, int 
             if (r + i * AC_THREADS < rows) w[r + i * AC_THREADS] -= s[i];
     }
 }
-__device__ __forceinline__ void ac_update(const CycleArgs& g, const double* V, int k, int r0, int rows,
-                                          const double* h, double* w) {
-    const size_t ldv = static_cast<size_t>(g.ldv);
-    if (k <= 2 && rows > AC_THREADS) ac_update_rows<4, 2>(V, ldv, k, r0, rows, h, w);
-    else ac_update_rows<1, 8>(V, ldv, k, r0, rows, h, w);
+__device__ __forceinline__ void ac_update(const double* V, size_t ldv, int k, int rows, const double* h, double* w) {
+    if (k <= 2 && rows > AC_THREADS) ac_update_rows<4, 2>(V, ldv, k, rows, h, w);
+    else ac_update_rows<1, 8>(V, ldv, k, rows, h, w);
 }
 
 // ---- one or two columns --------------------------------------------------------
@@ -885,8 +883,10 @@ __device__ __forceinline__ double ac_norm_sum(const AcExchange& ex, int np) {
 
 // CLUSTER: one cluster, the separate kernels' sums. DIGITS: the sweeps over
 // the digit columns. WSMEM: the block's rows of w fit in shared memory (else
-// they stay in x). NARROW: a window of at most two columns.
-template <bool CLUSTER, bool DIGITS, bool WSMEM, bool NARROW = false>
+// they stay in x). NARROW: a window of at most two columns. VSMEM: the block's
+// rows of the basis too (they are read four times a step, and from L2 each
+// time costs a round trip).
+template <bool CLUSTER, bool DIGITS, bool WSMEM, bool NARROW = false, bool VSMEM = false>
 __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs g) {
     constexpr bool EXACT = CLUSTER;
     __shared__ AcShared sh;
@@ -923,12 +923,20 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         }
     };
     exchanges(0);
+    // the block's rows of the columns in shared memory, column c at c * rows
+    double* const vs = ac_smem + g.rows + (CLUSTER ? (2 * g.m + 1) * AC_PS : 0);
+    if (VSMEM) {
+        for (int r = threadIdx.x; r < rows; r += AC_THREADS) vs[r] = r < n_rows ? g.V[r0 + r] : 0.0;
+        __syncthreads();
+    }
     if (CLUSTER) cooperative_groups::this_cluster().sync();  // every block runs before another writes to its memory
     if (!CLUSTER && lead && ac_test_dead_wait(&st->status, g.bar)) return;
     for (int j = g.j0; j < g.j1; ++j) {
         const int lo = g.window > 0 ? max(0, j + 1 - g.window) : 0;
         const int k = j + 1 - lo;
         const double* V = g.V + static_cast<size_t>(lo) * ldv;
+        const double* const Vb = VSMEM ? vs + lo * rows : V + r0;
+        const size_t ldb = VSMEM ? static_cast<size_t>(rows) : ldv;
         const bool scaled = j > g.j0 && g.scale_gather;
         if (!EXACT) exchanges(j & 1);
         if (g.product) {
@@ -938,9 +946,9 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         }
         __syncthreads();
         auto dots = [&](const AcExchange& e) {
-            if (k <= 8) ac_dots<0, EXACT>(g, V, k, r0, nsub, w, e, sh);
-            else if (k <= 16) ac_dots<1, EXACT>(g, V, k, r0, nsub, w, e, sh);
-            else ac_dots<2, EXACT>(g, V, k, r0, nsub, w, e, sh);
+            if (k <= 8) ac_dots<0, EXACT>(g, Vb, ldb, k, r0, nsub, w, e, sh);
+            else if (k <= 16) ac_dots<1, EXACT>(g, Vb, ldb, k, r0, nsub, w, e, sh);
+            else ac_dots<2, EXACT>(g, Vb, ldb, k, r0, nsub, w, e, sh);
         };
         constexpr bool narrow = NARROW;
         double sum[2];
@@ -972,7 +980,7 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
             ac_coefficients(lo, k, sh.h1, sh);
             mag = ac_block_mag(ac_update_digits(g, lo, k, r0, rows, w, sh.h1, sh), turn, sh);
         } else {
-            ac_update(g, V, k, r0, rows, sh.h1, w);
+            ac_update(Vb, ldb, k, rows, sh.h1, w);
             __syncthreads();
         }
         if (g.reortho) {
@@ -987,7 +995,7 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
                 ac_coefficients(lo, k, sh.h, sh);
                 mag = ac_block_mag(ac_update_digits(g, lo, k, r0, rows, w, sh.h, sh), turn, sh);
             } else {
-                ac_update(g, V, k, r0, rows, sh.h, w);
+                ac_update(Vb, ldb, k, rows, sh.h, w);
             }
         }
         if (lead)
@@ -1031,6 +1039,13 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
                 sh.vexp[j + 1] = E;
                 g.vexp[(j + 1) * CYCLE_MAX_BLOCKS + blockIdx.x] = E;
             }
+        } else if (VSMEM && j + 1 < g.j1) {
+            double* const vq = vs + (j + 1) * rows;
+            for (int r = threadIdx.x; r < rows; r += AC_THREADS) {
+                const double v = w[r] * inv;
+                vq[r] = v;
+                if (r < n_rows) __stcg(q + r, v);
+            }
         } else {
             for (int r = threadIdx.x; r < n_rows; r += AC_THREADS) __stcg(q + r, w[r] * inv);
         }
@@ -1060,6 +1075,9 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
 int sm_total() { return std::min(device_sm_count(), CYCLE_MAX_BLOCKS); }
 
 }  // namespace
+
+// Dynamic shared memory beside the kernel's own.
+constexpr int AC_SMEM_TOTAL = 227 * 1024 - static_cast<int>(sizeof(AcShared)) - 64;
 
 bool arnoldi_cycle_fits(int n) { return n <= CYCLE_ROWS_MAX; }
 
@@ -1091,6 +1109,12 @@ int arnoldi_cycle_prepare() {
     MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cl));
     MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true>,
                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true, false, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM_TOTAL));
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true, false, true>,
+                                 cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, false, true, false, true>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM_TOTAL));
     MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
     MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
     MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, false, true, true>,
@@ -1132,6 +1156,13 @@ int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s) {
     if (!wsmem) a.scale_gather = 0;  // x holds w
     cfg.dynamicSmemBytes = sizeof(double) * ((wsmem ? static_cast<size_t>(a.rows) * (digits ? 2 : 1) : 0) +
                                              (cluster ? (2 * static_cast<size_t>(a.m) + 1) * AC_PS : 0));
+    // the basis on chip as well, where all m columns fit and one launch runs all steps. From L2 / on chip, one
+    // solve: random 1,500 rows 556 / 528 us, 20,000 753 / 727, 80,000 1222 / 1197; 8,000 rows, 100 columns 18.9 /
+    // 17.2 ms; heat 48^2 2854 / 2700 us, 300^2 5226 / 4997.
+    const size_t vbytes = sizeof(double) * static_cast<size_t>(a.rows) * a.m;
+    const bool vsmem = a.product && wsmem && !digits && !narrow &&
+                       cfg.dynamicSmemBytes + vbytes <= static_cast<size_t>(AC_SMEM_TOTAL);
+    if (vsmem) cfg.dynamicSmemBytes += vbytes;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     if (cluster) {
@@ -1148,7 +1179,9 @@ int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s) {
         cfg.numAttrs = 1;
     }
     cfg.attrs = attr;
-    const cudaError_t e = cluster           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true, false, true>, a)
+    const cudaError_t e = cluster && vsmem  ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true, false, true, false, true>, a)
+                          : cluster         ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true, false, true>, a)
+                          : vsmem           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, true, false, true>, a)
                           : narrow && wsmem ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, true, true>, a)
                           : narrow          ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, false, true>, a)
                           : digits && wsmem ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true, true>, a)
