@@ -363,11 +363,12 @@ struct GramArgs;
 // dots (FP32, a step j >= 1 over columns j-1 and j): the SpMV also
 // accumulates that step's a = U^T w and |w|^2 and its last block finishes the
 // step (the b partials come from the previous step's update, write_b).
-// direct: the unstaged form, one thread block per row block (no dots).
+// direct: the unstaged form, one thread block per row block (no dots);
+// uneven: its FP64 rows by length (matrices with rows longer than SEQ_ROW_MAX).
 template <typename TA, typename TX>
 int launch_spmv(int n, int nblocks, const int4* tiles, const uint16_t* col16, bool all_narrow, const int* row_ptr,
                 const int* col_idx, const TA* values, const TX* x, TX* y, const int* skip_flag, int* status,
-                cudaStream_t s, const GramArgs* dots = nullptr, bool direct = false);
+                cudaStream_t s, const GramArgs* dots = nullptr, bool direct = false, bool uneven = false);
 // w = A x in the pattern form; dots as for launch_spmv (FP32 only).
 template <typename TX>
 int launch_spmv_pattern(int n, int major, int major_len, int max_len, const uint8_t* pid, const RowPatterns* T,

@@ -390,7 +390,8 @@ int context_spmv(mexk_context_t ctx, int j, bool fp32, const int* skip, cudaStre
                                             ctx->d_w32, skip, &ctx->d_state->status, s, dots, direct)
                 : launch_spmv<double, double>(ctx->n, ctx->nblocks, ctx->d_tiles, ctx->d_col16, ctx->spmv_narrow,
                                               ctx->d_row_ptr, ctx->d_col, ctx->d_val, ctx->d_V + j * ldv, ctx->d_w,
-                                              skip, &ctx->d_state->status, s, dots, direct);
+                                              skip, &ctx->d_state->status, s, dots, direct,
+                                              ctx->max_row > SEQ_ROW_MAX);
 }
 
 // m: size of the basis being built in order (0 for a step on its own: then

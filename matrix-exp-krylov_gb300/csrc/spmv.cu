@@ -618,9 +618,16 @@ __device__ __forceinline__ void gquad<double>(const double* p, double (&o)[4]) {
 // (every product a separate gather, e.g. the power-law rows) this form is
 // faster, for banded ones the staged form is. A context runs this form when
 // some row block's columns span 65,536 or more (the staged form's 16-bit
-// column layout does not apply).
-template <typename TA, typename TX>
-__global__ void __launch_bounds__(ST_THREADS)
+// column layout does not apply). SORT (FP64, matrices with a row longer than
+// SEQ_ROW_MAX): an add of a warp holds its scheduler's
+// FP64 units for 64 cycles however few of its rows still have entries: on
+// power-law rows (mean 14 entries, up to 64 summed by one thread) in matrix
+// order the adds took 26 of 58 us at 300,007 rows; the rows go by length (48 us
+// in all, four blocks an SM; three 52, five 54 with spills), the same sums. Rows
+// of even lengths only pay for the ranks (400,000 random rows: a solve 2968 us
+// without, 3113 with).
+template <typename TA, typename TX, bool SORT>
+__global__ void __launch_bounds__(ST_THREADS, sizeof(TX) == 8 ? 4 : 0)
     spmv_direct_kernel(int nblocks, const int4* __restrict__ tiles, const int* __restrict__ row_ptr,
                        const int* __restrict__ col_idx, const TA* __restrict__ values, const TX* __restrict__ x,
                        TX* __restrict__ y, const int* __restrict__ skip) {
@@ -630,6 +637,10 @@ __global__ void __launch_bounds__(ST_THREADS)
     __shared__ TP red[32];
     __shared__ int s_long[ST_TILE / (SEQ_ROW_MAX + 1) + 1];
     __shared__ int s_nlong;
+    // SORT: the rows of at most SEQ_ROW_MAX entries by falling length, so that a
+    // warp's rows are about as long as one another
+    __shared__ int s_count[SORT ? SEQ_ROW_MAX + 1 : 1], s_start[SORT ? SEQ_ROW_MAX + 1 : 1];
+    __shared__ unsigned s_row[SORT ? ST_ROWS : 1];  // first product, length, row
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int b = blockIdx.x;
@@ -670,6 +681,38 @@ __global__ void __launch_bounds__(ST_THREADS)
             cq[q] = make_int4(0, 0, 0, 0);
         }
     }
+    if constexpr (SORT) {
+        // while the entries are on their way: ranks among the rows of a length
+        static_assert(SEQ_ROW_MAX == 64 && ST_ROWS <= 512 && QMAX * 4 <= 4096, "a warp's scan, a row's packing");
+        if (tid <= SEQ_ROW_MAX) s_count[tid] = 0;
+        __syncthreads();
+        int rank[ST_RPT];
+#pragma unroll
+        for (int q = 0; q < ST_RPT; ++q) {
+            const bool on = r0 + tid + q * ST_THREADS < r1 && rz[q] - ra[q] <= SEQ_ROW_MAX;
+            rank[q] = on ? atomicAdd(&s_count[rz[q] - ra[q]], 1) : -1;
+        }
+        __syncthreads();
+        if (tid < 32) {  // lengths 64 - 2 tid and 63 - 2 tid
+            const int v0 = s_count[SEQ_ROW_MAX - 2 * tid], v1 = s_count[SEQ_ROW_MAX - 1 - 2 * tid];
+            int x = v0 + v1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += up;
+            }
+            s_start[SEQ_ROW_MAX - 2 * tid] = x - v0 - v1;
+            s_start[SEQ_ROW_MAX - 1 - 2 * tid] = x - v1;
+            if (tid == 31) s_start[0] = x;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < ST_RPT; ++q)
+            if (rank[q] >= 0)
+                s_row[s_start[rz[q] - ra[q]] + rank[q]] = static_cast<unsigned>(ra[q] - base) |
+                                                          static_cast<unsigned>(rz[q] - ra[q]) << 12 |
+                                                          static_cast<unsigned>(tid + q * ST_THREADS) << 19;
+    }
     pdl_wait();
     if (skip != nullptr && *skip) return;
     if (b == static_cast<int>(gridDim.x) - 1) pdl_trigger();
@@ -697,11 +740,21 @@ __global__ void __launch_bounds__(ST_THREADS)
         if (r < r1) {
             if (rz[q] - ra[q] > SEQ_ROW_MAX) {
                 s_long[atomicAdd(&s_nlong, 1)] = r;
-            } else {
+            } else if (!SORT) {
                 TP s = 0;
                 for (int p = ra[q] - base; p < rz[q] - base; ++p) s += prod[p];
                 y[r] = static_cast<TX>(s);
             }
+        }
+    }
+    if constexpr (SORT) {
+        const int rows = s_start[0] + s_count[0];
+        for (int i = tid; i < rows; i += ST_THREADS) {
+            const unsigned w = s_row[i];
+            const int p0 = w & 4095u, p1 = p0 + static_cast<int>((w >> 12) & 127u);
+            TP s = 0;
+            for (int p = p0; p < p1; ++p) s += prod[p];
+            y[r0 + static_cast<int>(w >> 19)] = static_cast<TX>(s);
         }
     }
     __syncthreads();
@@ -748,9 +801,13 @@ int launch_spmv_as(int nblocks, const int4* tiles, const uint16_t* col16, const 
 
 template <typename TA, typename TX>
 int launch_spmv_direct(int nblocks, const int4* tiles, const int* row_ptr, const int* col_idx, const TA* values,
-                       const TX* x, TX* y, const int* skip_flag, cudaStream_t s) {
-    const cudaError_t e = launch_dependent(spmv_direct_kernel<TA, TX>, nblocks, ST_THREADS, 0, s, nblocks, tiles,
-                                           row_ptr, col_idx, values, x, y, skip_flag);
+                       const TX* x, TX* y, const int* skip_flag, bool uneven, cudaStream_t s) {
+    const cudaError_t e =
+        uneven && sizeof(TX) == 8
+            ? launch_dependent(spmv_direct_kernel<TA, TX, sizeof(TX) == 8>, nblocks, ST_THREADS, 0, s, nblocks, tiles,
+                               row_ptr, col_idx, values, x, y, skip_flag)
+            : launch_dependent(spmv_direct_kernel<TA, TX, false>, nblocks, ST_THREADS, 0, s, nblocks, tiles, row_ptr,
+                               col_idx, values, x, y, skip_flag);
     if (e != cudaSuccess) {
         set_cuda_error(e, "spmv_direct_kernel", __FILE__, __LINE__);
         return MEXK_ERR_CUDA;
@@ -761,7 +818,7 @@ int launch_spmv_direct(int nblocks, const int4* tiles, const int* row_ptr, const
 template <typename TA, typename TX>
 int launch_spmv(int n, int nblocks, const int4* tiles, const uint16_t* col16, bool all_narrow, const int* row_ptr,
                 const int* col_idx, const TA* values, const TX* x, TX* y, const int* skip_flag, int* status,
-                cudaStream_t s, const GramArgs* dots, bool direct) {
+                cudaStream_t s, const GramArgs* dots, bool direct, bool uneven) {
     if (n <= 0 || nblocks <= 0) return MEXK_OK;
     if (reinterpret_cast<uintptr_t>(col_idx) % 16 != 0 || reinterpret_cast<uintptr_t>(values) % 16 != 0 ||
         reinterpret_cast<uintptr_t>(row_ptr) % 16 != 0 || reinterpret_cast<uintptr_t>(col16) % 16 != 0) {
@@ -769,7 +826,8 @@ int launch_spmv(int n, int nblocks, const int4* tiles, const uint16_t* col16, bo
         return MEXK_ERR_INVALID;
     }
     const GramArgs none{};
-    if (direct && !dots) return launch_spmv_direct<TA, TX>(nblocks, tiles, row_ptr, col_idx, values, x, y, skip_flag, s);
+    if (direct && !dots)
+        return launch_spmv_direct<TA, TX>(nblocks, tiles, row_ptr, col_idx, values, x, y, skip_flag, uneven, s);
     if constexpr (sizeof(TX) == 4) {
         if (dots) {
             // the staged form takes u_{j-1}.w itself (sym is the pattern form's)
@@ -790,10 +848,10 @@ int launch_spmv(int n, int nblocks, const int4* tiles, const uint16_t* col16, bo
 
 template int launch_spmv<double, double>(int, int, const int4*, const uint16_t*, bool, const int*, const int*,
                                          const double*, const double*, double*, const int*, int*, cudaStream_t,
-                                         const GramArgs*, bool);
+                                         const GramArgs*, bool, bool);
 template int launch_spmv<float, float>(int, int, const int4*, const uint16_t*, bool, const int*, const int*,
                                        const float*, const float*, float*, const int*, int*, cudaStream_t,
-                                       const GramArgs*, bool);
+                                       const GramArgs*, bool, bool);
 
 // FP32 copy of the FP64 matrix values for the mixed-precision form
 // (round to nearest).
