@@ -14,7 +14,7 @@
 // |w|^2 - h.c, into [1, 2): any p near it serves (the next step measures
 // the norm exactly), and this one costs no root and rounds nothing.
 //
-// Up to CL_ROWS rows the blocks are one cluster of 16 which meet at hardware
+// Up to 8,192 rows (gc_cluster) the blocks are one cluster of 16 which meet at hardware
 // barriers and write their partial sums into each other's shared memory;
 // beyond, a cooperative grid with bounded waits and exact integer sums
 // (cycle.cuh). Columns that do not fit on chip are read from L2.
@@ -32,7 +32,6 @@ constexpr int GC_THREADS = 512;
 constexpr int GC_NW = GC_THREADS / 32;
 constexpr int GC_SUB = 128;       // rows of a sub-block: one warp's float4s
 constexpr int GC_CLUSTER = 16;
-constexpr int CL_ROWS = 4096;
 constexpr int GC_EPT = 8;         // matrix entries a thread can keep
 constexpr int GC_TILE = GC_THREADS * GC_EPT;
 constexpr int GC_GROUP = 4;       // columns of a warp's task
@@ -685,13 +684,22 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gram_cycle_kernel(GramCycleArgs
 
 constexpr int GC_SMEM = 227 * 1024 - static_cast<int>(sizeof(GcShared)) - 1024;
 
+// Whether the blocks are one cluster. Up to 4,096 rows always; to 8,192, whose
+// rows are a thread's at most, where a block's entries stay few. Grid /
+// cluster, one solve: heat 66^2 1093 / 911 us, 90^2 1081 / 925 (110^2 1086 /
+// 1022, its window 2 889 / 868, 126^2 1080 / 1061); random rows of 11: 4,500
+// 417 / 365, 8,000 424 / 412, 10,000 420 / 461; power law 8,000 1664 / 1996.
+bool gc_cluster(int n, long long nnz, bool long_rows, bool csr) {
+    if (n <= 4096) return true;
+    return n <= GRAM_CLUSTER_ROWS && (!csr || (!long_rows && nnz <= 90000));
+}
+
 struct GcShape {
     int grid, rows, on;
     size_t smem;
 };
-GcShape gc_shape(int n, int m, bool csr) {
+GcShape gc_shape(int n, int m, bool cluster, bool csr) {
     GcShape s;
-    const bool cluster = n <= CL_ROWS;
     const int blocks = cluster ? GC_CLUSTER : std::min(device_sm_count(), CYCLE_MAX_BLOCKS);
     s.rows = ((n + blocks - 1) / blocks + 31) / 32 * 32;
     s.grid = cluster ? GC_CLUSTER : (n + s.rows - 1) / s.rows;
@@ -719,7 +727,7 @@ bool gram_cycle_fits(int n, long long nnz, int m, int max_row, bool pattern, int
     if (m < 1 || m > GRAM_M) return false;
     if (window > 0 && window <= 4 && n > 400000) return false;
     if (!pattern && (max_row > GC_LONG_MAX || nnz > (max_row > SEQ_ROW_MAX ? 600000 : 2000000))) return false;
-    return 8 * gc_shape(n, m, !pattern).on >= m;
+    return 8 * gc_shape(n, m, gc_cluster(n, nnz, max_row > SEQ_ROW_MAX, !pattern), !pattern).on >= m;
 }
 
 int gram_cycle_prepare() {
@@ -737,8 +745,8 @@ int gram_cycle_test_hook(int enable) {
 
 int launch_gram_cycle(GramCycleArgs a, cudaStream_t s) {
     if (a.m < 1 || a.m > GRAM_M || a.scale == INT_MAX) return MEXK_ERR_INVALID;
-    const bool cluster = a.n <= CL_ROWS;
-    const GcShape sp = gc_shape(a.n, a.m, a.pid == nullptr);
+    const bool cluster = gc_cluster(a.n, a.nnz, a.long_rows != 0, a.pid == nullptr);
+    const GcShape sp = gc_shape(a.n, a.m, cluster, a.pid == nullptr);
     if (sp.on < 1) return MEXK_ERR_UNSUPPORTED;
     a.rows = sp.rows;
     a.on = sp.on;

@@ -512,12 +512,14 @@ struct GramArgs {
 // V, H, the Gram state and the solver state written as the stepwise kernels
 // do, H(m, m-1) included. scale, bar, words: as CycleArgs. The products come
 // from the row patterns (pid, T) or the FP32 CSR arrays.
+constexpr int GRAM_CLUSTER_ROWS = 8192;  // one cluster at most (gc_cluster)
 struct GramCycleArgs {
     int n, m, ldv, ldh, reortho, window;
     int rows = 0, on = 0;  // rows per block, columns held on chip (the launch's)
     int scale;
     int max_len;           // of the row patterns
     int long_rows;         // whether a CSR row has more than SEQ_ROW_MAX entries
+    long long nnz;
     const int* row_ptr;
     const int* col_idx;
     const float* values;

@@ -546,10 +546,10 @@ int enqueue_arnoldi_cycle(mexk_context_t ctx, int m, int reortho, int window, cu
 }
 
 // Whether an FP32 basis is built in one launch, by stencil_cycle.cu (a window
-// of 2) or gram_cycle.cu (up to 4096 rows, where its blocks are a cluster,
-// also for a window of 2).
+// of 2) or gram_cycle.cu (up to GRAM_CLUSTER_ROWS, where its blocks are a
+// cluster, also for a window of 2: heat 90^2 881 / 777 us).
 bool use_stencil_cycle(mexk_context_t ctx, int m, int window) {
-    return window == 2 && ctx->n > 4096 && ctx->spmv_form32 == MEXK_SPMV_PATTERN &&
+    return window == 2 && ctx->n > GRAM_CLUSTER_ROWS && ctx->spmv_form32 == MEXK_SPMV_PATTERN &&
            stencil_cycle_fits(ctx->n, m, ctx->pat_major_len, ctx->pat_reach);
 }
 bool use_gram_cycle(mexk_context_t ctx, int m, int window) {
@@ -569,6 +569,7 @@ int enqueue_gram_cycle(mexk_context_t ctx, int m, int reortho, int window, cudaS
     a.scale = ctx->cycle_scale;
     a.max_len = ctx->pat_max_len;
     a.long_rows = ctx->max_row > SEQ_ROW_MAX ? 1 : 0;
+    a.nnz = ctx->nnz;
     a.row_ptr = ctx->d_row_ptr;
     a.col_idx = ctx->d_col;
     a.values = ctx->d_val32;

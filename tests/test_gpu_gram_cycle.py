@@ -1,6 +1,6 @@
 """The one-launch FP32 basis (rows on chip, Gram-corrected steps) around the
-edges of its sub-blocks (128 rows), blocks (32), the cluster (4096 rows) and
-the grid, with columns on and off chip, for each form of the product, with and
+edges of its sub-blocks (128 rows), blocks (32), the cluster (4096 to 8192
+rows) and the grid, with columns on and off chip, for each form of the product, with and
 without reorthogonalisation and with a window.
 
 With u = 2^-24, rows of at most 64 entries and at most 64 columns, one step's
@@ -42,6 +42,10 @@ CASES += [("random", 2000, 1, 1, 0), ("random", 2000, 33, 1, 0), ("random", 2000
           ("random", 300007, 40, 1, 0), ("powerlaw", 2048, 20, 1, 0), ("powerlaw", 12345, 20, 1, 0),
           ("longrow", 2000, 8, 1, 0), ("longrow", 6000, 8, 1, 0), ("heat", 7, 30, 1, 0), ("heat", 64, 30, 1, 3),
           ("heat", 64, 20, 0, 3), ("heat", 131, 17, 1, 0), ("heat", 131, 30, 1, 5), ("heat", 401, 40, 1, 0)]
+# the cluster's end: 8192 rows, 90,000 CSR entries, no long rows
+CASES += [("random", 8192, 12, 1, 0), ("random", 8193, 12, 1, 0), ("random", 9000, 40, 1, 0), ("random", 7001, 64, 1, 0),
+          ("powerlaw", 6001, 20, 1, 0), ("heat", 90, 40, 1, 0), ("heat", 91, 40, 1, 0), ("heat", 90, 30, 1, 2),
+          ("heat", 91, 30, 1, 2)]
 # a window of 2 in the row-pattern form: the recurrence on chip past 4096 rows (blocks of one edge, of two, with
 # row groups between them; a stencil that reaches past the edges)
 CASES += [("heat", N, 30, 1, 2) for N in (64, 65, 97, 131, 556, 700, 801, 1303)]
