@@ -178,3 +178,41 @@ def test_basis_launches_and_profile(kind, n, precision, window, one):
         assert ctx.basis_launches(5, precision, window) <= ctx.basis_launches(20, precision, window)
         t5, t20 = (ctx.profile_kernel("basis", j, 3, precision) for j in (4, 19))
         assert 0.0 < t5 < t20 < 50.0
+
+
+def test_contexts_in_threads_share_the_gpu():
+    """Cooperative, cluster and tensor-memory bases of several contexts at once: every
+    thread gets the bits it gets alone."""
+    import threading
+
+    from mexk.api import Context
+
+    jobs = []
+    for i, (kind, n, kw) in enumerate([("random", 20000, {}), ("random", 60000, dict(precision="mixed", controller="search")),
+                                       ("heat", 300, dict(precision="mixed", controller="search", window=2)),
+                                       ("heat", 120, dict(window=2)), ("random", 3000, {}),
+                                       ("heat", 500, dict(precision="mixed", controller="search", window=2))]):
+        A = make(kind, n)
+        jobs.append((A, 0.5 / A.max_abs(), kw, np.random.default_rng(i).uniform(0, 1, A.n)))
+    alone = []
+    for A, t, kw, v in jobs:
+        with Context(A, m_alloc=20) as ctx:
+            alone.append(ctx.expmv(v, t, 20, **kw)[0])
+    wrong = []
+
+    def work(i):
+        A, t, kw, v = jobs[i]
+        try:
+            with Context(A, m_alloc=20) as ctx:
+                for _ in range(10):
+                    if not np.array_equal(ctx.expmv(v, t, 20, **kw)[0], alone[i]):
+                        wrong.append((i, "differs"))
+        except Exception as e:  # reported below
+            wrong.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not wrong, wrong
