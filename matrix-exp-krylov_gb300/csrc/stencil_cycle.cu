@@ -145,16 +145,18 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) stencil_cycle_kernel(StencilArgs 
     // what a pattern takes of the major one
     const int len = g.len;
     for (int p = tid; p < PAT_MAX; p += SC_BLOCK) {
-        int mask = 0;
+        // each entry another one of the major pattern's, in its order: a row may store a column twice
+        int mask = 0, next = 0;
         const int pl = p < T->count ? __ldg(T->len + p) : 0;
-        for (int e = 0; e < pl; ++e) {
+        for (int e = 0; e < pl && mask != SC_OTHER; ++e) {
             const int o = __ldg(T->off + p * PAT_LEN + e);
             const float v = __ldg(T->v32 + p * PAT_LEN + e);
-            int hit = SC_OTHER;
+            int hit = -1;
 #pragma unroll
-            for (int q = 0; q < L; ++q)
-                if (q < len && g.off[q] == o && __float_as_int(g.val[q]) == __float_as_int(v)) hit = 1 << q;
-            mask |= hit;
+            for (int q = L - 1; q >= 0; --q)
+                if (q >= next && q < len && g.off[q] == o && __float_as_int(g.val[q]) == __float_as_int(v)) hit = q;
+            mask = hit < 0 ? SC_OTHER : mask | 1 << hit;
+            next = hit + 1;
         }
         sh.mask[p] = static_cast<unsigned char>(mask);
     }
