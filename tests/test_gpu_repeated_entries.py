@@ -38,7 +38,8 @@ def test_every_entry_counts(N, kind):
 
     A = grid(N, kind)
     v = np.random.default_rng(N).standard_normal(A.n)
-    M = sp.csr_matrix((A.values, A.col_idx, A.row_ptr), shape=(A.n, A.n))
+    M = sp.csr_matrix((A.values, A.col_idx, A.row_ptr), shape=(A.n, A.n), copy=True)
+    M.sum_duplicates()  # in place: of the copy
     t = 0.5 / abs(M).sum(axis=1).max()
     ref, term = v.copy(), v.copy()
     for i in range(1, 24):
