@@ -331,8 +331,9 @@ __device__ __forceinline__ void ac_sums(const AcExchange& ex, int k, int np, int
     __syncthreads();
 }
 
-// w -= V h over the block's rows (one FMA chain per row, in column order);
-// RU rows of a thread and CH columns in flight.
+// w -= V h over the block's rows (one FMA chain per row, in column order; not
+// the padding after them, which stays zero where h is not finite); RU rows of
+// a thread and CH columns in flight.
 template <int RU, int CH>
 __device__ __forceinline__ void ac_update_rows(const double* V, size_t ldv, int k, int rows, const double* h,
                                                double* w) {
@@ -370,7 +371,8 @@ __device__ __forceinline__ void ac_update(const double* V, size_t ldv, int k, in
 // columns once: the dots; the first update with the second dots; the second
 // update with the norm (a sweep of its own for each took 38 of a step's 85
 // thousand cycles at 777^2 rows, window 2). UPDATE: w -= h0 v0 + h1 v1.
-// The thread's sums of v0.w, v1.w (or |w|^2 in sum[0]) over its rows.
+// The thread's sums of v0.w, v1.w (or |w|^2 in sum[0]) over its rows, in
+// pairs: past the last row w stays zero, also where h is not finite.
 enum AcPass { AC_PASS_DOTS, AC_PASS_NORM };
 template <bool UPDATE, AcPass PASS>
 __device__ __forceinline__ void ac_narrow_pass(const double* V, size_t ldv, int k, int r0, int rows, const double* h,
@@ -404,6 +406,7 @@ __device__ __forceinline__ void ac_narrow_pass(const double* V, size_t ldv, int 
                     x[u].x = fma(h1, b[u].x, x[u].x);
                     x[u].y = fma(h1, b[u].y, x[u].y);
                 }
+                if (q + 1 == rows) x[u].y = 0.0;
                 *reinterpret_cast<double2*>(w + q) = x[u];
             }
             if (PASS == AC_PASS_DOTS) {
@@ -487,7 +490,7 @@ __device__ __forceinline__ void ac_coefficients(int lo, int k, const double* h, 
 // w -= V h over the block's rows (columns lo..lo+k-1), RP rows per thread and
 // eight columns in flight, three of each eight in FP64 and five in digits;
 // returns the thread's largest high word of |w|. Coefficients that are not
-// finite make w NaN, which ends the basis.
+// finite make w NaN, which ends the basis; the padding after the rows stays zero.
 template <int RP>
 __device__ __forceinline__ unsigned ac_update_digit_rows(const CycleArgs& g, int lo, int k, int r0, int rows, double* w,
                                                          const double* hc, const AcShared& sh) {
@@ -553,8 +556,8 @@ __device__ __forceinline__ unsigned ac_update_digit_rows(const CycleArgs& g, int
         }
 #pragma unroll
         for (int i = 0; i < RP; ++i) {
-            const double x =
-                finite ? w[r + i] - (f[i] + ac_row_value(a[i], E)) : __longlong_as_double(0x7ff8000000000000ll);
+            double x = finite ? w[r + i] - (f[i] + ac_row_value(a[i], E)) : __longlong_as_double(0x7ff8000000000000ll);
+            if (r + i >= rows) x = 0.0;
             w[r + i] = x;
             mag = max(mag, ac_mag(x));
         }
@@ -954,7 +957,7 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         double sum[2];
         unsigned mag = 0u;
         if (narrow) {
-            ac_narrow_pass<false, AC_PASS_DOTS>(V, ldv, k, r0, rows, nullptr, w, sum);
+            ac_narrow_pass<false, AC_PASS_DOTS>(V, ldv, k, r0, n_rows, nullptr, w, sum);
             ac_narrow_publish(g, k, sum, ex[0], sh);
         } else if (DIGITS) {
             for (int r = 2 * static_cast<int>(threadIdx.x); r < rows; r += 2 * AC_THREADS) {
@@ -974,13 +977,13 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         }
         ac_sums<EXACT>(ex[0], k, np, g.scale, sh.h1, sh);
         if (narrow) {
-            if (g.reortho) ac_narrow_pass<true, AC_PASS_DOTS>(V, ldv, k, r0, rows, sh.h1, w, sum);
-            else ac_narrow_pass<true, AC_PASS_NORM>(V, ldv, k, r0, rows, sh.h1, w, sum);
+            if (g.reortho) ac_narrow_pass<true, AC_PASS_DOTS>(V, ldv, k, r0, n_rows, sh.h1, w, sum);
+            else ac_narrow_pass<true, AC_PASS_NORM>(V, ldv, k, r0, n_rows, sh.h1, w, sum);
         } else if (DIGITS) {
             ac_coefficients(lo, k, sh.h1, sh);
-            mag = ac_block_mag(ac_update_digits(g, lo, k, r0, rows, w, sh.h1, sh), turn, sh);
+            mag = ac_block_mag(ac_update_digits(g, lo, k, r0, n_rows, w, sh.h1, sh), turn, sh);
         } else {
-            ac_update(Vb, ldb, k, rows, sh.h1, w);
+            ac_update(Vb, ldb, k, n_rows, sh.h1, w);
             __syncthreads();
         }
         if (g.reortho) {
@@ -990,12 +993,12 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
             if (!ac_meet<CLUSTER>(g.bar, target, &st->status, &sh.ok)) return;
             ac_sums<EXACT>(ex[1], k, np, g.scale, sh.h, sh);
             if (narrow) {
-                ac_narrow_pass<true, AC_PASS_NORM>(V, ldv, k, r0, rows, sh.h, w, sum);
+                ac_narrow_pass<true, AC_PASS_NORM>(V, ldv, k, r0, n_rows, sh.h, w, sum);
             } else if (DIGITS) {
                 ac_coefficients(lo, k, sh.h, sh);
-                mag = ac_block_mag(ac_update_digits(g, lo, k, r0, rows, w, sh.h, sh), turn, sh);
+                mag = ac_block_mag(ac_update_digits(g, lo, k, r0, n_rows, w, sh.h, sh), turn, sh);
             } else {
-                ac_update(Vb, ldb, k, rows, sh.h, w);
+                ac_update(Vb, ldb, k, n_rows, sh.h, w);
             }
         }
         if (lead)
