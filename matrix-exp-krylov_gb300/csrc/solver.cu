@@ -265,9 +265,11 @@ int ensure_mixed(mexk_context_t ctx) {
     int rc;
     if ((rc = dalloc(&ctx->d_V32, static_cast<size_t>(ctx->ldv) * (ctx->m_alloc + 1)))) return rc;
     if ((rc = dalloc(&ctx->d_w32, static_cast<size_t>(ctx->ldv)))) return rc;
-    // Rows n..ldv-1 stay zero: the vectorised sweeps read and write them.
-    MEXK_CK(cudaMemset(ctx->d_V32, 0, sizeof(float) * static_cast<size_t>(ctx->ldv) * (ctx->m_alloc + 1)));
-    MEXK_CK(cudaMemset(ctx->d_w32, 0, sizeof(float) * static_cast<size_t>(ctx->ldv)));
+    // Rows n..ldv-1 stay zero: the vectorised sweeps read and write them. (On the context's stream, synchronised
+    // below: it does not wait for the legacy default stream, whose queue may be long.)
+    MEXK_CK(cudaMemsetAsync(ctx->d_V32, 0, sizeof(float) * static_cast<size_t>(ctx->ldv) * (ctx->m_alloc + 1),
+                            ctx->stream));
+    MEXK_CK(cudaMemsetAsync(ctx->d_w32, 0, sizeof(float) * static_cast<size_t>(ctx->ldv), ctx->stream));
     if ((rc = dalloc(&ctx->d_gram, 1))) return rc;
     if ((rc = dalloc(&ctx->d_gram_part, static_cast<size_t>(GRAM_MAX_ROW_BLOCKS) * GRAM_SLOTS))) return rc;
     if ((rc = reset_gram(ctx, ctx->stream))) return rc;
@@ -282,14 +284,17 @@ int ensure_mixed(mexk_context_t ctx) {
 // any capture by the first solve that does, and done without when it does not
 // fit (those sweeps then run in FP64).
 void ensure_digits(mexk_context_t ctx, int window) {
-    if (ctx->d_vq || ctx->no_digits || !arnoldi_cycle_fits(ctx->n) || !arnoldi_cycle_digits(ctx->n, ctx->m_alloc, window)) return;
+    if (ctx->d_vq || ctx->no_digits || ctx->cycle_scale == INT_MAX || !arnoldi_cycle_fits(ctx->n) ||
+        !arnoldi_cycle_digits(ctx->n, ctx->m_alloc, window))
+        return;
     const size_t count = static_cast<size_t>(ctx->ldv) * (ctx->m_alloc + 2);  // the columns, then w's digits
     const size_t nexp = static_cast<size_t>(ctx->m_alloc + 1) * CYCLE_MAX_BLOCKS;
     if (cudaMalloc(reinterpret_cast<void**>(&ctx->d_vq), sizeof(unsigned long long) * count) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&ctx->d_vexp), sizeof(int) * nexp) != cudaSuccess ||
-        // rows n..ldv-1 stay zero
-        cudaMemset(ctx->d_vq, 0, sizeof(unsigned long long) * count) != cudaSuccess ||
-        cudaMemset(ctx->d_vexp, 0, sizeof(int) * nexp) != cudaSuccess) {
+        // rows n..ldv-1 stay zero; done before a solve on whichever stream
+        cudaMemsetAsync(ctx->d_vq, 0, sizeof(unsigned long long) * count, ctx->stream) != cudaSuccess ||
+        cudaMemsetAsync(ctx->d_vexp, 0, sizeof(int) * nexp, ctx->stream) != cudaSuccess ||
+        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         (void)cudaGetLastError();
         dfree(ctx->d_vq);
         dfree(ctx->d_vexp);
