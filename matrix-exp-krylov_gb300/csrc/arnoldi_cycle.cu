@@ -6,8 +6,9 @@
 // serial tails are what a step costs (about 40 us at 2,000 rows, 50 us at
 // 9,216, 100 us at 600,000 with a window of 2) while its FP64 arithmetic,
 // 8 n k flops at about two FMAs per clock per SM, would take 1 to 10 us.
-// Measured per step now: 13, 15 and 38 us; whole solves 1.2 to 2.8 times
-// faster from 2,000 to 4,000,000 rows. Here every thread block owns a
+// Measured per step now: 13, 15 and 38 us; whole solves 3.0 times faster at
+// 2,000 rows, 2.4 at 50,021 with 100 columns, 1.06 at 4,194,304 with 30, where
+// FP64 issue in the sweeps is nearly all of a step. Here every thread block owns a
 // contiguous range of rows for the whole basis, keeps its part of w in shared
 // memory, and the blocks meet three times a step, each time to exchange k (or
 // one) partial sums:
@@ -99,128 +100,17 @@ __device__ __forceinline__ void ac_place(int lane, int* column, int* copy) {
 extern __shared__ double ac_smem[];  // w (the block's rows); a cluster: then the exchanges' partials
 
 constexpr int AC_TILE = 2048;  // products staged at a time
-constexpr int AC_SMEM_DOUBLES = 22528;  // rows of w, and of its digits, that a block keeps in shared memory (176 KB)
+constexpr int AC_SMEM_DOUBLES = 22528;  // rows of w that a block keeps in shared memory (176 KB)
 
 struct AcShared {
     double h[MEXK_M_MAX];               // the second pass's coefficients
     double h1[MEXK_M_MAX];              // the first pass's
     double red[AC_NW][MEXK_M_MAX + 1];  // row slices' dots, then the partial sums' slices
     double prod[AC_TILE];
-    int4 hd[MEXK_M_MAX + 8];            // digits of the update's coefficients, zero past the last
-    int vexp[MEXK_M_MAX + 1];           // exponents of the block's digit columns
     double inv;
-    unsigned mag[3];                    // largest high words, by turns
-    int escale;
     int ok, nlong;
     int rows_long[AC_THREADS];
 };
-
-// ---- 61-bit fixed point in three digits ---------------------------------------
-// This GPU issues about 1.7 FP64 FMAs per clock and SM, where memory delivers
-// 2.1 (from L2) to 2.6 (HBM, long columns) doubles; integer multiply-adds of
-// 32 bits into 64 run at 60. So a wide basis also keeps its columns as
-// X = v 2^(61-E), |X| < 2^61 rounded to nearest, with one exponent E per
-// block and column, packed as three balanced 21-bit digits (d2 2^42 + d1 2^21
-// + d0), and w and h are taken to the same form: a product's six leading
-// digit products are exact in three 64-bit sums, what is dropped is below
-// 2^-60 of the largest product. The quantum, 2^-62 of the block's largest
-// entry, keeps a dot or update at least as close to exact as FP64's rounding
-// of 2^-53 per entry: by 2^6 for entries of similar size, and for one large
-// entry among 27,000 small ones in every block by sqrt(27000) 2^-62 = 2^-54.6
-// against 2^-53. An element costs about 20 integer instructions (2.4 elements
-// per clock alone), so of each eight columns three stay on the FP64 units,
-// which work beside the integer ones. Sweeps of heat 2048^2 (27,600 rows a
-// block): 249,000 / 298,000 clocks a dot / update sweep in FP64, 228,000 /
-// 217,000 so.
-constexpr int AC_FRAC = 61;
-constexpr int AC_FP64_COLS = 3;  // of eight columns, those left to the FP64 units, which work beside the integer ones
-constexpr unsigned long long AC_BIAS = (1ull << 20) | (1ull << 41);
-struct Digits {
-    int d2, d1, d0;
-};
-__device__ __forceinline__ unsigned long long ac_pack(double v, int E) {
-    const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v));
-    const int e = static_cast<int>((u >> 52) & 0x7ff);
-    const unsigned long long m = e ? (u & 0xfffffffffffffull) | 0x10000000000000ull : 0ull;
-    const int sh = e - 1075 - (E - AC_FRAC);
-    unsigned long long x;
-    if (sh >= 0) x = m << sh;  // |v| < 2^E: sh <= 8
-    else x = sh > -55 ? (m + (1ull << (-sh - 1))) >> -sh : 0ull;
-    if (u >> 63) x = 0ull - x;
-    return (x + AC_BIAS) ^ AC_BIAS;  // balanced digits in two's complement fields
-}
-__device__ __forceinline__ Digits ac_digits(unsigned long long p) {
-    const unsigned lo = static_cast<unsigned>(p), hi = static_cast<unsigned>(p >> 32);
-    Digits d;
-    d.d2 = static_cast<int>(hi) >> 10;
-    d.d1 = static_cast<int>(__funnelshift_l(lo, hi, 22)) >> 11;
-    d.d0 = static_cast<int>(lo << 11) >> 11;
-    return d;
-}
-// s + a b in one integer instruction
-__device__ __forceinline__ void ac_mad(long long& s, int a, int b) {
-    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(s) : "r"(a), "r"(b));
-}
-struct DigitSum {
-    long long s4, s3, s2;  // weights 2^84, 2^63, 2^42
-    __device__ __forceinline__ void zero() { s4 = s3 = s2 = 0; }
-    __device__ __forceinline__ void add(const Digits& a, const Digits& b) {
-        ac_mad(s4, a.d2, b.d2);
-        ac_mad(s3, a.d2, b.d1);
-        ac_mad(s2, a.d2, b.d0);
-        ac_mad(s3, a.d1, b.d2);
-        ac_mad(s2, a.d1, b.d1);
-        ac_mad(s2, a.d0, b.d2);
-    }
-    // the sum times 2^E as a double, rounded once (integer arithmetic: a
-    // conversion would cost an FP64 instruction per part)
-    __device__ __forceinline__ double value(int E) const {
-        __int128 t = (static_cast<__int128>(s4) << 42) + (static_cast<__int128>(s3) << 21) + s2;
-        const bool neg = t < 0;
-        if (neg) t = -t;
-        const unsigned long long hi = static_cast<unsigned long long>(t >> 64), lo = static_cast<unsigned long long>(t);
-        if ((hi | lo) == 0ull) return 0.0;
-        const int lz = hi ? __clzll(static_cast<long long>(hi)) : 64 + __clzll(static_cast<long long>(lo));
-        const unsigned __int128 n = static_cast<unsigned __int128>(t) << lz;  // leading one at bit 127
-        const unsigned long long top = static_cast<unsigned long long>(n >> 64);
-        const int e = 127 - lz + 42 + E + 1023;  // biased exponent of the leading one
-        if (e <= 0 || e >= 2046) return ldexp(neg ? -static_cast<double>(top) : static_cast<double>(top), e - 1023 - 63);
-        unsigned long long b = (static_cast<unsigned long long>(e) << 52) + ((top >> 11) & 0xfffffffffffffull);
-        b += (top >> 10) & 1ull;  // to nearest, ties away (the bits below are not looked at)
-        return __longlong_as_double(static_cast<long long>(b | (neg ? 1ull << 63 : 0ull)));
-    }
-};
-// The same for one row of an update, whose coefficients have AC_HFRAC bits:
-// (s4 2^21 + s3 + s2 / 2^21) stays inside 64 bits for 128 columns.
-constexpr int AC_HFRAC = 57;
-__device__ __forceinline__ double ac_row_value(const DigitSum& s, int E) {
-    long long hi = (s.s4 << 21) + s.s3 + (s.s2 >> 21);
-    unsigned lo = static_cast<unsigned>(s.s2) & 0x1fffffu;
-    const bool neg = hi < 0;
-    if (neg) {  // -(hi 2^21 + lo)
-        hi = lo ? ~hi : -hi;
-        lo = (0u - lo) & 0x1fffffu;
-    }
-    unsigned long long u = static_cast<unsigned long long>(hi);
-    int shift = 63;  // weight 2^63 per unit of u
-    if (u >> 32 == 0ull) {  // fewer than 53 bits above lo: bring it in
-        u = (u << 21) | lo;
-        lo = 0u;
-        shift = 42;
-    }
-    if (u == 0ull) return 0.0;
-    const int lz = __clzll(static_cast<long long>(u));
-    u = (u << lz) | (lz <= 21 ? lo >> (21 - lz) : static_cast<unsigned long long>(lo) << (lz - 21));
-    const int e = 63 - lz + shift + E + 1023;
-    if (e <= 0 || e >= 2046) return ldexp(neg ? -static_cast<double>(u) : static_cast<double>(u), e - 1023 - 63);
-    const unsigned long long b =
-        (static_cast<unsigned long long>(e) << 52) + ((u >> 11) & 0xfffffffffffffull) + ((u >> 10) & 1ull);
-    return __longlong_as_double(static_cast<long long>(b | (neg ? 1ull << 63 : 0ull)));
-}
-// E with |v| < 2^E from the high word of |v| (0 for a zero or subnormal v)
-__device__ __forceinline__ int ac_exponent(unsigned hi) { return static_cast<int>(hi >> 20) - 1022; }
-__device__ __forceinline__ unsigned ac_mag(double v) { return static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu; }
-constexpr unsigned AC_INF = 0x7ff00000u;
 
 // One exchange: where the partial sums go. EXACT: part (in every block's
 // shared memory), column c's sub-block b at part[c * AC_PS + b]. Else the
@@ -438,283 +328,6 @@ __device__ __forceinline__ void ac_narrow_publish(const CycleArgs& g, int k, dou
     ac_publish<AC_THREADS>(ex.words, &sh.red[0][0], MEXK_M_MAX + 1, k, AC_NW, g.scale);
 }
 
-// ---- the sweeps over the digit columns ---------------------------------------
-// Largest high word over the block of m (every thread calls it); the three
-// slots are used by turns.
-__device__ __forceinline__ unsigned ac_block_mag(unsigned m, int& turn, AcShared& sh) {
-    const int slot = turn;
-    turn = slot == 2 ? 0 : slot + 1;
-    m = __reduce_max_sync(AC_FULL, m);
-    if ((threadIdx.x & 31) == 0 && m != 0u) atomicMax(&sh.mag[slot], m);
-    __syncthreads();
-    const unsigned r = sh.mag[slot];
-    if (threadIdx.x == 0) sh.mag[slot == 0 ? 2 : slot - 1] = 0u;  // the last turn's: read by all before this barrier
-    return r;
-}
-
-// Digits of the update's coefficients: h_c 2^(E_c) relative to the largest
-// (E_c: the exponent of column lo + c in this block); sh.escale its exponent,
-// INT_MAX when a coefficient is not finite.
-__device__ __forceinline__ void ac_coefficients(int lo, int k, const double* h, AcShared& sh) {
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        int E[MEXK_M_MAX / 32], best = INT_MIN;
-        bool finite = true;
-#pragma unroll
-        for (int i = 0; i < MEXK_M_MAX / 32; ++i) {
-            const int c = lane + 32 * i;
-            E[i] = INT_MIN;
-            if (c < k && (ac_mag(h[c]) >> 20) != 0u) {
-                finite = finite && ac_mag(h[c]) < AC_INF;
-                E[i] = sh.vexp[lo + c];
-                best = max(best, E[i] + ac_exponent(ac_mag(h[c])));
-            }
-        }
-        best = __reduce_max_sync(AC_FULL, best);
-        if (best == INT_MIN) best = 0;
-#pragma unroll
-        for (int i = 0; i < MEXK_M_MAX / 32; ++i) {
-            const int c = lane + 32 * i;
-            if (c < 8) sh.hd[k + c] = make_int4(0, 0, 0, 0);
-            if (c < k) {
-                const Digits d = E[i] == INT_MIN ? Digits{0, 0, 0} : ac_digits(ac_pack(h[c], best - E[i] + AC_FRAC - AC_HFRAC));
-                sh.hd[c] = make_int4(d.d2, d.d1, d.d0, 0);
-            }
-        }
-        finite = __all_sync(AC_FULL, finite);
-        if (lane == 0) sh.escale = finite ? best : INT_MAX;
-    }
-    __syncthreads();
-}
-
-// w -= V h over the block's rows (columns lo..lo+k-1), RP rows per thread and
-// eight columns in flight, three of each eight in FP64 and five in digits;
-// returns the thread's largest high word of |w|. Coefficients that are not
-// finite make w NaN, which ends the basis; the padding after the rows stays zero.
-template <int RP>
-__device__ __forceinline__ unsigned ac_update_digit_rows(const CycleArgs& g, int lo, int k, int r0, int rows, double* w,
-                                                         const double* hc, const AcShared& sh) {
-    constexpr int CH = 8;
-    const size_t ldv = static_cast<size_t>(g.ldv);
-    const bool finite = sh.escale != INT_MAX;
-    const int E = sh.escale - AC_HFRAC - AC_FRAC;
-    const ptrdiff_t qoff = reinterpret_cast<const char*>(g.vq) - reinterpret_cast<const char*>(g.V);
-    unsigned mag = 0u;
-    unsigned long long v[CH][RP];
-    // each column's registers are reloaded, for the next eight columns or the
-    // next rows, as soon as they are used: the loads stay in flight
-    const char* next = reinterpret_cast<const char*>(g.V + static_cast<size_t>(lo) * ldv + r0 +
-                                                     RP * static_cast<int>(threadIdx.x));
-    auto load = [&](int u, bool on) {  // column u of the eight at next
-        const char* p = next + static_cast<size_t>(u) * ldv * 8 + (u < AC_FP64_COLS ? 0 : qoff);
-        if constexpr (RP == 2) {
-            const ulonglong2 t = on ? *reinterpret_cast<const ulonglong2*>(p) : make_ulonglong2(0ull, 0ull);
-            v[u][0] = t.x;
-            v[u][1] = t.y;
-        } else {
-            v[u][0] = on ? *reinterpret_cast<const unsigned long long*>(p) : 0ull;
-        }
-    };
-    int r = RP * static_cast<int>(threadIdx.x);
-#pragma unroll
-    for (int u = 0; u < CH; ++u) load(u, r < rows && u < k);
-    for (; r < rows; r += RP * AC_THREADS) {
-        DigitSum a[RP];
-        double f[RP];
-#pragma unroll
-        for (int i = 0; i < RP; ++i) {
-            a[i].zero();
-            f[i] = 0.0;
-        }
-        const char* const here = next;
-        const char* p = here;
-        for (int c = 0; c < k; c += CH) {
-            const bool more = c + CH < k;
-            p += CH * ldv * 8;
-            if (!more) p = here + RP * AC_THREADS * 8;
-            next = p;
-            const bool on = more || r + RP * AC_THREADS < rows;
-            const int left = more ? k - c - CH : k;
-#pragma unroll
-            for (int u = 0; u < CH; ++u) {
-                if (u < AC_FP64_COLS) {
-                    const double h = c + u < k ? hc[c + u] : 0.0;
-#pragma unroll
-                    for (int i = 0; i < RP; ++i) f[i] = fma(__longlong_as_double(static_cast<long long>(v[u][i])), h, f[i]);
-                    load(u, on && u < left);
-                } else {
-                    const int4 h4 = sh.hd[c + u];  // zero past column k
-                    const Digits h = {h4.x, h4.y, h4.z};
-                    Digits d[RP];
-#pragma unroll
-                    for (int i = 0; i < RP; ++i) d[i] = ac_digits(v[u][i]);
-                    load(u, on && u < left);
-#pragma unroll
-                    for (int i = 0; i < RP; ++i) a[i].add(d[i], h);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < RP; ++i) {
-            double x = finite ? w[r + i] - (f[i] + ac_row_value(a[i], E)) : __longlong_as_double(0x7ff8000000000000ll);
-            if (r + i >= rows) x = 0.0;
-            w[r + i] = x;
-            mag = max(mag, ac_mag(x));
-        }
-    }
-    return mag;
-}
-__device__ __forceinline__ unsigned ac_update_digits(const CycleArgs& g, int lo, int k, int r0, int rows, double* w,
-                                                     const double* hc, const AcShared& sh) {
-    // pairs of rows where they leave no larger share of the threads idle in the last round
-    const bool pairs = 2 * ((rows + 2 * AC_THREADS - 1) / (2 * AC_THREADS)) <= (rows + AC_THREADS - 1) / AC_THREADS;
-    return pairs ? ac_update_digit_rows<2>(g, lo, k, r0, rows, w, hc, sh)
-                 : ac_update_digit_rows<1>(g, lo, k, r0, rows, w, hc, sh);
-}
-
-// The warp's dots of CN columns from c0 (kc of them real) with w over
-// sub-blocks s0..s1-1, into red[sl]: the first ND in FP64, the rest in digits.
-template <int CN>
-__device__ __forceinline__ void ac_digit_task(const CycleArgs& g, int lo, int c0, int kc, int r0, int s0, int s1, int sl,
-                                              const double* w, const unsigned long long* wq, int E, bool finite,
-                                              AcShared& sh) {
-    constexpr int ND = CN == 8 ? AC_FP64_COLS : CN >= 4 ? 2 : CN / 2;
-    const int lane = threadIdx.x & 31;
-    const size_t ldv = static_cast<size_t>(g.ldv);
-    DigitSum acc[CN - ND];
-    double f[ND > 0 ? ND : 1];
-#pragma unroll
-    for (int c = 0; c < CN - ND; ++c) acc[c].zero();
-#pragma unroll
-    for (int c = 0; c < ND; ++c) f[c] = 0.0;
-    const size_t off = static_cast<size_t>(lo + c0) * ldv + (r0 + s0 * AC_SUB + 2 * lane);
-    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(g.V + off);
-    const ulonglong2* pq = reinterpret_cast<const ulonglong2*>(g.vq + off);
-    const size_t ld2 = ldv / 2;
-    ulonglong2 v[CN];
-    auto load = [&](int c, bool on) {
-        v[c] = (c < kc && on) ? (c < ND ? p : pq)[c * ld2] : make_ulonglong2(0ull, 0ull);
-    };
-#pragma unroll
-    for (int c = 0; c < CN; ++c) load(c, s0 < s1);
-    for (int s = s0; s < s1; ++s) {
-        p += AC_SUB / 2;
-        pq += AC_SUB / 2;
-        const int lr = s * AC_SUB + 2 * lane;
-        const double2 x = *reinterpret_cast<const double2*>(w + lr);
-        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(wq + lr);
-        const Digits x0 = ac_digits(q.x), x1 = ac_digits(q.y);
-        const bool more = s + 1 < s1;
-        // a column's registers are reloaded as soon as it is used: the loads stay in flight
-#pragma unroll
-        for (int c = 0; c < ND; ++c) {
-            f[c] = fma(__longlong_as_double(static_cast<long long>(v[c].x)), x.x, f[c]);
-            f[c] = fma(__longlong_as_double(static_cast<long long>(v[c].y)), x.y, f[c]);
-            load(c, more);
-        }
-#pragma unroll
-        for (int c = ND; c < CN; ++c) {
-            const Digits d0 = ac_digits(v[c].x), d1 = ac_digits(v[c].y);
-            load(c, more);
-            acc[c - ND].add(d0, x0);
-            acc[c - ND].add(d1, x1);
-        }
-    }
-    if constexpr (ND > 0) {
-        constexpr int NP = ND > 2 ? 4 : ND;
-        double t[NP];
-#pragma unroll
-        for (int c = 0; c < NP; ++c) t[c] = c < ND ? f[c < ND ? c : 0] : 0.0;
-        const double tot = ac_reduce<2, NP>(t, lane);
-        int c, copy;
-        ac_place<2, NP>(lane, &c, &copy);
-        if (copy == 0 && c < ND && c < kc) sh.red[sl][c0 + c] = tot;
-    }
-    // the warp's totals, the columns transposed over the lanes
-    constexpr int CQ = CN - ND, CP = CQ > 4 ? 8 : CQ > 2 ? 4 : CQ;  // a power of two
-    DigitSum sum[CP];
-#pragma unroll
-    for (int c = 0; c < CP; ++c) {
-        if (c < CQ) sum[c] = acc[c < CQ ? c : 0];
-        else sum[c].zero();
-    }
-    auto swap_add = [&](long long& keep_lo, long long hi, bool up, int b) {
-        const long long send = up ? keep_lo : hi, keep = up ? hi : keep_lo;
-        keep_lo = keep + __shfl_xor_sync(AC_FULL, send, b);
-    };
-    int b = 16, cc = 0;
-#pragma unroll
-    for (int h = CP / 2; h >= 1; h >>= 1, b >>= 1) {
-        const bool up = (lane & b) != 0;
-        if (up) cc += h;
-#pragma unroll
-        for (int i = 0; i < h; ++i) {
-            swap_add(sum[i].s4, sum[i + h].s4, up, b);
-            swap_add(sum[i].s3, sum[i + h].s3, up, b);
-            swap_add(sum[i].s2, sum[i + h].s2, up, b);
-        }
-    }
-    const int rest = 2 * b - 1;  // the lane bits that name copies
-    for (; b >= 1; b >>= 1) {
-        sum[0].s4 += __shfl_xor_sync(AC_FULL, sum[0].s4, b);
-        sum[0].s3 += __shfl_xor_sync(AC_FULL, sum[0].s3, b);
-        sum[0].s2 += __shfl_xor_sync(AC_FULL, sum[0].s2, b);
-    }
-    cc += ND;
-    if ((lane & rest) == 0 && cc < kc) {
-        const double t = sum[0].value(E + sh.vexp[lo + c0 + cc] - 2 * AC_FRAC);
-        sh.red[sl][c0 + cc] = finite ? t : __longlong_as_double(0x7ff8000000000000ll);
-    }
-}
-
-// Dots of all k columns with w over the block's rows into the exchange: w's
-// digits first (relative to its largest entry in the block, whose high word
-// is mag), then every warp its (group of columns, row slice) without meeting.
-__device__ __forceinline__ void ac_dots_digits(const CycleArgs& g, int lo, int k, int r0, int nsub, const double* w,
-                                               unsigned mag, unsigned long long* wq, const AcExchange& ex,
-                                               AcShared& sh) {
-    const int warp = threadIdx.x >> 5;
-    const bool finite = mag < AC_INF;
-    const int E = ac_exponent(min(mag, AC_INF - 1u));
-    for (int r = 2 * static_cast<int>(threadIdx.x); r < nsub * AC_SUB; r += 2 * AC_THREADS) {
-        const double2 x = *reinterpret_cast<const double2*>(w + r);
-        *reinterpret_cast<ulonglong2*>(wq + r) = finite ? make_ulonglong2(ac_pack(x.x, E), ac_pack(x.y, E))
-                                                        : make_ulonglong2(0ull, 0ull);
-    }
-    __syncthreads();
-    const int cgs = (k + 7) >> 3;  // groups of columns as even as they come
-    const int slices = max(1, min(nsub, AC_NW / cgs));
-    const int cg = warp % cgs, sl = warp / cgs;  // at most one task per warp: cgs <= AC_NW
-    if (sl < slices) {
-        const int c0 = cg * k / cgs, kc = (cg + 1) * k / cgs - c0;
-        const int s0 = sl * nsub / slices, s1 = (sl + 1) * nsub / slices;
-        if (kc > 6) ac_digit_task<8>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
-        else if (kc > 4) ac_digit_task<6>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
-        else if (kc > 2) ac_digit_task<4>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
-        else if (kc > 1) ac_digit_task<2>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
-        else ac_digit_task<1>(g, lo, c0, kc, r0, s0, s1, sl, w, wq, E, finite, sh);
-    }
-    __syncthreads();
-    ac_publish<AC_THREADS>(ex.words, &sh.red[0][0], MEXK_M_MAX + 1, k, slices, g.scale);
-}
-
-// Column c of the basis into digits from the block's rows of the FP64 column
-// (the cycle's first column).
-__device__ __forceinline__ void ac_pack_column(const CycleArgs& g, int c, int r0, int rows, AcShared& sh, int& turn) {
-    const double* v = g.V + static_cast<size_t>(c) * g.ldv + r0;
-    unsigned long long* q = g.vq + static_cast<size_t>(c) * g.ldv + r0;
-    unsigned mag = 0u;
-    for (int r = threadIdx.x; r < rows; r += AC_THREADS) mag = max(mag, ac_mag(v[r]));
-    mag = ac_block_mag(mag, turn, sh);
-    const int E = ac_exponent(min(mag, AC_INF - 1u));  // non-finite columns are caught by w
-    for (int r = threadIdx.x; r < rows; r += AC_THREADS) q[r] = ac_pack(v[r], E);
-    if (threadIdx.x == 0) {
-        sh.vexp[c] = E;
-        g.vexp[c * CYCLE_MAX_BLOCKS + blockIdx.x] = E;
-    }
-    __syncthreads();
-}
-
 // The block's rows of w = A x in the row-pattern form, patterns of at most LM
 // entries: rounded products added in column order (spmv_pattern.cu). Gathered
 // entries times inv (scaled) or as they are.
@@ -884,12 +497,11 @@ __device__ __forceinline__ double ac_norm_sum(const AcExchange& ex, int np) {
     return s;
 }
 
-// CLUSTER: one cluster, the separate kernels' sums. DIGITS: the sweeps over
-// the digit columns. WSMEM: the block's rows of w fit in shared memory (else
-// they stay in x). NARROW: a window of at most two columns. VSMEM: the block's
-// rows of the basis too (they are read four times a step, and from L2 each
-// time costs a round trip).
-template <bool CLUSTER, bool DIGITS, bool WSMEM, bool NARROW = false, bool VSMEM = false>
+// CLUSTER: one cluster, the separate kernels' sums. WSMEM: the block's rows of
+// w fit in shared memory (else they stay in x). NARROW: a window of at most
+// two columns. VSMEM: the block's rows of the basis too (they are read four
+// times a step, and from L2 each time costs a round trip).
+template <bool CLUSTER, bool WSMEM, bool NARROW = false, bool VSMEM = false>
 __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs g) {
     constexpr bool EXACT = CLUSTER;
     __shared__ AcShared sh;
@@ -906,14 +518,6 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
     unsigned target = 0;
     double inv = 1.0;
     double* const w = WSMEM ? ac_smem : g.x + r0;
-    unsigned long long* const wq = WSMEM ? reinterpret_cast<unsigned long long*>(ac_smem + g.rows) : g.wq + r0;
-    int turn = 0;
-    if (DIGITS) {
-        if (threadIdx.x < 3) sh.mag[threadIdx.x] = 0u;
-        for (int c = threadIdx.x; c <= g.j0; c += AC_THREADS) sh.vexp[c] = g.vexp[c * CYCLE_MAX_BLOCKS + blockIdx.x];
-        __syncthreads();
-        if (g.j0 == 0) ac_pack_column(g, 0, r0, rows, sh, turn);
-    }
     // the exchanges of a step: first dots, second dots, norm; a grid's words
     // alternate by step parity, so that one set is cleared while the other is
     // in use
@@ -955,17 +559,9 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         };
         constexpr bool narrow = NARROW;
         double sum[2];
-        unsigned mag = 0u;
         if (narrow) {
             ac_narrow_pass<false, AC_PASS_DOTS>(V, ldv, k, r0, n_rows, nullptr, w, sum);
             ac_narrow_publish(g, k, sum, ex[0], sh);
-        } else if (DIGITS) {
-            for (int r = 2 * static_cast<int>(threadIdx.x); r < rows; r += 2 * AC_THREADS) {
-                const double2 x = *reinterpret_cast<const double2*>(w + r);
-                mag = max(mag, max(ac_mag(x.x), ac_mag(x.y)));
-            }
-            mag = ac_block_mag(mag, turn, sh);
-            ac_dots_digits(g, lo, k, r0, nsub, w, mag, wq, ex[0], sh);
         } else {
             dots(ex[0]);
         }
@@ -979,24 +575,17 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         if (narrow) {
             if (g.reortho) ac_narrow_pass<true, AC_PASS_DOTS>(V, ldv, k, r0, n_rows, sh.h1, w, sum);
             else ac_narrow_pass<true, AC_PASS_NORM>(V, ldv, k, r0, n_rows, sh.h1, w, sum);
-        } else if (DIGITS) {
-            ac_coefficients(lo, k, sh.h1, sh);
-            mag = ac_block_mag(ac_update_digits(g, lo, k, r0, n_rows, w, sh.h1, sh), turn, sh);
         } else {
             ac_update(Vb, ldb, k, n_rows, sh.h1, w);
             __syncthreads();
         }
         if (g.reortho) {
             if (narrow) ac_narrow_publish(g, k, sum, ex[1], sh);
-            else if (DIGITS) ac_dots_digits(g, lo, k, r0, nsub, w, mag, wq, ex[1], sh);
             else dots(ex[1]);
             if (!ac_meet<CLUSTER>(g.bar, target, &st->status, &sh.ok)) return;
             ac_sums<EXACT>(ex[1], k, np, g.scale, sh.h, sh);
             if (narrow) {
                 ac_narrow_pass<true, AC_PASS_NORM>(V, ldv, k, r0, n_rows, sh.h, w, sum);
-            } else if (DIGITS) {
-                ac_coefficients(lo, k, sh.h, sh);
-                mag = ac_block_mag(ac_update_digits(g, lo, k, r0, n_rows, w, sh.h, sh), turn, sh);
             } else {
                 ac_update(Vb, ldb, k, n_rows, sh.h, w);
             }
@@ -1029,20 +618,7 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         if (!sh.ok) break;  // the same sums in every block
         inv = sh.inv;
         double* q = g.V + static_cast<size_t>(j + 1) * ldv + r0;
-        if (DIGITS) {
-            // |w| < 2^a, 1/|w| < 2^b: every entry of the new column below 2^(a+b)
-            const int E = ac_exponent(min(mag, AC_INF - 1u)) + ac_exponent(ac_mag(inv));
-            unsigned long long* vq = g.vq + static_cast<size_t>(j + 1) * ldv + r0;
-            for (int r = threadIdx.x; r < n_rows; r += AC_THREADS) {
-                const double v = w[r] * inv;
-                __stcg(q + r, v);
-                __stcg(vq + r, ac_pack(v, E));
-            }
-            if (threadIdx.x == 0) {
-                sh.vexp[j + 1] = E;
-                g.vexp[(j + 1) * CYCLE_MAX_BLOCKS + blockIdx.x] = E;
-            }
-        } else if (VSMEM && j + 1 < g.j1) {
+        if (VSMEM && j + 1 < g.j1) {
             double* const vq = vs + (j + 1) * rows;
             for (int r = threadIdx.x; r < rows; r += AC_THREADS) {
                 const double v = w[r] * inv;
@@ -1084,16 +660,6 @@ constexpr int AC_SMEM_TOTAL = 227 * 1024 - static_cast<int>(sizeof(AcShared)) - 
 
 bool arnoldi_cycle_fits(int n) { return n <= CYCLE_ROWS_MAX; }
 
-// Digits pay from about 20,000 entries per block and sweep. FP64 sweeps against
-// them, by rows x allocated columns: 8,000 x 100 19.4 / 19.7 ms, 50,000 x 30
-// 1008 / 1032 us, 100,000 x 30 1365 / 1349 us, 50,021 x 100 32.7 / 29.7 ms,
-// 604,000 x 30 16.3 / 14.4 ms, 4,194,304 x 30 247 / 209 ms. The allocation
-// decides (not the step), so that a solve's sums do not depend on the ones
-// before it. A window of up to four columns has next to no sweeps.
-bool arnoldi_cycle_digits(int n, int m_alloc, int window) {
-    return n > EXACT_ROWS && static_cast<long long>(n) * m_alloc >= 3000000 && (window == 0 || window > 4);
-}
-
 // Measured on random rows (degree 10, m = 30, one cycle): own product against
 // the context's SpMV and a launch per step, 661 / 871 us at 5,000 rows, 997 /
 // 1108 at 50,000, 1367 / 1382 at 100,000, 1971 / 1957 at 200,000 (2.2 million
@@ -1109,19 +675,17 @@ bool arnoldi_cycle_product(int n, long long nnz, int max_row, bool pattern) {
 int arnoldi_cycle_prepare() {
     const int cl = static_cast<int>(sizeof(double)) * (EXACT_ROWS / AC_CLUSTER + (2 * MEXK_M_MAX + 1) * AC_PS);
     const int ws = static_cast<int>(sizeof(double)) * AC_SMEM_DOUBLES;
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cl));
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true>,
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, cl));
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, true>,
                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true, false, true>,
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, true, false, true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM_TOTAL));
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, false, true, false, true>,
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<true, true, false, true>,
                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, false, true, false, true>,
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, true, false, true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, AC_SMEM_TOTAL));
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
+    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
     MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
-    MEXK_CK(cudaFuncSetAttribute(arnoldi_cycle_kernel<false, false, true, true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, ws));
     return MEXK_OK;
 }
 
@@ -1150,20 +714,19 @@ int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(AC_THREADS);
-    const bool digits = !cluster && a.vq != nullptr;
     // Three passes against five sweeps, heat grids, window 2, one solve: 200^2 (320 rows a block) 2911 / 2890 us,
     // 300^2 3804 / 3302, 777^2 7271 / 6787, 1500^2 18442 / 16838; below 256 rows a block the sweeps share a column's
     // few rows out better (131^2 2695 / 2763).
-    const bool narrow = !cluster && !digits && a.window > 0 && a.window <= 2 && a.rows >= 256;
-    const bool wsmem = a.rows * (digits ? 2 : 1) <= AC_SMEM_DOUBLES;
+    const bool narrow = !cluster && a.window > 0 && a.window <= 2 && a.rows >= 256;
+    const bool wsmem = a.rows <= AC_SMEM_DOUBLES;
     if (!wsmem) a.scale_gather = 0;  // x holds w
-    cfg.dynamicSmemBytes = sizeof(double) * ((wsmem ? static_cast<size_t>(a.rows) * (digits ? 2 : 1) : 0) +
+    cfg.dynamicSmemBytes = sizeof(double) * ((wsmem ? static_cast<size_t>(a.rows) : 0) +
                                              (cluster ? (2 * static_cast<size_t>(a.m) + 1) * AC_PS : 0));
     // the basis on chip as well, where all m columns fit and one launch runs all steps. From L2 / on chip, one
     // solve: random 1,500 rows 556 / 528 us, 20,000 753 / 727, 80,000 1222 / 1197; 8,000 rows, 100 columns 18.9 /
     // 17.2 ms; heat 48^2 2854 / 2700 us, 300^2 5226 / 4997.
     const size_t vbytes = sizeof(double) * static_cast<size_t>(a.rows) * a.m;
-    const bool vsmem = a.product && wsmem && !digits && !narrow &&
+    const bool vsmem = a.product && wsmem && !narrow &&
                        cfg.dynamicSmemBytes + vbytes <= static_cast<size_t>(AC_SMEM_TOTAL);
     if (vsmem) cfg.dynamicSmemBytes += vbytes;
     cfg.stream = s;
@@ -1182,15 +745,13 @@ int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s) {
         cfg.numAttrs = 1;
     }
     cfg.attrs = attr;
-    const cudaError_t e = cluster && vsmem  ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true, false, true, false, true>, a)
-                          : cluster         ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true, false, true>, a)
-                          : vsmem           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, true, false, true>, a)
-                          : narrow && wsmem ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, true, true>, a)
-                          : narrow          ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, false, true>, a)
-                          : digits && wsmem ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true, true>, a)
-                          : digits          ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true, false>, a)
-                          : wsmem           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, true>, a)
-                                            : cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, false>, a);
+    const cudaError_t e = cluster && vsmem  ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true, true, false, true>, a)
+                          : cluster         ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<true, true>, a)
+                          : vsmem           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true, false, true>, a)
+                          : narrow && wsmem ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true, true>, a)
+                          : narrow          ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false, true>, a)
+                          : wsmem           ? cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, true>, a)
+                                            : cudaLaunchKernelEx(&cfg, arnoldi_cycle_kernel<false, false>, a);
     if (e != cudaSuccess) {
         set_cuda_error(e, "arnoldi_cycle_kernel", __FILE__, __LINE__);
         return MEXK_ERR_CUDA;

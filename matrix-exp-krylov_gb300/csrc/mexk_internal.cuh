@@ -443,9 +443,6 @@ struct CycleArgs {
     const uint8_t* pid;  // the row-pattern form, or null: the CSR arrays
     const RowPatterns* T;
     double* V;
-    unsigned long long* vq = nullptr;  // the basis in digits, as V (arnoldi_cycle_digits), or null
-    int* vexp = nullptr;               // its exponents, column c's at c * CYCLE_MAX_BLOCKS
-    unsigned long long* wq = nullptr;  // ldv words: w in digits, where it does not fit on chip
     double* x;
     double* H;
     DevState* st;
@@ -456,8 +453,6 @@ struct CycleArgs {
 // sum of |values|, and the entries of the longest row.
 int launch_row_bounds(int n, const int* row_ptr, const double* values, unsigned long long* out, cudaStream_t s);
 bool arnoldi_cycle_fits(int n);
-// Whether a basis runs its sweeps on digit columns (vq, vexp, wq).
-bool arnoldi_cycle_digits(int n, int m_alloc, int window);
 // Whether the launch also takes the products (else one launch per step after
 // the context's SpMV).
 bool arnoldi_cycle_product(int n, long long nnz, int max_row, bool pattern);

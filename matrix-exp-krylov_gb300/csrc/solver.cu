@@ -23,7 +23,6 @@
 //   basis V    column-major, leading dimension ldv = n rounded up to 64,
 //              m_alloc+1 columns, f64 (+ f32 basis for the mixed form, whose
 //              columns carry f64 scales, with the Gram matrix, in GramState)
-//              wide FP64 bases also in 61-bit digits (d_vq) with their exponents
 //   w, y       work vector (basis precision) and result (f64)
 //   H          f64 (m_alloc+1) x m_alloc column-major; h1, h2, coef f64
 //   partials   f64[4096 x RED_STRIDE] grid-reduction scratch + counter
@@ -114,9 +113,6 @@ struct mexk_context_s {
     float pat_val[PAT_LEN] = {};
     double* d_V = nullptr;
     float* d_V32 = nullptr;
-    unsigned long long* d_vq = nullptr;  // the FP64 basis in digits (arnoldi_cycle.cu), and its exponents
-    int* d_vexp = nullptr;
-    bool no_digits = false;  // no memory for them: the FP64 sweeps stay
     double* d_w = nullptr;
     float* d_w32 = nullptr;
     double* d_y = nullptr;
@@ -278,28 +274,6 @@ int ensure_mixed(mexk_context_t ctx) {
     ctx->spmv_form32 = ctx->d_pat ? MEXK_SPMV_PATTERN : ctx->spmv_narrow ? MEXK_SPMV_STAGED : MEXK_SPMV_DIRECT;
     MEXK_CK(cudaStreamSynchronize(ctx->stream));
     return MEXK_OK;
-}
-
-// The digit copy of an FP64 basis, where its sweeps use one: allocated before
-// any capture by the first solve that does, and done without when it does not
-// fit (those sweeps then run in FP64).
-void ensure_digits(mexk_context_t ctx, int window) {
-    if (ctx->d_vq || ctx->no_digits || ctx->cycle_scale == INT_MAX || !arnoldi_cycle_fits(ctx->n) ||
-        !arnoldi_cycle_digits(ctx->n, ctx->m_alloc, window))
-        return;
-    const size_t count = static_cast<size_t>(ctx->ldv) * (ctx->m_alloc + 2);  // the columns, then w's digits
-    const size_t nexp = static_cast<size_t>(ctx->m_alloc + 1) * CYCLE_MAX_BLOCKS;
-    if (cudaMalloc(reinterpret_cast<void**>(&ctx->d_vq), sizeof(unsigned long long) * count) != cudaSuccess ||
-        cudaMalloc(reinterpret_cast<void**>(&ctx->d_vexp), sizeof(int) * nexp) != cudaSuccess ||
-        // rows n..ldv-1 stay zero; done before a solve on whichever stream
-        cudaMemsetAsync(ctx->d_vq, 0, sizeof(unsigned long long) * count, ctx->stream) != cudaSuccess ||
-        cudaMemsetAsync(ctx->d_vexp, 0, sizeof(int) * nexp, ctx->stream) != cudaSuccess ||
-        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-        (void)cudaGetLastError();
-        dfree(ctx->d_vq);
-        dfree(ctx->d_vexp);
-        ctx->no_digits = true;
-    }
 }
 
 GsArgs gs_args(mexk_context_t ctx, int j, int reortho, bool fp32) {
@@ -524,11 +498,6 @@ int enqueue_arnoldi_cycle(mexk_context_t ctx, int m, int reortho, int window, cu
     a.pid = ctx->spmv_form64 == MEXK_SPMV_PATTERN ? ctx->d_pid : nullptr;
     a.T = ctx->d_pat;
     a.V = ctx->d_V;
-    if (ctx->d_vq && arnoldi_cycle_digits(ctx->n, ctx->m_alloc, window)) {
-        a.vq = ctx->d_vq;
-        a.vexp = ctx->d_vexp;
-        a.wq = ctx->d_vq + static_cast<size_t>(ctx->ldv) * (ctx->m_alloc + 1);
-    }
     a.x = ctx->d_w;
     a.H = ctx->d_H;
     a.st = ctx->d_state;
@@ -753,7 +722,6 @@ int solve(mexk_context_t ctx, const mexk_params_t* p, const double* v_dev, doubl
     int rc = check_params(ctx, p);
     if (rc) return rc;
     if (p->precision == MEXK_PREC_MIXED && (rc = ensure_mixed(ctx))) return rc;
-    if (p->precision == MEXK_PREC_FP64) ensure_digits(ctx, p->ortho_window);
     if (s == nullptr) s = ctx->stream;
     ctx->last_window = p->ortho_window;
     ctx->last_controller = p->controller;
@@ -1085,8 +1053,6 @@ int mexk_context_destroy(mexk_context_t ctx) {
     dfree(ctx->d_pid);
     dfree(ctx->d_V);
     dfree(ctx->d_V32);
-    dfree(ctx->d_vq);
-    dfree(ctx->d_vexp);
     dfree(ctx->d_w);
     dfree(ctx->d_w32);
     dfree(ctx->d_y);
