@@ -108,7 +108,9 @@ struct AcShared {
     double red[AC_NW][MEXK_M_MAX + 1];  // row slices' dots, then the partial sums' slices
     double prod[AC_TILE];
     double inv;
-    int ok, nlong;
+    int ok;   // the meetings' (cycle.cuh)
+    int bad;  // the step's breakdown: a word of its own, no barrier follows the last read of ok
+    int nlong;
     int rows_long[AC_THREADS];
 };
 
@@ -604,7 +606,7 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         if (threadIdx.x == 0) {
             const double beta = sqrt(w2);
             const bool bad = beta < 1e-14 || isnan(beta) || isinf(beta);
-            sh.ok = bad ? 0 : 1;
+            sh.bad = bad ? 1 : 0;
             if (!bad) sh.inv = 1.0 / beta;
             if (lead) {
                 g.H[(j + 1) + j * ldh] = bad ? 0.0 : beta;
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
             }
         }
         __syncthreads();
-        if (!sh.ok) break;  // the same sums in every block
+        if (sh.bad) break;  // the same sums in every block
         inv = sh.inv;
         double* q = g.V + static_cast<size_t>(j + 1) * ldv + r0;
         if (VSMEM && j + 1 < g.j1) {
