@@ -443,6 +443,19 @@ int mexk_context_set_spmv_form(mexk_context_t ctx, int precision, int form);
 int mexk_context_get_lanczos_form(mexk_context_t ctx, int* form);
 int mexk_context_set_lanczos_form(mexk_context_t ctx, int form);
 
+/* How a solve's bases run: MEXK_BASIS_ONE_LAUNCH (the default) in one launch
+ * where that is implemented and faster, as a thread-block cluster of 16 (up to
+ * some thousand rows) or a cooperative grid of a block per SM;
+ * MEXK_BASIS_SEPARATE as separate kernels per step. A cooperative grid starts
+ * when every SM has room for a block of it: a solve that has to run beside
+ * another kernel which holds SMs until the solve is done needs the separate
+ * form. Where such a launch is refused (a process that was given part of the
+ * SMs) a solve takes the separate kernels by itself. The two forms agree to
+ * rounding. No reference counterpart. */
+#define MEXK_BASIS_ONE_LAUNCH 0
+#define MEXK_BASIS_SEPARATE 1
+int mexk_context_set_basis_form(mexk_context_t ctx, int form);
+
 /* Kernels a solve with this precision and ortho_window launches for a basis of
  * m columns: 1 where one launch runs all its steps (and, but for FP64 matrices
  * of long or very many rows, their products), else per step the SpMV and its
@@ -462,6 +475,11 @@ int mexk_context_basis_launches(mexk_context_t ctx, int precision, int m, int or
  * result of a solve that uses none of them. No reference counterpart (the
  * reference has no bounded device waits). */
 int mexk_test_force_wait_timeout(int device, int enable);
+
+/* enable != 0: the context's launches of a basis in one launch are refused
+ * before they reach the device, as a grid that does not fit is; its solves
+ * take the separate kernels. For failure-path tests only. */
+int mexk_test_refuse_one_launch(mexk_context_t ctx, int enable);
 
 #ifdef __cplusplus
 }

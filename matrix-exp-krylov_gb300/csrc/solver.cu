@@ -73,6 +73,7 @@ using namespace mexk;
 
 struct GraphEntry {
     int m, prec, reortho, ctrl, window;
+    bool separate;  // without the one-launch bases
     cudaGraphExec_t exec;
 };
 
@@ -134,6 +135,9 @@ struct mexk_context_s {
     mexk_step_t* d_log = nullptr;
     bool uploaded = false;
     bool use_graph = true;
+    int basis_form = MEXK_BASIS_ONE_LAUNCH;
+    bool basis_refused = false;  // the running solve: a basis in one launch could not be placed
+    bool test_refuse = false;    // mexk_test_refuse_one_launch
     std::vector<GraphEntry> graphs;
 };
 
@@ -477,10 +481,13 @@ int enqueue_lanczos_cycle(mexk_context_t ctx, int m, int reortho, cudaStream_t s
     return launch_lanczos_cycle(a, s);
 }
 
+// Whether bases run as their separate kernels whatever else holds.
+bool separate_basis(mexk_context_t ctx) { return ctx->basis_form == MEXK_BASIS_SEPARATE || ctx->basis_refused; }
+
 // Whether an FP64 basis is built by arnoldi_cycle.cu: in one launch with its
 // products, or in one launch per step after the SpMV.
 bool use_arnoldi_cycle(mexk_context_t ctx) {
-    return ctx->cycle_scale != INT_MAX && arnoldi_cycle_fits(ctx->n);
+    return !separate_basis(ctx) && ctx->cycle_scale != INT_MAX && arnoldi_cycle_fits(ctx->n);
 }
 
 int enqueue_arnoldi_cycle(mexk_context_t ctx, int m, int reortho, int window, cudaStream_t s) {
@@ -527,7 +534,7 @@ bool use_stencil_cycle(mexk_context_t ctx, int m, int window) {
            stencil_cycle_fits(ctx->n, m, ctx->pat_major_len, ctx->pat_reach);
 }
 bool use_gram_cycle(mexk_context_t ctx, int m, int window) {
-    if (ctx->cycle_scale == INT_MAX || use_lanczos_cycle(ctx, m, true, window)) return false;
+    if (separate_basis(ctx) || ctx->cycle_scale == INT_MAX || use_lanczos_cycle(ctx, m, true, window)) return false;
     return use_stencil_cycle(ctx, m, window) ||
            gram_cycle_fits(ctx->n, ctx->nnz, m, ctx->max_row, ctx->spmv_form32 == MEXK_SPMV_PATTERN, window);
 }
@@ -589,6 +596,10 @@ int enqueue_basis(mexk_context_t ctx, int m, int reortho, int window, bool fp32,
     // a window's FP64 steps leave H(0:lo-1, j) alone: the cycle starts from zero
     if (!fp32 && window > 0)
         MEXK_CK(cudaMemsetAsync(ctx->d_H, 0, sizeof(double) * static_cast<size_t>(ctx->ldh) * m, s));
+    if (ctx->test_refuse && (fp32 ? use_gram_cycle(ctx, m, window) : use_arnoldi_cycle(ctx))) {
+        set_cuda_error(cudaErrorCooperativeLaunchTooLarge, "one-launch basis (testing hook)", __FILE__, __LINE__);
+        return MEXK_ERR_CUDA;
+    }
     if (!fp32 && use_arnoldi_cycle(ctx)) return enqueue_arnoldi_cycle(ctx, m, reortho, window, s);
     if (fp32 && use_gram_cycle(ctx, m, window))
         return use_stencil_cycle(ctx, m, window) ? enqueue_stencil_cycle(ctx, m, reortho, s)
@@ -625,8 +636,10 @@ int enqueue_cycle_any(mexk_context_t ctx, int m, int prec, int reortho, int ctrl
 }
 
 int get_graph(mexk_context_t ctx, int m, int prec, int reortho, int ctrl, int window, cudaGraphExec_t* out) {
+    const bool separate = separate_basis(ctx);
     for (auto& g : ctx->graphs) {
-        if (g.m == m && g.prec == prec && g.reortho == reortho && g.ctrl == ctrl && g.window == window) {
+        if (g.m == m && g.prec == prec && g.reortho == reortho && g.ctrl == ctrl && g.window == window &&
+            g.separate == separate) {
             *out = g.exec;
             return MEXK_OK;
         }
@@ -650,7 +663,7 @@ int get_graph(mexk_context_t ctx, int m, int prec, int reortho, int ctrl, int wi
         set_cuda_error(e, "cudaGraphInstantiate", __FILE__, __LINE__);
         return MEXK_ERR_CUDA;
     }
-    ctx->graphs.push_back({m, prec, reortho, ctrl, window, exec});
+    ctx->graphs.push_back({m, prec, reortho, ctrl, window, separate, exec});
     *out = exec;
     return MEXK_OK;
 }
@@ -725,6 +738,7 @@ int solve(mexk_context_t ctx, const mexk_params_t* p, const double* v_dev, doubl
     if (s == nullptr) s = ctx->stream;
     ctx->last_window = p->ortho_window;
     ctx->last_controller = p->controller;
+    ctx->basis_refused = false;
     init_state(ctx->h_state, p, LOG_CAP);
     MEXK_CK(cudaMemcpyAsync(ctx->d_state, ctx->h_state, sizeof(DevState), cudaMemcpyHostToDevice, s));
     MEXK_CK(cudaMemsetAsync(ctx->d_bar, 0, BAR_BYTES, s));
@@ -753,16 +767,27 @@ int solve(mexk_context_t ctx, const mexk_params_t* p, const double* v_dev, doubl
         int m_cycle = p->m;
         for (long long cyc = 0; cyc < max_cycles; ++cyc) {
             NvtxRange cycle_range("arnoldi_step_attempt");
-            if (ctx->use_graph) {
+            auto cycle = [&]() -> int {
+                if (!ctx->use_graph)
+                    return enqueue_cycle_any(ctx, m_cycle, p->precision, reortho, p->controller, p->ortho_window, s);
                 // Graphs are captured on the context stream and launched on `s`.
                 cudaGraphExec_t exec = nullptr;
-                if ((rc = get_graph(ctx, m_cycle, p->precision, reortho, p->controller, p->ortho_window, &exec)))
-                    return rc;
+                const int r = get_graph(ctx, m_cycle, p->precision, reortho, p->controller, p->ortho_window, &exec);
+                if (r) return r;
                 MEXK_CK(cudaGraphLaunch(exec, s));
-            } else if ((rc = enqueue_cycle_any(ctx, m_cycle, p->precision, reortho, p->controller, p->ortho_window,
-                                               s))) {
-                return rc;
+                return MEXK_OK;
+            };
+            rc = cycle();
+            const bool one_launch = p->precision == MEXK_PREC_MIXED ? use_gram_cycle(ctx, m_cycle, p->ortho_window)
+                                                                    : use_arnoldi_cycle(ctx);
+            if (rc == MEXK_ERR_CUDA && one_launch) {
+                // a cluster or a grid that has to be resident as a whole was refused (a process or stream with part
+                // of the SMs): the cycle has changed nothing that its separate kernels read
+                (void)cudaGetLastError();
+                ctx->basis_refused = true;
+                rc = cycle();
             }
+            if (rc) return rc;
             MEXK_CK(cudaMemcpyAsync(ctx->h_state, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s));
             MEXK_CK(cudaStreamSynchronize(s));
             if (ctx->h_state->done) break;
@@ -1320,6 +1345,20 @@ int mexk_context_basis_launches(mexk_context_t ctx, int precision, int m, int or
     for (int j = 0; j < m; ++j)
         k += ctx->spmv_form32 != MEXK_SPMV_DIRECT && fused_step(j, ortho_window) ? 2 : 3;
     *launches = k;
+    return MEXK_OK;
+}
+
+int mexk_context_set_basis_form(mexk_context_t ctx, int form) {
+    if (!ctx || !ctx->uploaded) return MEXK_ERR_INVALID;
+    if (form != MEXK_BASIS_ONE_LAUNCH && form != MEXK_BASIS_SEPARATE) return MEXK_ERR_INVALID;
+    ctx->basis_form = form;
+    return MEXK_OK;
+}
+
+int mexk_test_refuse_one_launch(mexk_context_t ctx, int enable) {
+    if (!ctx || !ctx->uploaded) return MEXK_ERR_INVALID;
+    ctx->test_refuse = enable != 0;
+    invalidate_graphs(ctx);
     return MEXK_OK;
 }
 

@@ -139,6 +139,8 @@ _PROTOS = {
     "mexk_controller_predict": ([_VP, _VP, C.c_int, C.c_int, C.c_double, C.c_double, C.c_double, C.c_double,
                                  C.c_double, _VP, _VP], C.c_int),
     "mexk_test_force_wait_timeout": ([C.c_int, C.c_int], C.c_int),
+    "mexk_context_set_basis_form": ([_VP, C.c_int], C.c_int),
+    "mexk_test_refuse_one_launch": ([_VP, C.c_int], C.c_int),
     "mexk_context_basis_launches": ([_VP, C.c_int, C.c_int, C.c_int, _IP], C.c_int),
     "mexk_context_get_lanczos_form": ([_VP, _IP], C.c_int),
     "mexk_context_set_lanczos_form": ([_VP, C.c_int], C.c_int),

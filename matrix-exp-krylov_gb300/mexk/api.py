@@ -220,6 +220,14 @@ class Context:
         check(lib().mexk_context_set_lanczos_form(self._h, self.LANCZOS_FORMS.index(form)),
               "mexk_context_set_lanczos_form")
 
+    BASIS_FORMS = ("one_launch", "separate")
+
+    def set_basis_form(self, form: str) -> None:
+        """"one_launch" (the default: all steps of a basis in one launch where
+        that is faster, a cooperative grid among them, which needs every SM) or
+        "separate" (kernels per step, which run beside other work)."""
+        check(lib().mexk_context_set_basis_form(self._h, self.BASIS_FORMS.index(form)), "mexk_context_set_basis_form")
+
     def basis_launches(self, m: int, precision="fp64", window: int = 0) -> int:
         """Kernels a solve launches for a basis of m columns (1: all steps in one launch)."""
         k = C.c_int(0)
