@@ -358,7 +358,9 @@ int mexk_batch_run(mexk_batch_t b);
 /* Y: rows x nrhs row-major; results: nrhs entries (may be null). */
 int mexk_batch_result(mexk_batch_t b, int problem, double* Y, mexk_result_t* results);
 /* The same with Y nrhs x rows, row-major (one right-hand side after another):
- * transposed on the device and copied straight into Y. */
+ * transposed on the device and copied straight into Y, through a device
+ * buffer of Y's size that the batch keeps; on the host where there is no
+ * memory for it. */
 int mexk_batch_result_columns(mexk_batch_t b, int problem, double* Y, mexk_result_t* results);
 int mexk_batch_info(mexk_batch_t b, mexk_batch_info_t* info);
 /* Times `iters` launches of one per-step kernel of the first wave at step j
@@ -480,6 +482,10 @@ int mexk_test_force_wait_timeout(int device, int enable);
  * before they reach the device, as a grid that does not fit is; its solves
  * take the separate kernels. For failure-path tests only. */
 int mexk_test_refuse_one_launch(mexk_context_t ctx, int enable);
+
+/* enable != 0: the batch gives back mexk_batch_result_columns' device buffer
+ * and finds no memory for another. For failure-path tests only. */
+int mexk_test_refuse_columns(mexk_batch_t b, int enable);
 
 #ifdef __cplusplus
 }

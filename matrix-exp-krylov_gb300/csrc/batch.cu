@@ -113,6 +113,7 @@ struct mexk_batch_s {
     double* d_npart = nullptr;
     double* d_cols = nullptr;  // a problem's results transposed (mexk_batch_result_columns), once asked for
     size_t cols_cap = 0;
+    bool test_refuse_cols = false;  // mexk_test_refuse_columns
     std::mutex cols_mutex;  // results of one batch may be fetched by several threads
     int tiles_total_cap = 0;
     std::vector<Wave> waves;
@@ -701,6 +702,17 @@ int mexk_batch_result(mexk_batch_t b, int problem, double* Y, mexk_result_t* res
     return MEXK_OK;
 }
 
+int mexk_test_refuse_columns(mexk_batch_t b, int enable) {
+    if (!b) return MEXK_ERR_INVALID;
+    const std::lock_guard<std::mutex> lock(b->cols_mutex);
+    b->test_refuse_cols = enable != 0;
+    if (b->test_refuse_cols) {
+        dfree(b->d_cols);
+        b->cols_cap = 0;
+    }
+    return MEXK_OK;
+}
+
 int mexk_batch_result_columns(mexk_batch_t b, int problem, double* Y, mexk_result_t* results) {
     if (!b || !b->uploaded || problem < 0 || problem >= P_of(b) || !Y) return MEXK_ERR_INVALID;
     if (!b->have_final) return MEXK_ERR_NOT_READY;
@@ -712,12 +724,21 @@ int mexk_batch_result_columns(mexk_batch_t b, int problem, double* Y, mexk_resul
     if (count > b->cols_cap) {
         dfree(b->d_cols);
         b->cols_cap = 0;
-        if ((rc = dalloc(&b->d_cols, count))) return rc;
-        b->cols_cap = count;
+        if (!b->test_refuse_cols && dalloc(&b->d_cols, count) == MEXK_OK) b->cols_cap = count;
+        else (void)cudaGetLastError();
     }
-    if ((rc = launch_columns(b->d_Y + b->prow0[problem] * BR, q.rows, q.nrhs, b->d_cols, b->stream))) return rc;
-    MEXK_CK(cudaMemcpyAsync(Y, b->d_cols, sizeof(double) * count, cudaMemcpyDeviceToHost, b->stream));
-    MEXK_CK(cudaStreamSynchronize(b->stream));
+    const double* const src = b->d_Y + b->prow0[problem] * BR;
+    if (b->cols_cap >= count) {
+        if ((rc = launch_columns(src, q.rows, q.nrhs, b->d_cols, b->stream))) return rc;
+        MEXK_CK(cudaMemcpyAsync(Y, b->d_cols, sizeof(double) * count, cudaMemcpyDeviceToHost, b->stream));
+        MEXK_CK(cudaStreamSynchronize(b->stream));
+    } else {  // no room for it on the device: transposed here
+        std::vector<double> tmp(static_cast<size_t>(q.rows) * BR);
+        MEXK_CK(cudaMemcpy(tmp.data(), src, sizeof(double) * tmp.size(), cudaMemcpyDeviceToHost));
+        for (int r = 0; r < q.nrhs; ++r)
+            for (int i = 0; i < q.rows; ++i)
+                Y[static_cast<size_t>(r) * q.rows + i] = tmp[static_cast<size_t>(i) * BR + r];
+    }
     if (results) fill_results(b, problem, results);
     return MEXK_OK;
 }

@@ -141,6 +141,7 @@ _PROTOS = {
     "mexk_test_force_wait_timeout": ([C.c_int, C.c_int], C.c_int),
     "mexk_context_set_basis_form": ([_VP, C.c_int], C.c_int),
     "mexk_test_refuse_one_launch": ([_VP, C.c_int], C.c_int),
+    "mexk_test_refuse_columns": ([_VP, C.c_int], C.c_int),
     "mexk_context_basis_launches": ([_VP, C.c_int, C.c_int, C.c_int, _IP], C.c_int),
     "mexk_context_get_lanczos_form": ([_VP, _IP], C.c_int),
     "mexk_context_set_lanczos_form": ([_VP, C.c_int], C.c_int),
