@@ -468,11 +468,11 @@ int mexk_context_basis_launches(mexk_context_t ctx, int precision, int m, int or
 /* enable != 0: from now on, thread block 0 of the staged CSR SpMV also waits
  * (1 ms limit) on a barrier that nothing arrives at, so its bounded wait runs
  * out: it drains its bulk copies in flight and sets the timeout status bit;
- * thread block 0 of an FP64 basis built by a cooperative grid (more than 4096
- * rows) waits 1 ms for an arrival that never comes, raises the status bit and
- * the abort word, and the others leave; and thread block 0 of the fused
- * Lanczos cycle leaves before its first grid barrier, so the other blocks'
- * bounded waits (1 s) run out. Each way the solve returns MEXK_ERR_DEVICE and the context stays usable. enable = 0
+ * thread block 0 of a basis built by a cooperative grid leaves before its
+ * first meeting, so the other blocks' bounded waits (1 ms under the hook, 1 s
+ * otherwise) run out; and thread block 0 of the fused Lanczos cycle leaves
+ * before its first grid barrier, with the same end after 1 s. Each way the
+ * solve returns MEXK_ERR_DEVICE and the context stays usable. enable = 0
  * restores normal operation. For failure-path tests only: it changes no
  * result of a solve that uses none of them. No reference counterpart (the
  * reference has no bounded device waits). */

@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(AC_THREADS, 1) arnoldi_cycle_kernel(CycleArgs 
         __syncthreads();
     }
     if (CLUSTER) cooperative_groups::this_cluster().sync();  // every block runs before another writes to its memory
-    if (!CLUSTER && lead && ac_test_dead_wait(&st->status, g.bar)) return;
+    if (!CLUSTER && lead && g_test_ac_dead_wait != 0) return;
     for (int j = g.j0; j < g.j1; ++j) {
         const int lo = g.window > 0 ? max(0, j + 1 - g.window) : 0;
         const int k = j + 1 - lo;

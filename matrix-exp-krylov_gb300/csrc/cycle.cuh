@@ -11,6 +11,12 @@ namespace {
 
 constexpr unsigned AC_FULL = 0xffffffffu;
 constexpr unsigned long long AC_WAIT_NS = 1000000000ull;
+constexpr unsigned long long AC_TEST_WAIT_NS = 1000000ull;  // the limit under the testing hook
+
+// Testing hook (mexk_test_force_wait_timeout): when set, block 0 of a grid
+// leaves before its first meeting, and the others' waits give up after
+// AC_TEST_WAIT_NS.
+__device__ int g_test_ac_dead_wait = 0;
 
 __device__ __forceinline__ unsigned long long ac_ns() {
     unsigned long long t;
@@ -53,7 +59,8 @@ __device__ __forceinline__ bool ac_wait(unsigned* bar, unsigned target, int* sta
                         ok = 0;
                         break;
                     }
-                    if (ac_ns() - t0 > AC_WAIT_NS) {
+                    const unsigned long long waited = ac_ns() - t0;
+                    if (waited > AC_WAIT_NS || (waited > AC_TEST_WAIT_NS && g_test_ac_dead_wait != 0)) {
                         atomicExch(&bar[1], 1u);
                         atomicOr(status, ST_TIMEOUT);
                         ok = 0;
@@ -72,22 +79,6 @@ template <bool CLUSTER>
 __device__ __forceinline__ bool ac_meet(unsigned* bar, unsigned& target, int* status, int* s_ok) {
     ac_arrive<CLUSTER>(bar, target);
     return ac_wait<CLUSTER>(bar, target, status, s_ok);
-}
-
-// Testing hook (mexk_test_force_wait_timeout): when set, block 0 of a grid
-// waits 1 ms for an arrival that never comes before its first meeting, then
-// raises the abort word and leaves.
-__device__ int g_test_ac_dead_wait = 0;
-__device__ __forceinline__ bool ac_test_dead_wait(int* status, unsigned* bar) {
-    if (g_test_ac_dead_wait == 0) return false;
-    if (threadIdx.x == 0) {
-        const unsigned long long t0 = ac_ns();
-        while (ac_ns() - t0 < 1000000ull) {
-        }
-        atomicOr(status, ST_TIMEOUT);
-        atomicExch(&bar[1], 1u);
-    }
-    return true;
 }
 
 // ---- exact sums over the blocks of a grid -----------------------------------

@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gram_cycle_kernel(GramCycleArgs
     if (tid == 0) sh.ip = gs->ip[0];
     if (CLUSTER) cooperative_groups::this_cluster().sync();  // every block runs before another writes to its memory
     else __syncthreads();
-    if (!CLUSTER && lead && ac_test_dead_wait(&st->status, g.bar)) return;
+    if (!CLUSTER && lead && g_test_ac_dead_wait != 0) return;
     {
         const int slices = gc_dots(B, 0, 0, own(0), 1, n4, fs + own(0), sh);
         __syncthreads();

@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) stencil_cycle_kernel(StencilArgs 
         if (warp == 0)
             asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh.tmem), "n"(SC_TMEM));
     };
-    if (lead && ac_test_dead_wait(&st->status, g.bar)) {
+    if (lead && g_test_ac_dead_wait != 0) {
         leave();
         return;
     }
