@@ -901,12 +901,12 @@ int context_csr_finish(mexk_context_t ctx, const int* row_ptr) {
     MEXK_CK(cudaMemset(ctx->d_counter, 0, sizeof(unsigned int) * 4));
     if ((rc = dalloc(&ctx->d_bar, BAR_BYTES / sizeof(unsigned int)))) return rc;
     MEXK_CK(cudaMemsetAsync(ctx->d_bar, 0, BAR_BYTES, ctx->stream));
-    // bounds of A's rows, read back with the pattern detection's flags (the
-    // words are cleared again before each solve)
+    // bounds of A's rows, read back with the pattern detection's flags
     unsigned long long* const d_bounds = reinterpret_cast<unsigned long long*>(ctx->d_bar + BAR_WORDS);
     if ((rc = launch_row_bounds(ctx->n, ctx->d_row_ptr, ctx->d_val, d_bounds, ctx->stream))) return rc;
     unsigned long long bounds[2] = {0, 0};
     MEXK_CK(cudaMemcpyAsync(bounds, d_bounds, sizeof(bounds), cudaMemcpyDeviceToHost, ctx->stream));
+    MEXK_CK(cudaMemsetAsync(ctx->d_bar, 0, BAR_BYTES, ctx->stream));
     if ((rc = dalloc(&ctx->d_state, 1))) return rc;
     if ((rc = dalloc(&ctx->d_log, LOG_CAP))) return rc;
     cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&ctx->h_state), sizeof(DevState));
@@ -1569,7 +1569,24 @@ int mexk_profile_kernel(mexk_context_t ctx, int kind, int precision, int j, int 
             set_cuda_error(ce, "profile setup", __FILE__, __LINE__);
             rc = MEXK_ERR_CUDA;
         }
+        // the meetings' words may be those of a solve whose wait gave up
+        if (rc == MEXK_OK && kind == MEXK_KERNEL_BASIS && (ce = cudaMemsetAsync(ctx->d_bar, 0, BAR_BYTES, s)) != cudaSuccess) {
+            set_cuda_error(ce, "profile setup", __FILE__, __LINE__);
+            rc = MEXK_ERR_CUDA;
+        }
         if (rc == MEXK_OK) rc = launch_one();
+        if (rc == MEXK_OK && kind == MEXK_KERNEL_BASIS) {
+            // after a breakdown (no start vector yet, say) the timed launches would return at once
+            ce = cudaMemcpyAsync(h_run, ctx->d_state, sizeof(DevState), cudaMemcpyDeviceToHost, s);
+            if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
+            if (ce != cudaSuccess) {
+                set_cuda_error(ce, "profile setup", __FILE__, __LINE__);
+                rc = MEXK_ERR_CUDA;
+            } else if (h_run->breakdown || (h_run->status & ST_TIMEOUT)) {
+                set_error_text("profile: the basis from the context's first column broke down");
+                rc = MEXK_ERR_DEVICE;
+            }
+        }
         if (rc == MEXK_OK) rc = timed(iters, &total);
     }
     cudaEventDestroy(e0);
