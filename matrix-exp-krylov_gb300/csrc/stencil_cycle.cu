@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) stencil_cycle_kernel(StencilArgs 
     auto wb = [&](int p) { return g.words + static_cast<size_t>(2 * p + 1) * CYCLE_EXCHANGE; };
     const auto scale_a = [&](int c) { return c == 0 ? g.scale + SC_MARGIN : 2 * (g.scale + SC_MARGIN); };
     const auto scale_b = [&](int c) { return c == 2 ? g.scale + SC_MARGIN : SC_MARGIN; };
-    if (warp == 0) {
+    if (warp == 0) {  // the only block on its SM (SC_SMEM_MIN): nobody it waits for waits for this
         const unsigned p = static_cast<unsigned>(__cvta_generic_to_shared(&sh.tmem));
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(p), "n"(SC_TMEM)
                      : "memory");
@@ -483,6 +483,12 @@ __global__ void __launch_bounds__(SC_BLOCK, 1) stencil_cycle_kernel(StencilArgs 
 }
 
 constexpr int SC_SMEM = 227 * 1024 - static_cast<int>(sizeof(ScShared)) - 64;
+// More than half an SM's shared memory, whatever a block needs: two blocks of
+// different grids on one SM would each wait, the one for tensor memory that
+// the other holds, the other at a meeting that the first one's grid delays. A
+// cooperative launch does not count tensor memory.
+constexpr int SC_SMEM_MIN = 116 * 1024;
+static_assert(2 * SC_SMEM_MIN > 228 * 1024, "one block an SM");
 
 int sc_rows(int n) {
     const int blocks = std::min(device_sm_count(), CYCLE_MAX_BLOCKS);
@@ -520,7 +526,7 @@ int launch_stencil_cycle(StencilArgs a, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((a.n + a.rows - 1) / a.rows);
     cfg.blockDim = dim3(SC_BLOCK);
-    cfg.dynamicSmemBytes = sc_bytes(a.rows, a.reach);
+    cfg.dynamicSmemBytes = std::max<size_t>(sc_bytes(a.rows, a.reach), SC_SMEM_MIN);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
