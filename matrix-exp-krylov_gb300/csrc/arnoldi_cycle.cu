@@ -660,7 +660,25 @@ int sm_total() { return std::min(device_sm_count(), CYCLE_MAX_BLOCKS); }
 // Dynamic shared memory beside the kernel's own.
 constexpr int AC_SMEM_TOTAL = 227 * 1024 - static_cast<int>(sizeof(AcShared)) - 64;
 
-bool arnoldi_cycle_fits(int n) { return n <= CYCLE_ROWS_MAX; }
+// Rows of a grid's blocks.
+static int grid_rows(int n) {
+    const int subs = (n + AC_SUB - 1) / AC_SUB;
+    return (subs + sm_total() - 1) / sm_total() * AC_SUB;
+}
+
+// Once w is no longer on chip (3.4 million rows), a window pays by how well it
+// fills the separate sweeps, which are 8, 16, 32 ... columns wide whatever of
+// them it has, where this kernel pays for the columns there are. One basis of
+// 40 columns on heat grids, separate / one launch (ms): 2048^2 window 4 16.2 /
+// 13.5, 5 16.2 / 16.0, 8 16.3 / 17.1, 9 23.4 / 19.4, 12 23.5 / 21.5, 16 23.4 /
+// 23.8, 20 29.0 / 27.2, 24 29.1 / 28.8; 3500^2 window 4 43.5 / 40.5, 5 43.6 /
+// 47.1, 8 43.9 / 49.4, 9 64.2 / 56.7, 12 64.3 / 62.2, 16 64.1 / 68.9, 24 80.5 /
+// 83.3. Without a window 2048^2 30 columns 21.8 / 20.8, 3500^2 60.4 / 60.3, 60
+// columns 227.8 / 193.4.
+bool arnoldi_cycle_fits(int n, int window) {
+    if (n > CYCLE_ROWS_MAX) return false;
+    return grid_rows(n) <= AC_SMEM_DOUBLES || window <= 4 || (window - 1) % 8 < 4;
+}
 
 // Measured on random rows (degree 10, m = 30, one cycle): own product against
 // the context's SpMV and a launch per step, 661 / 871 us at 5,000 rows, 997 /
@@ -700,16 +718,15 @@ int arnoldi_cycle_test_hook(int enable) {
 int launch_arnoldi_cycle(CycleArgs a, cudaStream_t s) {
     const bool cluster = a.n <= EXACT_ROWS;
     if (a.j0 < 0 || a.j1 > a.m || a.j0 >= a.j1 || (!a.product && a.j1 != a.j0 + 1)) return MEXK_ERR_INVALID;
-    const int subs = (a.n + AC_SUB - 1) / AC_SUB;
     int grid;
     if (cluster) {
+        const int subs = (a.n + AC_SUB - 1) / AC_SUB;
         grid = AC_CLUSTER;
         a.rows = (subs + grid - 1) / grid * AC_SUB;
         a.scale_gather = 1;
     } else {
-        const int per = (subs + sm_total() - 1) / sm_total();
-        a.rows = per * AC_SUB;
-        grid = (subs + per - 1) / per;
+        a.rows = grid_rows(a.n);
+        grid = (a.n + a.rows - 1) / a.rows;
         a.scale_gather = a.product && a.nnz * a.rows <= 6000ll * a.n ? 1 : 0;
     }
     if (!cluster && grid > CYCLE_MAX_BLOCKS) return MEXK_ERR_UNSUPPORTED;

@@ -452,7 +452,8 @@ struct CycleArgs {
 // out (device, zero before the call): the bits of a bound of the largest row
 // sum of |values|, and the entries of the longest row.
 int launch_row_bounds(int n, const int* row_ptr, const double* values, unsigned long long* out, cudaStream_t s);
-bool arnoldi_cycle_fits(int n);
+// Whether a basis with this window (0: none) runs in arnoldi_cycle.cu.
+bool arnoldi_cycle_fits(int n, int window);
 // Whether the launch also takes the products (else one launch per step after
 // the context's SpMV).
 bool arnoldi_cycle_product(int n, long long nnz, int max_row, bool pattern);

@@ -486,8 +486,8 @@ bool separate_basis(mexk_context_t ctx) { return ctx->basis_form == MEXK_BASIS_S
 
 // Whether an FP64 basis is built by arnoldi_cycle.cu: in one launch with its
 // products, or in one launch per step after the SpMV.
-bool use_arnoldi_cycle(mexk_context_t ctx) {
-    return !separate_basis(ctx) && ctx->cycle_scale != INT_MAX && arnoldi_cycle_fits(ctx->n);
+bool use_arnoldi_cycle(mexk_context_t ctx, int window) {
+    return !separate_basis(ctx) && ctx->cycle_scale != INT_MAX && arnoldi_cycle_fits(ctx->n, window);
 }
 
 int enqueue_arnoldi_cycle(mexk_context_t ctx, int m, int reortho, int window, cudaStream_t s) {
@@ -596,11 +596,11 @@ int enqueue_basis(mexk_context_t ctx, int m, int reortho, int window, bool fp32,
     // a window's FP64 steps leave H(0:lo-1, j) alone: the cycle starts from zero
     if (!fp32 && window > 0)
         MEXK_CK(cudaMemsetAsync(ctx->d_H, 0, sizeof(double) * static_cast<size_t>(ctx->ldh) * m, s));
-    if (ctx->test_refuse && (fp32 ? use_gram_cycle(ctx, m, window) : use_arnoldi_cycle(ctx))) {
+    if (ctx->test_refuse && (fp32 ? use_gram_cycle(ctx, m, window) : use_arnoldi_cycle(ctx, window))) {
         set_cuda_error(cudaErrorCooperativeLaunchTooLarge, "one-launch basis (testing hook)", __FILE__, __LINE__);
         return MEXK_ERR_CUDA;
     }
-    if (!fp32 && use_arnoldi_cycle(ctx)) return enqueue_arnoldi_cycle(ctx, m, reortho, window, s);
+    if (!fp32 && use_arnoldi_cycle(ctx, window)) return enqueue_arnoldi_cycle(ctx, m, reortho, window, s);
     if (fp32 && use_gram_cycle(ctx, m, window))
         return use_stencil_cycle(ctx, m, window) ? enqueue_stencil_cycle(ctx, m, reortho, s)
                                                  : enqueue_gram_cycle(ctx, m, reortho, window, s);
@@ -779,7 +779,7 @@ int solve(mexk_context_t ctx, const mexk_params_t* p, const double* v_dev, doubl
             };
             rc = cycle();
             const bool one_launch = p->precision == MEXK_PREC_MIXED ? use_gram_cycle(ctx, m_cycle, p->ortho_window)
-                                                                    : use_arnoldi_cycle(ctx);
+                                                                    : use_arnoldi_cycle(ctx, p->ortho_window);
             if (rc == MEXK_ERR_CUDA && one_launch) {
                 // a cluster or a grid that has to be resident as a whole was refused (a process or stream with part
                 // of the SMs): the cycle has changed nothing that its separate kernels read
@@ -1329,7 +1329,7 @@ int mexk_context_basis_launches(mexk_context_t ctx, int precision, int m, int or
     if (precision == MEXK_PREC_FP64) {
         const bool product = arnoldi_cycle_product(ctx->n, ctx->nnz, ctx->max_row, ctx->spmv_form64 == MEXK_SPMV_PATTERN);
         const int chunks = (m + GS_DOT_COLS - 1) / GS_DOT_COLS;  // of the separate sweeps' dots
-        *launches = use_arnoldi_cycle(ctx) ? (product ? 1 : 2 * m) : (chunks > 1 ? 7 : 5) * m;
+        *launches = use_arnoldi_cycle(ctx, ortho_window) ? (product ? 1 : 2 * m) : (chunks > 1 ? 7 : 5) * m;
         return MEXK_OK;
     }
     if ((rc = ensure_mixed(ctx))) return rc;
