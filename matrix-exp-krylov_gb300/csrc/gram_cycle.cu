@@ -744,10 +744,15 @@ GcShape gc_shape(int n, int m, bool cluster, bool csr) {
 // blocks waiting for one another (power law: 5,000 1608 / 1147, 20,000 3363 /
 // 2475, 50,000 3917 / 3730, 100,000 4857 / 5929). A window of two or so columns
 // has next to no sweeps (heat 400^2 1445 / 1244, 600^2 1991 / 1907, 777^2
-// 2169 / 2224).
+// 2169 / 2224). A few columns are on chip at any size, but above 1.8 million
+// rows a block's own rows outlast the launches saved (5 columns: 1300^2 276 /
+// 272, 1400^2 283 / 297, 1500^2 285 / 331; 8: 377 / 371, 384 / 404, 390 / 433),
+// and up to three are over before they have paid for the start (2: 600^2 254 /
+// 262, 1000^2 270 / 284; 3: 281 / 286 at 777^2).
 bool gram_cycle_fits(int n, long long nnz, int m, int max_row, bool pattern, int window) {
     if (m < 1 || m > GRAM_M) return false;
     if (window > 0 && window <= 4 && n > 400000) return false;
+    if (n > 1800000 || (m <= 3 && n > 300000)) return false;
     if (!pattern && (max_row > GC_LONG_MAX || nnz > (max_row > SEQ_ROW_MAX ? 600000 : 2000000))) return false;
     return 8 * gc_shape(n, m, gc_cluster(n, nnz, max_row > SEQ_ROW_MAX, !pattern), !pattern).on >= m;
 }

