@@ -359,8 +359,8 @@ int mexk_batch_run(mexk_batch_t b);
 int mexk_batch_result(mexk_batch_t b, int problem, double* Y, mexk_result_t* results);
 /* The same with Y nrhs x rows, row-major (one right-hand side after another):
  * transposed on the device and copied straight into Y, through a device
- * buffer of Y's size that the batch keeps; on the host where there is no
- * memory for it. */
+ * buffer of Y's size that the batch keeps; small results (up to 512 rows and
+ * 4096 values) and those there is no memory for on the host. */
 int mexk_batch_result_columns(mexk_batch_t b, int problem, double* Y, mexk_result_t* results);
 int mexk_batch_info(mexk_batch_t b, mexk_batch_info_t* info);
 /* Times `iters` launches of one per-step kernel of the first wave at step j

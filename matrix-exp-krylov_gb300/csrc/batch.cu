@@ -721,18 +721,22 @@ int mexk_batch_result_columns(mexk_batch_t b, int problem, double* Y, mexk_resul
     const size_t count = static_cast<size_t>(q.rows) * q.nrhs;
     const std::lock_guard<std::mutex> lock(b->cols_mutex);
     int rc;
-    if (count > b->cols_cap) {
+    // A small result copied and transposed here costs less than a launch and a copy (host / device, us a result
+    // through Batch.result): 100 x 1 23 / 30, 500 x 1 18.7 / 20.0, 300 x 4 19.9 / 22.3, 200 x 16 29.7 / 33.4,
+    // 257 x 16 31.0 / 32.9, 500 x 16 36.0 / 32.5.
+    const bool on_device = q.rows > 512 || q.rows * q.nrhs > 4096;
+    if (on_device && count > b->cols_cap) {
         dfree(b->d_cols);
         b->cols_cap = 0;
         if (!b->test_refuse_cols && dalloc(&b->d_cols, count) == MEXK_OK) b->cols_cap = count;
         else (void)cudaGetLastError();
     }
     const double* const src = b->d_Y + b->prow0[problem] * BR;
-    if (b->cols_cap >= count) {
+    if (on_device && b->cols_cap >= count) {
         if ((rc = launch_columns(src, q.rows, q.nrhs, b->d_cols, b->stream))) return rc;
         MEXK_CK(cudaMemcpyAsync(Y, b->d_cols, sizeof(double) * count, cudaMemcpyDeviceToHost, b->stream));
         MEXK_CK(cudaStreamSynchronize(b->stream));
-    } else {  // no room for it on the device: transposed here
+    } else {  // small, or no room for it on the device
         std::vector<double> tmp(static_cast<size_t>(q.rows) * BR);
         MEXK_CK(cudaMemcpy(tmp.data(), src, sizeof(double) * tmp.size(), cudaMemcpyDeviceToHost));
         for (int r = 0; r < q.nrhs; ++r)

@@ -12,7 +12,7 @@ def test_results_without_a_device_buffer(nrhs):
     from mexk._lib import check, lib
     from mexk.batch import Batch
 
-    probs = [S.random_diag_dominant(n, 5, seed=n) for n in (65, 700)]
+    probs = [S.random_diag_dominant(n, 5, seed=n) for n in (65, 256, 257, 512, 513)]
     rng = np.random.default_rng(nrhs)
     with Batch(m=20, tol=1e-8) as b:
         for A in probs:
