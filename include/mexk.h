@@ -419,7 +419,8 @@ int mexk_profile_kernel(mexk_context_t ctx, int kind, int precision, int j, int 
  * mixed solves take the two-column steps' dots in a form-dependent order and
  * agree to rounding. A basis built in one launch (mexk_context_basis_launches)
  * takes its products itself: from the row patterns under the pattern form, else
- * from the CSR arrays. No reference counterpart: the reference's SpMV is one
+ * from the CSR arrays, whichever of the other two forms is set (their kernels
+ * run under MEXK_BASIS_SEPARATE). No reference counterpart: the reference's SpMV is one
  * cuSPARSE call (main.cu:1743). */
 #define MEXK_SPMV_STAGED 0
 #define MEXK_SPMV_DIRECT 1
@@ -431,10 +432,10 @@ int mexk_context_set_spmv_form(mexk_context_t ctx, int precision, int form);
  * symmetric matrix in the row-pattern SpMV form) runs its steps 1..m-1:
  * MEXK_LANCZOS_FUSED as one cooperative launch in which one thread block
  * per SM keeps its rows' ids and A u_j on chip and the blocks meet at two
- * bounded grid barriers per step; MEXK_LANCZOS_STEPWISE (the default) as two
- * the library does by default: in one launch with the recurrence on chip
- * where it fits (about 5 million rows), else as two launches per step (the
- * SpMV with the step's dot products, the update).
+ * bounded grid barriers per step; MEXK_LANCZOS_STEPWISE (the default) in one
+ * launch with the recurrence on chip where it fits (about 5 million rows),
+ * else as two launches per step (the SpMV with the step's dot products, the
+ * update).
  * The fused form applies when every block's rows fit its shared memory
  * (about 7 million rows on a 152-SM GB300); get reports the form a solve
  * would run. Both compute the same row sums and updates and sum the dot

@@ -1,7 +1,8 @@
 // K2: Gram-Schmidt sweeps over the Krylov basis, with the Hessenberg column
 // and the normalisation written on the device: single steps, the
 // allocation-free variant, and the bases arnoldi_cycle.cu does not take
-// (matrices with non-finite entries or more than 16 million rows).
+// (matrices with non-finite entries or more than 16 million rows, some windows
+// past 3.4 million rows, launches that were refused, by choice).
 //
 // Replaces orthogonalize_mgs (reference main.cu:1769-1876: per basis vector
 // a cublasDdot, an NCCL allreduce, a negate kernel, a cublasDaxpy and a D2H
