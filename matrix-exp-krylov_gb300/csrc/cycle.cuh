@@ -60,11 +60,15 @@ __device__ __forceinline__ bool ac_wait(unsigned* bar, unsigned target, int* sta
                         break;
                     }
                     const unsigned long long waited = ac_ns() - t0;
-                    if (waited > AC_WAIT_NS || (waited > AC_TEST_WAIT_NS && g_test_ac_dead_wait != 0)) {
-                        atomicExch(&bar[1], 1u);
-                        atomicOr(status, ST_TIMEOUT);
-                        ok = 0;
-                        break;
+                    if (waited > AC_TEST_WAIT_NS) {
+                        int hook;  // volatile: not read ahead of the test on every poll
+                        asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(hook) : "l"(&g_test_ac_dead_wait) : "memory");
+                        if (waited > AC_WAIT_NS || hook != 0) {
+                            atomicExch(&bar[1], 1u);
+                            atomicOr(status, ST_TIMEOUT);
+                            ok = 0;
+                            break;
+                        }
                     }
                     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
                 } while (static_cast<int>(seen - target) < 0);
